@@ -61,6 +61,12 @@ struct KParams {
     float inv_dr, inv_dz, inv_vdx, inv_vdy, inv_vdz;   // reciprocals for the fast mode
     // tallies (fixed point, 2^32 per unit weight)
     unsigned long long *sft, *rtd, *rz, *vox, *rbins, *region, *det, *counters;
+    // where the r-z deposits go: rz_mask + 1 (a power of two) copies of the image, each of
+    // rz_stride values, one for every block index modulo their number; launch_fold adds
+    // them to rz.  One copy: rz itself.
+    unsigned long long *rz_part;
+    int64_t rz_stride;
+    uint32_t rz_mask;
     int32_t vox_nx, vox_ny, vox_nz;
     float vox_dx, vox_dy, vox_dz;
     int32_t n_rbins;

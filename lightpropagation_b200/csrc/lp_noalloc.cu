@@ -342,6 +342,7 @@ extern "C" int lp_run_noalloc(const lp_noalloc_args *a, void *stream)
     P.sft = reinterpret_cast<unsigned long long *>(a->sft);
     P.rtd = reinterpret_cast<unsigned long long *>(a->rtd);
     P.rz = reinterpret_cast<unsigned long long *>(a->rz);
+    P.rz_part = P.rz;   // no room for copies of the image: rz_mask stays 0
     P.region = reinterpret_cast<unsigned long long *>(a->region);
     P.counters = reinterpret_cast<unsigned long long *>(sb + OFF_CNT);
     P.work = reinterpret_cast<unsigned long long *>(sb + OFF_WORK);

@@ -40,6 +40,24 @@ __global__ void __launch_bounds__(kBlock) query_kernel(const __grid_constant__ K
     }
 }
 
+// dst[k][i] += the sum of part[k][0..copies)[i], and the copies are left at zero for the
+// next launch.  k < images, i < n.  Bound by the bytes of the copies (HBM or L2).
+__global__ void __launch_bounds__(256) fold_kernel(unsigned long long *dst, unsigned long long *part, int copies,
+                                                   int64_t n, int64_t images)
+{
+    for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < n * images;
+         x += (int64_t)gridDim.x * blockDim.x) {
+        unsigned long long *const p = part + (x / n) * copies * n + x % n;
+        unsigned long long sum = 0;
+        for (int c = 0; c < copies; ++c) {
+            const unsigned long long v = p[c * n];
+            if (v) p[c * n] = 0;
+            sum += v;
+        }
+        if (sum) dst[x] += sum;
+    }
+}
+
 __global__ void philox_kernel(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, uint32_t k0,
                               uint32_t k1, int64_t n, uint32_t *out)
 {
@@ -95,6 +113,14 @@ cudaError_t launch_query(const KParams &P, int smem, int64_t n, const float *ori
     int grid = (int)std::min<int64_t>((n + kBlock - 1) / kBlock, 148 * 8);
     if (grid < 1) grid = 1;
     query_kernel<<<grid, kBlock, smem, s>>>(P, n, orig, dir, ref, tmax, id_out, t_out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_fold(unsigned long long *dst, unsigned long long *part, int copies, int64_t n, int64_t images,
+                        cudaStream_t s)
+{
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n * images + 255) / 256, 148 * 8));
+    fold_kernel<<<grid, 256, 0, s>>>(dst, part, copies, n, images);
     return cudaGetLastError();
 }
 

@@ -650,6 +650,7 @@ __device__ __forceinline__ bool complete_step(const KParams &P, const Medium *s_
         }
         if (!rz_in) cnt.rz_drop++;
         const int rz_key = rz_in ? row * P.rz_nr + col : -1;
+        unsigned long long *const rz = P.rz_part + (int64_t)(blockIdx.x & P.rz_mask) * P.rz_stride;
         if (Agg) {
             // warp-aggregated deposits: the lanes of this branch that hit the same cell
             // are matched, their fixed-point values summed exactly, and one leader per
@@ -660,7 +661,7 @@ __device__ __forceinline__ bool complete_step(const KParams &P, const Medium *s_
             if (rz_key >= 0) {
                 const unsigned long long a = group_sum_u64(g_rz, fdw), b = group_sum_u64(g_rz, fdm);
                 if (lane == (unsigned)(__ffs(g_rz) - 1)) {
-                    unsigned long long *c = P.rz + 2 * (int64_t)rz_key;
+                    unsigned long long *c = rz + 2 * (int64_t)rz_key;
                     if (a) atomicAdd(c, a);
                     if (b) atomicAdd(c + 1, b);
                     atomicAdd(s_cnt + 15, 1ull);   // leaders: 1 - leaders / deposits is the match rate
@@ -673,7 +674,7 @@ __device__ __forceinline__ bool complete_step(const KParams &P, const Medium *s_
             }
         } else {
             if (rz_key >= 0) {
-                unsigned long long *c = P.rz + 2 * (int64_t)rz_key;
+                unsigned long long *c = rz + 2 * (int64_t)rz_key;
                 if (fdw) atomicAdd(c, fdw);
                 if (fdm) atomicAdd(c + 1, fdm);
             }
