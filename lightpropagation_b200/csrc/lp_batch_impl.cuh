@@ -24,6 +24,7 @@ namespace lp {
 struct WarpSlot {
     KParams P;
     MeshView M;
+    WarpQueue Q;
     Medium media[kBatchMedia];
 };
 
@@ -144,14 +145,16 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_kernel(const __grid_constan
                 }
             }
         }
+        const bool more = step_photon<Exact, Grad, STACK>(S.P, S.M, S.M, S.Q, S.media, S.P.region, S.P.counters, alive, ph,
+                                                          cnt, &ga);
         if (alive) {
-            if (!step_photon<Exact, Grad, STACK>(S.P, S.M, S.media, S.P.region, S.P.counters, ph, cnt, &ga)) {
+            if (!more) {
                 if (ph.region_acc) atomicAdd(S.P.region + ph.curr, ph.region_acc);
                 if (Grad) {
                     ga.L[ph.curr] += ph.seg_len;
                     ga.k[ph.curr] += ph.seg_k;
                 }
-                finish_photon<Grad>(S.P, ph, Grad ? &ga : nullptr);
+                finish_photon<Grad>(S.P, exit_state(ph), Grad ? &ga : nullptr);
                 photons++;
                 alive = false;
             }

@@ -133,16 +133,18 @@ __device__ __forceinline__ bool in_range_dbg(unsigned long long *dbg, long long 
 
 constexpr uint32_t kCellEmpty = 0x80000000u;
 constexpr uint32_t kCellDense = 127u;
-constexpr int kLocalMaxCells = 8;   // larger segment boxes go to the BVH
+constexpr uint32_t kCellOutside = 0x00010000u;
 
-// The cell word at p; points outside the grid read as an empty cell with bound 0.
+// The cell word at p; points outside the grid read as an empty cell with bound 0 and
+// kCellOutside set.
 __device__ __forceinline__ uint32_t cell_at(const KParams &P, float px, float py, float pz)
 {
-    if (!P.cell_word) return kCellEmpty;
+    if (!P.cell_word) return kCellEmpty | kCellOutside;
     const int ix = (int)floorf((px - P.g_ox) * P.g_inv_h);
     const int iy = (int)floorf((py - P.g_oy) * P.g_inv_h);
     const int iz = (int)floorf((pz - P.g_oz) * P.g_inv_h);
-    if (ix < 0 || iy < 0 || iz < 0 || ix >= P.g_nx || iy >= P.g_ny || iz >= P.g_nz) return kCellEmpty;
+    if (ix < 0 || iy < 0 || iz < 0 || ix >= P.g_nx || iy >= P.g_ny || iz >= P.g_nz)
+        return kCellEmpty | kCellOutside;
     return __ldg(P.cell_word + ((int64_t)iz * P.g_ny + iy) * P.g_nx + ix);
 }
 
@@ -261,80 +263,60 @@ struct MeshView {
     unsigned long long *dbg;         // its counter of skipped accesses (may be null)
 };
 
-__device__ __forceinline__ void test_tri(const MeshView &M, int j, V3 p, V3 v, int ref_tri, float &best,
-                                         int &bid)
-{
-    if (!LP_IN_RANGE(M.dbg, j, M.n_tri)) return;
+// A triangle record in BVH order: staged in shared memory or read from the mesh arrays.
+struct TriRec {
     float4 a, b, c;
+};
+__device__ __forceinline__ TriRec load_tri(const MeshView &M, int j)
+{
+    TriRec T;
     if (j < M.tris_smem) {
-        a = M.s_ta[j]; b = M.s_tb[j]; c = M.s_tc[j];
+        T.a = M.s_ta[j]; T.b = M.s_tb[j]; T.c = M.s_tc[j];
     } else {
-        a = __ldg(M.ta + j); b = __ldg(M.tb + j); c = __ldg(M.tc + j);
+        T.a = __ldg(M.ta + j); T.b = __ldg(M.tb + j); T.c = __ldg(M.tc + j);
     }
-    const int o = __float_as_int(c.y);
-    if (o == ref_tri) return;
-    const V3 Mv = v3(a.x, a.y, a.z), E = v3(a.w, b.x, b.y), F = v3(b.z, b.w, c.x);
-    const V3 G = sub3(p, Mv);
-    const V3 GE = cross3(G, E), VF = cross3(v, F);
-    float t = dot3(GE, F);
+    return T;
+}
+
+// The reference's ray/triangle test (.cl:1047-1083) of the ray (p, v), with G = p - M,
+// GE = G x E and t0 = GE . F already formed: true when the triangle is hit at t in
+// (0, kNoHit) with t not above `limit` by more than the filter's margin.
+__device__ __forceinline__ bool tri_hit(const MeshView &M, V3 E, V3 F, V3 G, V3 GE, float t0, V3 v, float limit,
+                                        float &t_out)
+{
+    const V3 VF = cross3(v, F);
+    float t = t0;
     const float w = dot3(VF, E);
     float k = dot3(VF, G);
     float l = dot3(GE, v);
     // Division-free filter, looser than the exact test below: t, k, l must share the
-    // sign of w, |k| + |l| may not exceed |w| and |t| may not exceed best * |w| (each
+    // sign of w, |k| + |l| may not exceed |w| and |t| may not exceed limit * |w| (each
     // with a relative margin far above the rounding of the divided values).  Only
     // candidates that pass pay for the three IEEE divisions of the reference test.
     const float aw = fabsf(w);
     const float ek = M.tri_eps * aw;
     const bool sgn = (w > 0.0f) ? (t > 0.0f && k >= -ek && l >= -ek) : (t < 0.0f && k <= ek && l <= ek);
-    if (!sgn || fabsf(k) + fabsf(l) > aw * (1.0001f + 3.0f * M.tri_eps) || fabsf(t) > best * aw * 1.0001f) return;
+    if (!sgn || fabsf(k) + fabsf(l) > aw * (1.0001f + 3.0f * M.tri_eps) || fabsf(t) > limit * aw * 1.0001f)
+        return false;
     t = t / w;
     k = k / w;
     l = l / w;
-    if (t > 0.0f && t < kNoHit && k >= -M.tri_eps && l >= -M.tri_eps && (k + l) < 1.0f + M.tri_eps &&
-        (t < best || (t == best && o < bid))) {
-        best = t;
-        bid = o;
-    }
+    t_out = t;
+    return t > 0.0f && t < kNoHit && k >= -M.tri_eps && l >= -M.tri_eps && (k + l) < 1.0f + M.tri_eps;
 }
 
-// test_tri plus a lower bound of the distance from p to the triangle: the distance to
-// its plane, |(G x E) . F| / |E x F|, less a bound of the rounding of that product
-// (tri_c.z = 1 / |E x F|, tri_c.w = the rounding factor per unit |G|, see lp_bvh.hpp).
-// safe is lowered to that bound; the hit test is test_tri's, operation for operation.
-__device__ __forceinline__ void test_tri_safe(const MeshView &M, int j, V3 p, V3 v, int ref_tri, float &best,
-                                              int &bid, float &safe)
+__device__ __forceinline__ void test_tri(const MeshView &M, int j, V3 p, V3 v, int ref_tri, float &best,
+                                         int &bid)
 {
-    if (!LP_IN_RANGE(M.dbg, j, M.n_tri)) {
-        safe = 0.0f;
-        return;
-    }
-    float4 a, b, c;
-    if (j < M.tris_smem) {
-        a = M.s_ta[j]; b = M.s_tb[j]; c = M.s_tc[j];
-    } else {
-        a = __ldg(M.ta + j); b = __ldg(M.tb + j); c = __ldg(M.tc + j);
-    }
-    const V3 Mv = v3(a.x, a.y, a.z), E = v3(a.w, b.x, b.y), F = v3(b.z, b.w, c.x);
-    const V3 G = sub3(p, Mv);
-    const V3 GE = cross3(G, E);
-    float t = dot3(GE, F);
-    safe = fminf(safe, fabsf(t) * c.z - c.w * (fabsf(G.x) + fabsf(G.y) + fabsf(G.z)));
-    const int o = __float_as_int(c.y);
+    if (!LP_IN_RANGE(M.dbg, j, M.n_tri)) return;
+    const TriRec T = load_tri(M, j);
+    const int o = __float_as_int(T.c.y);
     if (o == ref_tri) return;
-    const V3 VF = cross3(v, F);
-    const float w = dot3(VF, E);
-    float k = dot3(VF, G);
-    float l = dot3(GE, v);
-    const float aw = fabsf(w);
-    const float ek = M.tri_eps * aw;
-    const bool sgn = (w > 0.0f) ? (t > 0.0f && k >= -ek && l >= -ek) : (t < 0.0f && k <= ek && l <= ek);
-    if (!sgn || fabsf(k) + fabsf(l) > aw * (1.0001f + 3.0f * M.tri_eps) || fabsf(t) > best * aw * 1.0001f) return;
-    t = t / w;
-    k = k / w;
-    l = l / w;
-    if (t > 0.0f && t < kNoHit && k >= -M.tri_eps && l >= -M.tri_eps && (k + l) < 1.0f + M.tri_eps &&
-        (t < best || (t == best && o < bid))) {
+    const V3 E = v3(T.a.w, T.b.x, T.b.y), F = v3(T.b.z, T.b.w, T.c.x);
+    const V3 G = sub3(p, v3(T.a.x, T.a.y, T.a.z));
+    const V3 GE = cross3(G, E);
+    float t;
+    if (tri_hit(M, E, F, G, GE, dot3(GE, F), v, best, t) && (t < best || (t == best && o < bid))) {
         best = t;
         bid = o;
     }
@@ -412,118 +394,183 @@ __device__ __noinline__ int query_nearest(const MeshView &M, V3 p, V3 v, int ref
     return bid;
 }
 
-// The same query answered from the cell grid when the segment [p, p + bound v] is short:
-// every triangle that touches a cell overlapping the segment's bounding box (widened by
-// g_eps) is tested with test_tri, so the candidate set holds every triangle the test can
-// accept within the bound, and the result (nearest t, then lowest original index) is
-// the BVH's bit for bit.  Boxes of more than kLocalMaxCells cells, or a dense cell, go
-// to query_nearest; *used_bvh reports which path answered.
-template <int STACK = kStackDepth>
-__device__ __forceinline__ int cell_query(const KParams &P, const MeshView &M, V3 p, V3 v, int ref_tri,
-                                          float bound, float &t_out, bool &used_bvh)
+// Per-warp shared memory of warp_query: the rays and results of up to kQueue queries,
+// and the list segments of one pass.
+constexpr int kQueue = 16;
+struct WarpQueue {
+    float4 ray0[kQueue], ray1[kQueue];     // (p, v.x), (v.y, v.z, bound, ref_tri as int bits)
+    unsigned long long best[kQueue];       // (t as float bits) << 32 | original index
+    uint32_t safe[kQueue];                 // distance bound as float bits (>= 0)
+    uint32_t seg[kQueue];                  // query << 27 | (first list entry - first item + kSegBias)
+};
+constexpr uint32_t kSegBias = 4096;        // above kQueue * kCellDense, so a segment's word is not negative
+constexpr uint32_t kNoTri = 0x7fffffffu;
+constexpr int kMarchMax = 512;             // cells of one march; a longer one goes to the BVH
+
+// Distance along the ray to the grid's box (0 inside, kNoHit when the ray misses it).
+__device__ __forceinline__ float grid_entry(const KParams &P, V3 p, V3 v)
 {
-    used_bvh = true;
-    if (!P.cell_refs || !(bound < kNoHit)) return query_nearest<STACK>(M, p, v, ref_tri, bound, t_out);
-    const float e = P.g_eps;
-    const float qx = p.x + bound * v.x, qy = p.y + bound * v.y, qz = p.z + bound * v.z;
-    const int nx = P.g_nx, ny = P.g_ny, nz = P.g_nz;
-    const int x0 = min(max((int)floorf((fminf(p.x, qx) - e - P.g_ox) * P.g_inv_h), 0), nx - 1);
-    const int x1 = min(max((int)floorf((fmaxf(p.x, qx) + e - P.g_ox) * P.g_inv_h), 0), nx - 1);
-    const int y0 = min(max((int)floorf((fminf(p.y, qy) - e - P.g_oy) * P.g_inv_h), 0), ny - 1);
-    const int y1 = min(max((int)floorf((fmaxf(p.y, qy) + e - P.g_oy) * P.g_inv_h), 0), ny - 1);
-    const int z0 = min(max((int)floorf((fminf(p.z, qz) - e - P.g_oz) * P.g_inv_h), 0), nz - 1);
-    const int z1 = min(max((int)floorf((fmaxf(p.z, qz) + e - P.g_oz) * P.g_inv_h), 0), nz - 1);
-    if ((x1 - x0 + 1) * (y1 - y0 + 1) * (z1 - z0 + 1) > kLocalMaxCells)
-        return query_nearest<STACK>(M, p, v, ref_tri, bound, t_out);
-    float best = bound;
-    int bid = 0x7fffffff;
-    for (int z = z0; z <= z1; ++z)
-        for (int y = y0; y <= y1; ++y)
-            for (int x = x0; x <= x1; ++x) {
-                const uint32_t w = __ldg(P.cell_word + ((int64_t)z * ny + y) * nx + x);
-                if (w & kCellEmpty) continue;
-                uint32_t cnt = (w >> 24) & 127u;
-                if (cnt == kCellDense) return query_nearest<STACK>(M, p, v, ref_tri, bound, t_out);
-                if (!LP_IN_RANGE(M.dbg, (int64_t)(w & 0xffffffu) + cnt - 1, P.n_cell_refs)) cnt = 0;
-                const int32_t *r = P.cell_refs + (w & 0xffffffu);
-                for (uint32_t k = 0; k < cnt; ++k) test_tri(M, __ldg(r + k), p, v, ref_tri, best, bid);
-            }
-    used_bvh = false;
-    if (bid == 0x7fffffff) {
-        t_out = kNoHit;
-        return -1;
+    float t0 = 0.0f, t1 = kNoHit;
+    const float o[3] = {P.g_ox, P.g_oy, P.g_oz}, q[3] = {p.x, p.y, p.z}, d[3] = {v.x, v.y, v.z};
+    const int n[3] = {P.g_nx, P.g_ny, P.g_nz};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float lo = o[a] - q[a], hi = o[a] + (float)n[a] * P.g_h - q[a];
+        if (fabsf(d[a]) > 1e-30f) {
+            const float x = lo / d[a], y = hi / d[a];
+            t0 = fmaxf(t0, fminf(x, y));
+            t1 = fminf(t1, fmaxf(x, y));
+        } else if (lo > 0.0f || hi < 0.0f) {
+            t0 = kNoHit;
+        }
     }
-    t_out = best;
-    return bid;
+    return t0 <= t1 ? t0 : kNoHit;
 }
 
-// The transport's query over the cell lists, one loop for both cases (one inlined copy of
-// the triangle test):
-//   * the step stays within the photon's own widened cell (word: its list word, not
-//     dense): that cell's list alone decides it.  The list holds every triangle touching
-//     the cell widened by g_margin + g_eps, so an unlisted triangle lies at least
-//     g_margin + dface from p (dface: distance from p to the cell's faces), and no
-//     segment from p of length <= reach = g_margin + dface - g_eps can reach one.  `safe`
-//     (coming in with a lower bound already known, the photon's carried one) is raised to
-//     a lower bound of the distance from p to every triangle: reach for the unlisted ones,
-//     their plane distance (test_tri_safe) for the listed ones, 0 on a triangle
-//     (ref_tri >= 0);
-//   * otherwise the lists of the cells the segment's box covers (at most kLocalMaxCells),
-//     as cell_query; longer segments and dense cells go to the BVH.  The bound of the own
-//     list would not outlast such a step (it is at most that list's reach), so `safe`
-//     stays as it is.
-// Same candidates, test and tie-break as cell_query and the BVH: the same hit.
+// The warp's nearest-triangle queries over the cell lists; every lane calls it, those with
+// `want` have a query: the nearest triangle along (p, v) with t in (0, bound] and
+// t < kNoHit, ref_tri excluded, equal distances resolving to the lower original index.
+// Returns its original index or -1 with t_out = kNoHit.
+//
+// A query marches along its ray.  At distance s it stands in a cell (word: the cell at
+// s = 0), d from the cell's faces:
+//   * a listed cell: its list holds every triangle touching the cell widened by
+//     g_margin + g_eps, so every triangle the ray can meet up to s + g_margin + d - g_eps;
+//     it is tested, and the march goes on from 15/16 of that distance;
+//   * an empty cell: no triangle lies within g_margin + d - g_eps, nor within the word's
+//     bound; the march goes on from 15/16 of the larger;
+//   * outside the grid: on to the grid's box, or the end when the ray does not meet it.
+// It ends when s has passed the bound or the nearest hit so far.  Most queries are
+// decided by the list they start in (bound <= g_margin + d - g_eps); for those `safe`
+// (coming in with a lower bound already known, the photon's carried one) is raised to a
+// lower bound of the distance from p to every triangle: g_margin + d - g_eps for the
+// unlisted ones, the distance to their plane for the listed ones, |(G x E) . F| / |E x F|
+// less a bound of the rounding of that product (tri_c.z = 1 / |E x F|, tri_c.w = the
+// rounding factor per unit |G|, see lp_bvh.hpp), 0 on a triangle (ref_tri >= 0).
+// Dense cells, marches past kMarchMax cells or stuck (lists without a margin), and a mesh
+// without lists go to the BVH (used_bvh).  Same test and tie-break everywhere, and the
+// lists' margins are wider than the BVH's boxes, so the hit is the BVH's bit for bit.
+//
+// About a tenth of the lanes have a query on the same step, each with a list of its own
+// length, so a loop per lane leaves the warp nearly empty.  Here the triangles of all the
+// warp's lists form one sequence of items and the 32 lanes test 32 items at a time, each
+// with the ray of the item's query read from shared memory; hits and distance bounds meet
+// in shared memory by atomic minimum, which no order can change.
+//
+// M and SM are the same view: M's members are the kernel's parameters, SM is its copy in
+// shared memory for the out-of-line BVH descent, which needs an address (that of M would
+// move M to local memory, and its pointers would be loaded from there for every item).
 template <int STACK = kStackDepth>
-__device__ __forceinline__ int grid_query(const KParams &P, const MeshView &M, V3 p, V3 v, int ref_tri, float bound,
-                                          uint32_t word, float &t_out, float &safe, bool &used_bvh)
+__device__ __forceinline__ int warp_query(const KParams &P, const MeshView &M, const MeshView &SM, WarpQueue &Q,
+                                          bool want, V3 p, V3 v, int ref_tri, float bound, uint32_t word, float &t_out,
+                                          float &safe, bool &used_bvh)
 {
-    used_bvh = true;
-    if (!P.cell_refs) return query_nearest<STACK>(M, p, v, ref_tri, bound, t_out);
-    const int nx = P.g_nx, ny = P.g_ny, nz = P.g_nz;
-    const bool listed = !(word & kCellEmpty) && ((word >> 24) & 127u) != kCellDense;
-    const bool own = listed && bound <= P.g_margin + cell_face_distance(P, p.x, p.y, p.z) - P.g_eps;
-    int x0, x1, y0, y1, z0, z1;
-    if (own) {
-        x0 = x1 = (int)floorf((p.x - P.g_ox) * P.g_inv_h);
-        y0 = y1 = (int)floorf((p.y - P.g_oy) * P.g_inv_h);
-        z0 = z1 = (int)floorf((p.z - P.g_oz) * P.g_inv_h);
-    } else {
-        if (!(bound < kNoHit)) return query_nearest<STACK>(M, p, v, ref_tri, bound, t_out);
-        const float e = P.g_eps;
-        const float qx = p.x + bound * v.x, qy = p.y + bound * v.y, qz = p.z + bound * v.z;
-        x0 = min(max((int)floorf((fminf(p.x, qx) - e - P.g_ox) * P.g_inv_h), 0), nx - 1);
-        x1 = min(max((int)floorf((fmaxf(p.x, qx) + e - P.g_ox) * P.g_inv_h), 0), nx - 1);
-        y0 = min(max((int)floorf((fminf(p.y, qy) - e - P.g_oy) * P.g_inv_h), 0), ny - 1);
-        y1 = min(max((int)floorf((fmaxf(p.y, qy) + e - P.g_oy) * P.g_inv_h), 0), ny - 1);
-        z0 = min(max((int)floorf((fminf(p.z, qz) - e - P.g_oz) * P.g_inv_h), 0), nz - 1);
-        z1 = min(max((int)floorf((fmaxf(p.z, qz) + e - P.g_oz) * P.g_inv_h), 0), nz - 1);
-        if ((x1 - x0 + 1) * (y1 - y0 + 1) * (z1 - z0 + 1) > kLocalMaxCells)
-            return query_nearest<STACK>(M, p, v, ref_tri, bound, t_out);
-    }
-    float best = bound, s = own ? P.g_margin + cell_face_distance(P, p.x, p.y, p.z) - P.g_eps : 0.0f;
-    int bid = 0x7fffffff;
-    for (int z = z0; z <= z1; ++z)
-        for (int y = y0; y <= y1; ++y)
-            for (int x = x0; x <= x1; ++x) {
-                const uint32_t w = own ? word : __ldg(P.cell_word + ((int64_t)z * ny + y) * nx + x);
-                if (w & kCellEmpty) continue;
-                uint32_t cnt = (w >> 24) & 127u;
-                if (cnt == kCellDense) return query_nearest<STACK>(M, p, v, ref_tri, bound, t_out);
-                if (!LP_IN_RANGE(M.dbg, (int64_t)(w & 0xffffffu) + cnt - 1, P.n_cell_refs)) {
-                    cnt = 0;
-                    s = 0.0f;
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned lt_mask = (1u << lane) - 1u;
+    int tri = -1;
+    t_out = kNoHit;
+    bool bvh = want && !P.cell_refs;
+    unsigned todo = __ballot_sync(0xffffffffu, want && !bvh);
+    while (todo) {
+        const int rank = __popc(todo & lt_mask);
+        const bool mine = ((todo >> lane) & 1u) && rank < kQueue;
+        float s = 0.0f, limit = fminf(bound, kNoHit);
+        int cells = 0;
+        bool first = true, own = false;
+        if (mine) {
+            Q.ray0[rank] = make_float4(p.x, p.y, p.z, v.x);
+            Q.ray1[rank] = make_float4(v.y, v.z, limit, __int_as_float(ref_tri));
+            Q.best[rank] = ((unsigned long long)__float_as_uint(limit) << 32) | kNoTri;
+        }
+        for (;;) {
+            // each query's next list
+            uint32_t cnt = 0, off = 0;
+            while (mine && !bvh && cnt == 0 && s <= limit) {
+                const V3 q = v3(p.x + s * v.x, p.y + s * v.y, p.z + s * v.z);
+                const uint32_t w = first ? word : cell_at(P, q.x, q.y, q.z);
+                float reach = P.g_margin + cell_face_distance(P, q.x, q.y, q.z) - P.g_eps;
+                if (w & kCellEmpty) {
+                    if (w & kCellOutside) {
+                        // just inside the box: its outermost cells hold no triangle
+                        const float t = grid_entry(P, q, v);
+                        reach = t < kNoHit ? t + 0.25f * P.g_h : 4.0f * kNoHit;
+                    } else {
+                        reach = fmaxf(reach, safe_distance(P, w));
+                    }
+                } else {
+                    cnt = (w >> 24) & 127u;
+                    off = w & 0xffffffu;
+                    bvh = cnt == kCellDense;
+                    own = first && bound <= reach && !bvh;
+                    if (first) Q.safe[rank] = __float_as_uint(ref_tri < 0 ? fmaxf(reach, 0.0f) : 0.0f);
+                    if (!LP_IN_RANGE(M.dbg, (int64_t)off + cnt - 1, P.n_cell_refs)) {
+                        cnt = 0;
+                        Q.safe[rank] = 0u;
+                    }
                 }
-                const int32_t *r = P.cell_refs + (w & 0xffffffu);
-                for (uint32_t k = 0; k < cnt; ++k) test_tri_safe(M, __ldg(r + k), p, v, ref_tri, best, bid, s);
+                first = false;
+                if (++cells > kMarchMax || !(reach > 0.125f * P.g_h)) bvh = bvh || !own;
+                s = own ? 2.0f * kNoHit : s + 0.9375f * reach;
+                if (bvh) cnt = 0;
             }
-    used_bvh = false;
-    if (own) safe = fmaxf(safe, ref_tri >= 0 ? 0.0f : fmaxf(s - P.g_eps, 0.0f));
-    if (bid == 0x7fffffff) {
-        t_out = kNoHit;
-        return -1;
+            const unsigned segs = __ballot_sync(0xffffffffu, cnt > 0);
+            if (!segs) break;
+            uint32_t end = cnt;   // items up to and including this lane's
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t x = __shfl_up_sync(0xffffffffu, end, o);
+                if (lane >= (unsigned)o) end += x;
+            }
+            const uint32_t total = __shfl_sync(0xffffffffu, end, 31);
+            const uint32_t start = end - cnt;
+            if (cnt) Q.seg[__popc(segs & lt_mask)] = ((uint32_t)rank << 27) | (off + kSegBias - start);
+            __syncwarp();
+            for (uint32_t r = 0; r < total; r += 32) {
+                // the segment of item r + lane: the last one that starts at or before it
+                const bool here = cnt && start >= r && start < r + 32u;
+                const unsigned heads = __reduce_or_sync(0xffffffffu, here ? 1u << (start - r) : 0u);
+                const int before = __popc(__ballot_sync(0xffffffffu, cnt && start < r));
+                const uint32_t item = r + lane;
+                if (item < total) {
+                    const uint32_t sg = Q.seg[before + __popc(heads & (lt_mask | (1u << lane))) - 1];
+                    const uint32_t k = sg >> 27;
+                    const int j = __ldg(P.cell_refs + ((sg & 0x7ffffffu) - kSegBias + item));
+                    if (LP_IN_RANGE(M.dbg, j, M.n_tri)) {
+                        const TriRec T = load_tri(M, j);
+                        const float4 r0 = Q.ray0[k], r1 = Q.ray1[k];
+                        const V3 E = v3(T.a.w, T.b.x, T.b.y), F = v3(T.b.z, T.b.w, T.c.x);
+                        const V3 G = sub3(v3(r0.x, r0.y, r0.z), v3(T.a.x, T.a.y, T.a.z));
+                        const V3 GE = cross3(G, E);
+                        const float t0 = dot3(GE, F);
+                        const float d = fabsf(t0) * T.c.z - T.c.w * (fabsf(G.x) + fabsf(G.y) + fabsf(G.z));
+                        atomicMin(&Q.safe[k], __float_as_uint(fmaxf(d, 0.0f)));
+                        const int o = __float_as_int(T.c.y);
+                        float t;
+                        if (o != __float_as_int(r1.w) &&
+                            tri_hit(M, E, F, G, GE, t0, v3(r0.w, r1.x, r1.y), r1.z, t) && t <= r1.z)
+                            atomicMin(&Q.best[k], ((unsigned long long)__float_as_uint(t) << 32) | (unsigned)o);
+                    } else {
+                        atomicMin(&Q.safe[k], 0u);
+                    }
+                }
+            }
+            __syncwarp();
+            if (mine) limit = __uint_as_float((uint32_t)(Q.best[rank] >> 32));
+        }
+        if (mine && !bvh) {
+            const unsigned long long b = Q.best[rank];
+            if ((uint32_t)b != kNoTri) {
+                tri = (int)(uint32_t)b;
+                t_out = __uint_as_float((uint32_t)(b >> 32));
+            }
+            if (own) safe = fmaxf(safe, fmaxf(__uint_as_float(Q.safe[rank]) - P.g_eps, 0.0f));
+        }
+        __syncwarp();
+        todo &= ~__ballot_sync(0xffffffffu, mine);
     }
-    t_out = best;
-    return bid;
+    if (bvh) tri = query_nearest<STACK>(SM, p, v, ref_tri, bound, t_out);
+    used_bvh = bvh;
+    return tri;
 }
 
 }  // namespace lp

@@ -26,17 +26,28 @@ __global__ void __launch_bounds__(kBlock) query_kernel(const __grid_constant__ K
                                                        int32_t *id_out, float *t_out)
 {
     extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ WarpQueue queues[kBlock / 32];
     const SmemLayout L = smem_layout(P.nodes_smem, P.tris_smem);
     const MeshView M = stage_mesh(P, smem, L);
+    __shared__ MeshView shared_view;
+    if (threadIdx.x == 0) shared_view = M;
     __syncthreads();
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const V3 p = v3(orig[3 * i], orig[3 * i + 1], orig[3 * i + 2]);
-        const V3 v = v3(dir[3 * i], dir[3 * i + 1], dir[3 * i + 2]);
-        float t;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    // warp-uniform trip count: the query is the whole warp's
+    for (int64_t w = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31u); w < n; w += stride) {
+        const int64_t i = w + (threadIdx.x & 31u);
+        const bool want = i < n;
+        const int64_t q = want ? i : 0;
+        const V3 p = v3(orig[3 * q], orig[3 * q + 1], orig[3 * q + 2]);
+        const V3 v = v3(dir[3 * q], dir[3 * q + 1], dir[3 * q + 2]);
+        float t, safe = 0.0f;
         bool used_bvh;
-        id_out[i] = cell_query(P, M, p, v, ref[i], tmax[i], t, used_bvh);
-        t_out[i] = t;
+        const int id = warp_query(P, M, shared_view, queues[threadIdx.x >> 5], want, p, v, ref[q], tmax[q],
+                                  cell_at(P, p.x, p.y, p.z), t, safe, used_bvh);
+        if (want) {
+            id_out[i] = id;
+            t_out[i] = t;
+        }
     }
 }
 

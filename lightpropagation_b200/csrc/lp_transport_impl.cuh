@@ -220,10 +220,22 @@ static __device__ __noinline__ void score_gradient(const KParams &P, const GradA
     }
 }
 
+// What an exit record needs of a photon, passed by value: a reference would take the photon's address out of the step loop, and every
+// step would then store it to local memory.
+struct ExitState {
+    float px, py, pz, vx, vy, vz, exit_w;
+    int32_t last_tri;
+    uint32_t flags, idx;
+};
+__device__ __forceinline__ ExitState exit_state(const Photon &ph)
+{
+    return ExitState{ph.px, ph.py, ph.pz, ph.vx, ph.vy, ph.vz, ph.exit_w, ph.last_tri, ph.flags, ph.idx};
+}
+
 // The normal of the photon's last boundary event as the transport used it: the face's unit
 // normal, the on-axis override (sign * eZ), or (0, 0, -1) before any event (PhotonClass
 // init, .cl:344-389).  Kept as the face index and two flag bits instead of three floats.
-__device__ __forceinline__ V3 photon_normal(const KParams &P, const Photon &ph)
+__device__ __forceinline__ V3 photon_normal(const KParams &P, const ExitState &ph)
 {
     const uint32_t axis = (ph.flags >> AXIS_SHIFT) & 3u;
     if (axis) {
@@ -237,7 +249,7 @@ __device__ __forceinline__ V3 photon_normal(const KParams &P, const Photon &ph)
 
 // Exit record binning of CalculatePropagation.cpp:1553-1626 plus radial bins and rings.
 template <bool Grad>
-static __device__ __noinline__ void finish_photon(const KParams &P, const Photon &ph, const GradAcc *ga)
+static __device__ __noinline__ void finish_photon(const KParams &P, const ExitState ph, const GradAcc *ga)
 {
     const V3 v = v3(ph.vx, ph.vy, ph.vz), nv = photon_normal(P, ph);
     const float alpha = fabsf(acosf(dot3(v, nv)));
@@ -557,24 +569,21 @@ __device__ __forceinline__ int propose_step(const KParams &P, const Medium *s_me
 }
 
 // The nearest triangle within the step's reach (-1: none) and its distance thit; updates
-// the distance bound the query establishes.
+// the distance bound the query establishes.  Every lane of the warp calls it, the ones
+// whose step needs a query with `want`.
 template <int STACK>
-__device__ __forceinline__ int query_step(const KParams &P, const MeshView &M, const Medium *s_media,
-                                          const Photon &ph, Counters &cnt, Pending &pd, float &thit)
+__device__ __forceinline__ int query_step(const KParams &P, const MeshView &M, const MeshView &SM, WarpQueue &Q,
+                                          const Medium *s_media, bool want, const Photon &ph, Counters &cnt, Pending &pd, float &thit)
 {
-    const V3 p = v3(ph.px, ph.py, ph.pz), v = v3(ph.vx, ph.vy, ph.vz);
-    int tri = -1;
-    if (s_media[ph.curr].ambient) {
-        tri = query_nearest<STACK>(M, p, v, ph.refTri, kNoHit, thit);
-        cnt.query++;
-        cnt.bvh++;
-        return tri;
-    }
+    thit = kNoHit;
+    if (!__any_sync(0xffffffffu, want)) return -1;
+    const bool ambient = want && s_media[ph.curr].ambient;
+    bool used_bvh;
     // an empty cell: pd.safe_here holds its bound, which the step exceeds; a listed cell
     // raises it from the planes of its triangles when its list decides the step
-    bool used_bvh;
-    tri = grid_query<STACK>(P, M, p, v, ph.refTri, pd.reach, pd.word, thit, pd.safe_here, used_bvh);
-    cnt.query++;
+    const int tri = warp_query<STACK>(P, M, SM, Q, want, v3(ph.px, ph.py, ph.pz), v3(ph.vx, ph.vy, ph.vz),
+                                      ph.refTri, ambient ? kNoHit : pd.reach, pd.word, thit, pd.safe_here, used_bvh);
+    cnt.query += want ? 1u : 0u;
     cnt.bvh += used_bvh ? 1u : 0u;
     return tri;
 }
@@ -700,19 +709,20 @@ __device__ __forceinline__ bool complete_step(const KParams &P, const Medium *s_
     return ph.w > 0.0f && (ph.w > P.w_th || (ph.flags & F_ROULETTE));
 }
 
-// One iteration of the reference's do-while loop, the three parts in turn.  Returns false
-// when the photon ends.
+// One iteration of the reference's do-while loop, the three parts in turn, for the warp's
+// photons (the whole warp calls it, `alive` lanes have one).  Returns false when the
+// lane's photon ends.
 template <bool Exact, bool Grad, int STACK = kStackDepth, bool Agg = false>
-__device__ __forceinline__ bool step_photon(const KParams &P, const MeshView &M, const Medium *s_media,
-                                            unsigned long long *s_region, unsigned long long *s_cnt,
+__device__ __forceinline__ bool step_photon(const KParams &P, const MeshView &M, const MeshView &SM, WarpQueue &Q,
+                                            const Medium *s_media, unsigned long long *s_region, unsigned long long *s_cnt, bool alive,
                                             Photon &ph, Counters &cnt, GradAcc *ga)
 {
     Pending pd;
-    const int st = propose_step<Exact>(P, s_media, ph, cnt, pd);
+    int st = kStepEnded;
+    if (alive) st = propose_step<Exact>(P, s_media, ph, cnt, pd);
+    float thit;
+    const int tri = query_step<STACK>(P, M, SM, Q, s_media, st == kStepQuery, ph, cnt, pd, thit);
     if (st == kStepEnded) return false;
-    float thit = kNoHit;
-    int tri = -1;
-    if (st == kStepQuery) tri = query_step<STACK>(P, M, s_media, ph, cnt, pd, thit);
     return complete_step<Exact, Grad, Agg>(P, s_media, s_region, s_cnt, ph, cnt, ga, pd, tri, thit);
 }
 
@@ -771,6 +781,7 @@ template <bool Exact, bool Grad, bool Agg = false>
 __global__ void __launch_bounds__(kBlock, LP_TRANSPORT_MIN_BLOCKS) transport_kernel(const __grid_constant__ KParams P)
 {
     extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ WarpQueue queues[kBlock / 32];
     const SmemLayout L = smem_layout(P.nodes_smem, P.tris_smem);
     Medium *s_media = reinterpret_cast<Medium *>(smem + L.off_media);
     unsigned long long *s_region = reinterpret_cast<unsigned long long *>(smem + L.off_region);
@@ -781,6 +792,8 @@ __global__ void __launch_bounds__(kBlock, LP_TRANSPORT_MIN_BLOCKS) transport_ker
     }
     if (threadIdx.x < 16) s_cnt[threadIdx.x] = 0;
     const MeshView M = stage_mesh(P, smem, L);
+    __shared__ MeshView shared_view;
+    if (threadIdx.x == 0) shared_view = M;
     __syncthreads();
 
     const unsigned lane = threadIdx.x & 31u;
@@ -814,14 +827,16 @@ __global__ void __launch_bounds__(kBlock, LP_TRANSPORT_MIN_BLOCKS) transport_ker
             }
         }
         if (!__any_sync(0xffffffffu, alive)) break;
+        const bool more = step_photon<Exact, Grad, kStackDepth, Agg>(P, M, shared_view, queues[threadIdx.x >> 5], s_media, s_region,
+                                                                     s_cnt, alive, ph, cnt, &ga);
         if (alive) {
-            if (!step_photon<Exact, Grad, kStackDepth, Agg>(P, M, s_media, s_region, s_cnt, ph, cnt, &ga)) {
+            if (!more) {
                 if (ph.region_acc) atomicAdd(s_region + ph.curr, ph.region_acc);
                 if (Grad) {
                     ga.L[ph.curr] += ph.seg_len;
                     ga.k[ph.curr] += ph.seg_k;
                 }
-                finish_photon<Grad>(P, ph, Grad ? &ga : nullptr);
+                finish_photon<Grad>(P, exit_state(ph), Grad ? &ga : nullptr);
                 photons++;
                 alive = false;
             }

@@ -1,0 +1,44 @@
+"""Nearest-triangle queries that march over the cell lists, against the BVH alone (which
+test_gpu_parity compares with the full scan): the same id and the same bits of t at the
+edges of the march."""
+import numpy as np
+import pytest
+
+from lightpropagation_b200 import Simulation, meshes
+
+pytestmark = pytest.mark.gpu
+
+
+def rays(n, rng):
+    """From inside, from outside (entering the grid or missing it), along the axes, on the
+    grid's corner planes, with bounds from negative to beyond every hit."""
+    o = rng.uniform(-160, 160, (n, 3))
+    o[::5] *= 20.0
+    d = rng.normal(size=(n, 3))
+    d[1::4] = np.eye(3)[rng.integers(0, 3, len(d[1::4]))] * rng.choice([-1.0, 1.0], (len(d[1::4]), 1))
+    d[::5] = rng.uniform(-100, 100, d[::5].shape) - o[::5]
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    t = rng.choice([-1.0, 0.0, 0.05, 0.7, 5.0, 60.0, 10000.0, 3e38], n)
+    return o.astype(np.float32), d.astype(np.float32), np.full(n, -1, np.int32), t.astype(np.float32)
+
+
+# margins of the lists (0: every march is stuck), cells of the grid (few: dense cells),
+# counts around a warp and the queries it takes at a time
+@pytest.mark.parametrize("margin,cells,n", [(0.5, 1 << 24, 20011), (0.0, 1 << 20, 3001), (2.0, 1 << 18, 3001),
+                                            (0.5, 1 << 9, 3001), (0.5, 1 << 24, 1), (0.5, 1 << 24, 17),
+                                            (0.5, 1 << 24, 33)])
+def test_march_equals_bvh(margin, cells, n):
+    tri, nrm, med = meshes.curved_abdomen(freq=14)
+    q = rays(n, np.random.default_rng(5))
+    got = []
+    for lists in (False, True):
+        with Simulation(0) as s:
+            s.set_mesh(tri, nrm, med)
+            s.set_safety_grid(cells)
+            s.set_cell_margin(margin)
+            s.set_cell_lists(lists)
+            got.append(s.query(*q))
+    assert np.array_equal(got[0][0], got[1][0])
+    assert np.array_equal(got[0][1].view(np.uint32), got[1][1].view(np.uint32))
+    if n > 1000:
+        assert (got[0][0] >= 0).mean() > 0.1
