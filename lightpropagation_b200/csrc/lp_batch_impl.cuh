@@ -31,7 +31,7 @@ struct WarpSlot {
 __device__ __forceinline__ void warp_flush_counters(const KParams &P, const Counters &c, uint32_t photons,
                                                     unsigned lane)
 {
-    const uint32_t v[10] = {c.scatter, c.boundary, c.query, c.roulette, c.rz_drop, c.vox_drop, photons, c.skip,
+    const uint32_t v[10] = {c.scatter(), c.boundary, c.query, c.roulette, c.rz_drop, c.vox_drop, photons, c.skip(),
                             c.bvh, 0u};
     const int slot[9] = {0, 1, 2, 3, 6, 7, 8, 10, 11};
 #pragma unroll
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_kernel(const __grid_constan
             }
         }
         const bool more = step_photon<Exact, Grad, STACK>(S.P, S.M, S.M, S.Q, S.media, S.P.region, S.P.counters, alive, ph,
-                                                          cnt, &ga);
+                                                          cnt, &ga, rz_copy_of(S.P));
         if (alive) {
             if (!more) {
                 if (ph.region_acc) atomicAdd(S.P.region + ph.curr, ph.region_acc);
@@ -155,6 +155,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_kernel(const __grid_constan
                     ga.k[ph.curr] += ph.seg_k;
                 }
                 finish_photon<Grad>(S.P, exit_state(ph), Grad ? &ga : nullptr);
+                cnt.steps += ph.steps;
                 photons++;
                 alive = false;
             }

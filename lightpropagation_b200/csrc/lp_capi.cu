@@ -424,8 +424,7 @@ void media_table(const float *nmuasg, int n_media, std::vector<Medium> &m)
         m[i].g = q[3];
         m[i].mut = q[1] + q[2];
         m[i].alb = q[1] / (q[1] + q[2]);
-        m[i].absorbs = (q[1] > 0.0f && q[2] > 0.0f) ? 1 : 0;
-        m[i].ambient = (q[1] == 0.0f && q[2] == 0.0f) ? 1 : 0;
+        m[i].kind = (q[1] > 0.0f && q[2] > 0.0f ? lp::kAbsorbs : 0u) | (q[1] == 0.0f && q[2] == 0.0f ? lp::kAmbient : 0u);
         m[i].inv_mut = (q[1] + q[2]) > 0.0f ? 1.0f / (q[1] + q[2]) : 0.0f;
         m[i].inv_mua = q[1] > 0.0f ? 1.0f / q[1] : 0.0f;
         const float g = q[3];
@@ -434,7 +433,6 @@ void media_table(const float *nmuasg, int n_media, std::vector<Medium> &m)
         m[i].hg_c = 2.0f * g;
         m[i].hg_d = 1.0f + g * g;
         m[i].hg_inv2g = g != 0.0f ? 1.0f / (2.0f * g) : 0.0f;
-        m[i].pad_ = 0.0f;
     }
 }
 
@@ -528,12 +526,11 @@ void fill_params(lp_ctx *c, KParams &P, int64_t first, int64_t n, int nodes_smem
     P.factor = c->factor;
     P.fetal_id = c->fetal_id;
     P.compat = c->compat;
-    P.key0 = (uint32_t)c->seed;
-    P.key1 = (uint32_t)(c->seed >> 32);
+    lp::set_keys(P, c->seed);
     P.stream = 0;
     P.first = first;
     P.n = n;
-    P.max_steps = c->max_steps;
+    P.step_cap = lp::step_cap_of(c->max_steps);
     const lp_geometry &g = c->geo;
     P.hx = g.dimx / 2; P.hy = g.dimy / 2; P.sft_nx = g.sft_nx;
     P.dimR = g.dimR; P.dimAlpha = g.dimAlpha; P.rz_nr = g.rz_nr; P.rz_nz = g.rz_nz;
@@ -543,6 +540,9 @@ void fill_params(lp_ctx *c, KParams &P, int64_t first, int64_t n, int nodes_smem
     P.inv_vdx = 1.0f / c->vox_d[0];
     P.inv_vdy = 1.0f / c->vox_d[1];
     P.inv_vdz = 1.0f / c->vox_d[2];
+    P.f_dimR = (float)g.dimR;
+    P.half_vnx = 0.5f * (float)c->vox_n[0];
+    P.half_vny = 0.5f * (float)c->vox_n[1];
     P.sft = c->sft.p; P.rtd = c->rtd.p; P.rz = c->rz.p; P.vox = c->vox.p; P.rbins = c->rbins.p;
     P.region = c->region.p; P.det = c->det.p; P.counters = c->counters.p;
     const int copies = rz_copies(rz_values(c));
@@ -580,9 +580,9 @@ void fill_params(lp_ctx *c, KParams &P, int64_t first, int64_t n, int nodes_smem
     P.g_oz = c->g_origin[2];
     P.g_inv_h = c->g_h > 0 ? 1.0f / c->g_h : 0.0f;
     P.g_unit = c->g_unit;
-    P.g_nx = c->g_n[0];
-    P.g_ny = c->g_n[1];
-    P.g_nz = c->g_n[2];
+    P.g_nx = grid ? c->g_n[0] : 0;
+    P.g_ny = grid ? c->g_n[1] : 0;
+    P.g_nz = grid ? c->g_n[2] : 0;
     P.g_h = c->g_h;
     P.g_margin = c->cell_margin * c->g_h;
     P.step_eps = c->g_step_eps;

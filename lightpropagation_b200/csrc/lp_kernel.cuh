@@ -19,17 +19,16 @@ constexpr float kNoHit = 10000.0f;   // FindTriangleInPath's initial distance (.
 // photons of one transport launch: the kernels index them with 32 bits
 constexpr int64_t kMaxLaunchPhotons = int64_t(1) << 31;
 
-struct Medium {
-    float n, mua, mus, g;
-    float mut;      // mua + mus
-    float alb;      // mua / (mua + mus)
-    int32_t absorbs;  // mua > 0 && mus > 0  (Absorb, .cl:841-847)
-    int32_t ambient;  // mua == 0 && mus == 0 (step = distance to boundary, .cl:1405-1410)
-    // precomputed factors of the fast arithmetic mode
-    float inv_mut, inv_mua;
-    float hg_a, hg_b, hg_c, hg_d, hg_inv2g;   // 1-g^2, 1-g, 2g, 1+g^2, 1/(2g)
-    float pad_;
+// The factors of one step sit together: two 16-byte loads in the production arithmetic.
+struct alignas(16) Medium {
+    float inv_mut, alb, inv_mua;   // 1 / (mua + mus), mua / (mua + mus), 1 / mua (0 for mua <= 0)
+    uint32_t kind;                 // kAbsorbs, kAmbient
+    float hg_a, hg_b, hg_c, hg_d;  // 1-g^2, 1-g, 2g, 1+g^2
+    float hg_inv2g, g, mua, mus;   // 1/(2g)
+    float n, mut, pad_[2];         // mut = mua + mus
 };
+constexpr uint32_t kAbsorbs = 1u;  // mua > 0 && mus > 0  (Absorb, .cl:841-847)
+constexpr uint32_t kAmbient = 2u;  // mua == 0 && mus == 0 (step = distance to boundary, .cl:1405-1410)
 
 struct KParams {
     // mesh (see lp_bvh.hpp)
@@ -53,12 +52,15 @@ struct KParams {
     float chance, w_th, factor;
     int32_t fetal_id;
     uint32_t compat;
-    uint32_t key0, key1, stream;
-    int64_t first, n, max_steps;
+    uint32_t key0[10], key1[10];     // Philox round keys (set_keys)
+    uint32_t stream;
+    uint32_t step_cap;               // steps after which a photon is stopped (step_cap_of)
+    int64_t first, n;
     // reference tally layout
     int32_t hx, hy, sft_nx, dimR, dimAlpha, rz_nr, rz_nz;
     float dg[6];
     float inv_dr, inv_dz, inv_vdx, inv_vdy, inv_vdz;   // reciprocals for the fast mode
+    float f_dimR, half_vnx, half_vny;                  // dimR, vox_nx / 2, vox_ny / 2
     // tallies (fixed point, 2^32 per unit weight)
     unsigned long long *sft, *rtd, *rz, *vox, *rbins, *region, *det, *counters;
     // where the r-z deposits go: rz_mask + 1 (a power of two) copies of the image, each of
@@ -135,17 +137,19 @@ constexpr uint32_t kCellEmpty = 0x80000000u;
 constexpr uint32_t kCellDense = 127u;
 constexpr uint32_t kCellOutside = 0x00010000u;
 
-// The cell word at p; points outside the grid read as an empty cell with bound 0 and
-// kCellOutside set.
+// The cell word at p; points outside the grid (every point when there is none: g_nx = 0)
+// read as an empty cell with bound 0 and kCellOutside set.  The grid has at most 2^28
+// cells, so 32-bit indices do.
 __device__ __forceinline__ uint32_t cell_at(const KParams &P, float px, float py, float pz)
 {
-    if (!P.cell_word) return kCellEmpty | kCellOutside;
     const int ix = (int)floorf((px - P.g_ox) * P.g_inv_h);
     const int iy = (int)floorf((py - P.g_oy) * P.g_inv_h);
     const int iz = (int)floorf((pz - P.g_oz) * P.g_inv_h);
-    if (ix < 0 || iy < 0 || iz < 0 || ix >= P.g_nx || iy >= P.g_ny || iz >= P.g_nz)
-        return kCellEmpty | kCellOutside;
-    return __ldg(P.cell_word + ((int64_t)iz * P.g_ny + iy) * P.g_nx + ix);
+    const bool in = ((unsigned)ix < (unsigned)P.g_nx) & ((unsigned)iy < (unsigned)P.g_ny) &
+                    ((unsigned)iz < (unsigned)P.g_nz);
+    uint32_t w = kCellEmpty | kCellOutside;
+    if (in) w = __ldg(P.cell_word + ((iz * P.g_ny + iy) * P.g_nx + ix));
+    return w;
 }
 
 // Distance from p to the nearest face of the cell containing it (0 outside the grid):
@@ -165,37 +169,70 @@ __device__ __forceinline__ float safe_distance(const KParams &P, uint32_t word)
 }
 
 // ----------------------------------------------------------------- Philox4x32-10
+__host__ __device__ __forceinline__ uint32_t philox_key0(uint32_t k0, int round)
+{
+    return k0 + 0x9E3779B9u * (uint32_t)round;
+}
+__host__ __device__ __forceinline__ uint32_t philox_key1(uint32_t k1, int round)
+{
+    return k1 + 0xBB67AE85u * (uint32_t)round;
+}
+
+// k0, k1: the ten round keys.  Kept in the kernel's parameters, they are operands of the
+// exclusive-ors instead of two additions a round; the 64-bit products give both halves of
+// a product in one instruction.
 __device__ __forceinline__ void philox4x32_10(uint32_t &c0, uint32_t &c1, uint32_t &c2, uint32_t &c3,
-                                              uint32_t k0, uint32_t k1)
+                                              const uint32_t *k0, const uint32_t *k1)
 {
 #pragma unroll
     for (int r = 0; r < 10; ++r) {
-        const uint32_t hi0 = __umulhi(0xD2511F53u, c0), lo0 = 0xD2511F53u * c0;
-        const uint32_t hi1 = __umulhi(0xCD9E8D57u, c2), lo1 = 0xCD9E8D57u * c2;
-        const uint32_t n0 = hi1 ^ c1 ^ k0, n2 = hi0 ^ c3 ^ k1;
+        const uint64_t p0 = (uint64_t)0xD2511F53u * c0, p1 = (uint64_t)0xCD9E8D57u * c2;
+        const uint32_t n0 = (uint32_t)(p1 >> 32) ^ c1 ^ k0[r], n2 = (uint32_t)(p0 >> 32) ^ c3 ^ k1[r];
         c0 = n0;
-        c1 = lo1;
+        c1 = (uint32_t)p1;
         c2 = n2;
-        c3 = lo0;
-        k0 += 0x9E3779B9u;
-        k1 += 0xBB67AE85u;
+        c3 = (uint32_t)p0;
     }
+}
+
+// The seed's round keys.
+__host__ __device__ inline void set_keys(KParams &P, uint64_t seed)
+{
+    for (int r = 0; r < 10; ++r) {
+        P.key0[r] = philox_key0((uint32_t)seed, r);
+        P.key1[r] = philox_key1((uint32_t)(seed >> 32), r);
+    }
+}
+
+// max_steps (<= 0: none) as the kernel's 32-bit cap; a photon's steps are counted in 32 bits
+__host__ __device__ inline uint32_t step_cap_of(int64_t max_steps)
+{
+    return max_steps <= 0 || max_steps > (int64_t)0xffffffff ? 0xffffffffu : (uint32_t)max_steps;
+}
+
+// ((x >> 8) | 1) * 2^-24, a uniform in (0, 1) that is never 0.  (x >> 8) | 1 is 2 k + 1
+// with k = x >> 9, so the value is k 2^-23 + 2^-24: k goes into the mantissa of a float
+// in [2^23, 2^24), and one exact fused multiply-add does the rest (no conversion).
+__device__ __forceinline__ float uniform24(uint32_t x)
+{
+    return __fmaf_rn(__uint_as_float(0x4B000000u | (x >> 9)), 0x1.0p-23f, -0x1.fffffep-1f);
 }
 
 // One Philox block per event: counter (photon lo, photon hi, event, stream), key =
 // seed.  Event 0 samples the source, loop iteration i is event i + 1.  The four words
 // are the event's draw slots (step, Fresnel or polar angle, azimuth, roulette), each
-// mapped to ((x >> 8) | 1) * 2^-24, a uniform in (0, 1) that is never 0.
+// mapped to a uniform by uniform24.
 struct EventRng {
     float u0, u1, u2, u3;
-    __device__ __forceinline__ void draw(uint64_t pid, uint32_t event, uint32_t stream, uint32_t k0, uint32_t k1)
+    __device__ __forceinline__ void draw(const KParams &P, uint32_t idx, uint32_t event)
     {
-        uint32_t c0 = (uint32_t)pid, c1 = (uint32_t)(pid >> 32), c2 = event, c3 = stream;
-        philox4x32_10(c0, c1, c2, c3, k0, k1);
-        u0 = __uint2float_rn((c0 >> 8) | 1u) * 0x1.0p-24f;
-        u1 = __uint2float_rn((c1 >> 8) | 1u) * 0x1.0p-24f;
-        u2 = __uint2float_rn((c2 >> 8) | 1u) * 0x1.0p-24f;
-        u3 = __uint2float_rn((c3 >> 8) | 1u) * 0x1.0p-24f;
+        const uint64_t pid = (uint64_t)(P.first + (int64_t)idx);
+        uint32_t c0 = (uint32_t)pid, c1 = (uint32_t)(pid >> 32), c2 = event, c3 = P.stream;
+        philox4x32_10(c0, c1, c2, c3, P.key0, P.key1);
+        u0 = uniform24(c0);
+        u1 = uniform24(c1);
+        u2 = uniform24(c2);
+        u3 = uniform24(c3);
     }
 };
 

@@ -91,8 +91,7 @@ __global__ void __launch_bounds__(256) noalloc_setup_kernel(const float *tri, co
         m.n = q.x; m.mua = q.y; m.mus = q.z; m.g = q.w;
         m.mut = __fadd_rn(q.y, q.z);
         m.alb = __fdiv_rn(q.y, m.mut);
-        m.absorbs = (q.y > 0.0f && q.z > 0.0f) ? 1 : 0;
-        m.ambient = (q.y == 0.0f && q.z == 0.0f) ? 1 : 0;
+        m.kind = (q.y > 0.0f && q.z > 0.0f ? kAbsorbs : 0u) | (q.y == 0.0f && q.z == 0.0f ? kAmbient : 0u);
         m.inv_mut = m.mut > 0.0f ? __fdiv_rn(1.0f, m.mut) : 0.0f;
         m.inv_mua = q.y > 0.0f ? __fdiv_rn(1.0f, q.y) : 0.0f;
         m.hg_a = __fsub_rn(1.0f, __fmul_rn(q.w, q.w));
@@ -100,7 +99,7 @@ __global__ void __launch_bounds__(256) noalloc_setup_kernel(const float *tri, co
         m.hg_c = __fmul_rn(2.0f, q.w);
         m.hg_d = __fadd_rn(1.0f, __fmul_rn(q.w, q.w));
         m.hg_inv2g = q.w != 0.0f ? __fdiv_rn(1.0f, __fmul_rn(2.0f, q.w)) : 0.0f;
-        m.pad_ = 0.0f;
+        m.pad_[0] = m.pad_[1] = 0.0f;
         media[i] = m;
     }
     __shared__ float s_b[6][256];
@@ -328,17 +327,17 @@ extern "C" int lp_run_noalloc(const lp_noalloc_args *a, void *stream)
     P.factor = a->factor;
     P.fetal_id = a->fetal_id;
     P.compat = a->compat & LP_COMPAT_ALL;
-    P.key0 = (uint32_t)a->seed;
-    P.key1 = (uint32_t)(a->seed >> 32);
+    set_keys(P, a->seed);
     P.first = a->first;
     P.n = a->n_photons;
-    P.max_steps = LP_NOALLOC_MAX_STEPS;
+    P.step_cap = step_cap_of(LP_NOALLOC_MAX_STEPS);
     P.hx = dimx / 2; P.hy = dimy / 2; P.sft_nx = 2 * (dimx / 2) + 1;
     P.dimR = dimR; P.dimAlpha = dimAlpha; P.rz_nr = 2 * dimR + 1; P.rz_nz = dimz + 1;
     for (int i = 0; i < 6; ++i) P.dg[i] = a->det_grid[i];
     P.inv_dr = 1.0f / a->det_grid[3];
     P.inv_dz = 1.0f / a->det_grid[2];
     P.inv_vdx = P.inv_vdy = P.inv_vdz = 1.0f;
+    P.f_dimR = (float)dimR;
     P.sft = reinterpret_cast<unsigned long long *>(a->sft);
     P.rtd = reinterpret_cast<unsigned long long *>(a->rtd);
     P.rz = reinterpret_cast<unsigned long long *>(a->rz);

@@ -74,8 +74,13 @@ __global__ void philox_kernel(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3
 {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
-        uint32_t a = c0, b = c1, c = c2 + (uint32_t)i, d = c3;
-        philox4x32_10(a, b, c, d, k0, k1);
+        uint32_t a = c0, b = c1, c = c2 + (uint32_t)i, d = c3, r0[10], r1[10];
+#pragma unroll
+        for (int r = 0; r < 10; ++r) {
+            r0[r] = philox_key0(k0, r);
+            r1[r] = philox_key1(k1, r);
+        }
+        philox4x32_10(a, b, c, d, r0, r1);
         out[4 * i] = a; out[4 * i + 1] = b; out[4 * i + 2] = c; out[4 * i + 3] = d;
     }
 }

@@ -9,13 +9,25 @@
 // which thread traced which photon; every loop iteration computes exactly one block,
 // which keeps the warp converged on the RNG.
 //
-// Per loop iteration (MCLightPropagation.cl:1375-1575):
-//   step length (.cl:1405-1442) -> nearest triangle within the step through the BVH
-//   (replaces the O(T) FindTriangleInPath, .cl:1037-1093) -> boundary
-//   (TransmitOrReflect, .cl:921-1018) or absorb + Henyey-Greenstein scatter +
-//   absorption tallies (.cl:1513-1537) -> roulette (.cl:1539-1545).
+// Per loop iteration (MCLightPropagation.cl:1375-1575), the warp's lanes together:
+//   step length (.cl:1405-1442) -> nearest triangle within the step (replaces the O(T)
+//   FindTriangleInPath, .cl:1037-1093; skipped by distance bounds, or answered by the
+//   whole warp from the cell lists) -> boundary (TransmitOrReflect, .cl:921-1018) or
+//   absorb + Henyey-Greenstein scatter + absorption tallies (.cl:1513-1537) -> roulette
+//   (.cl:1539-1545).
 // At the end of a photon its exit record (.cl:1583-1594) is binned on the device into
 // the reference's SFT and RTd images (CalculatePropagation.cpp:1553-1626).
+//
+// What bounds it: the instructions of one step, about 500 of them in one chain that
+// branches on its own results.  A warp with one photon left issues one every 4.7 cycles
+// (fixed latencies and the special-function unit, 2,600 cycles a step), so short runs
+// and the ends of long ones wait for their longest photon; full warps (24 per SM at 80
+// registers) issue two cycles of three.  Hence the form of the step: selects instead of
+// branches where both sides are a few operations, round keys and derived constants in
+// the kernel's parameters, 32-bit indices, one 16-byte load for a medium's factors, and
+// no counter that another one implies.  Against the same step without these: slab, 1e6
+// photons, 114 -> 99 ms; curved abdomen at 660 nm, 3e6 photons, 201 -> 181 ms; 1e5
+// photons 40 -> 34 ms.
 //
 // Exact = true  keeps the reference's arithmetic operation by operation (compiled
 //               with --fmad=false): a photon follows the oracle's trajectory for the
@@ -43,11 +55,11 @@ constexpr int kBlock = 256;
 
 struct Photon {
     float px, py, pz, vx, vy, vz;
-    float w, unfin, absorbed;
+    float w, unfin;          // unfin: residual step; the exit weight once the photon has left
+    float absorbed;
     int32_t last_tri;        // face of the last boundary event, -1 before any: its normal is
                              // CalcAlphaOut's (.cl:1583), see photon_normal
-    float exit_w;            // exit weight once scored
-    int32_t curr, refTri;
+    int32_t curr;
     uint32_t steps;
     uint32_t flags;          // see F_*, EXIT_SHIFT, AXIS_SHIFT
     unsigned long long region_acc;
@@ -63,13 +75,19 @@ struct GradAcc {
     float L[kGradRegions];
     uint32_t k[kGradRegions];
 };
-// flags: bit 0 traversedFetalTissue, bit 1 roulette, bits 2-3 exit kind, bits 4-5 the
-// on-axis normal override at the last boundary (0 none, 1 +eZ, 2 -eZ, 3 zero vector)
-enum : uint32_t { F_FETAL = 1u, F_ROULETTE = 2u, EXIT_SHIFT = 2, AXIS_SHIFT = 4 };
+// flags: bit 0 traversedFetalTissue, bit 1 the photon is on last_tri (refTri of the
+// reference: no scattering since the boundary event), bits 2-3 exit kind, bits 4-5 the
+// on-axis normal override at the last boundary (0 none, 1 +eZ, 2 -eZ, 3 zero vector).
+// The reference's roulette flag is left out: it is clear only when the weight is 0.
+enum : uint32_t { F_FETAL = 1u, F_ON_FACE = 2u, EXIT_SHIFT = 2, AXIS_SHIFT = 4 };
 enum : uint32_t { EXIT_NONE = 0, EXIT_SURF = 1, EXIT_SURF_FETAL = 2, EXIT_TRANS = 3 };
 
+// steps: of the finished photons.  Each step is a scatter or a boundary event, and has a
+// query or skips it, so the other two counts follow.
 struct Counters {
-    uint32_t scatter, boundary, query, roulette, rz_drop, vox_drop, skip, bvh;
+    uint32_t steps, boundary, query, roulette, rz_drop, vox_drop, bvh;
+    __device__ __forceinline__ uint32_t scatter() const { return steps - boundary; }
+    __device__ __forceinline__ uint32_t skip() const { return steps - query; }
 };
 
 template <bool Exact>
@@ -83,12 +101,10 @@ __device__ __forceinline__ float hg_cos_theta(const Medium &m, float xi)
         if (g != 0.0f) cosTheta = (1.0f + g * g - g1 * g1) / (2.0f * g);
         else cosTheta = 2.0f * xi - 1.0f;
     } else {
-        if (m.g != 0.0f) {
-            const float g1 = __fdividef(m.hg_a, __fmaf_rn(m.hg_c, xi, m.hg_b));
-            cosTheta = __fmaf_rn(-g1, g1, m.hg_d) * m.hg_inv2g;
-        } else {
-            cosTheta = __fmaf_rn(2.0f, xi, -1.0f);
-        }
+        // both cases and a select: the step loop pays more for a branch
+        const float g1 = __fdividef(m.hg_a, __fmaf_rn(m.hg_c, xi, m.hg_b));
+        cosTheta = __fmaf_rn(-g1, g1, m.hg_d) * m.hg_inv2g;
+        if (m.hg_c == 0.0f) cosTheta = __fmaf_rn(2.0f, xi, -1.0f);
     }
     return fminf(fmaxf(cosTheta, -1.0f), 1.0f);
 }
@@ -139,18 +155,19 @@ __device__ __forceinline__ V3 scatter_direction(V3 v, const Medium &m, float xt,
         const float sinTheta = sqrtf(fmaxf(0.0f, __fmaf_rn(-cosTheta, cosTheta, 1.0f)));
         float sinPsi, cosPsi;
         sincospif(2.0f * xp, &sinPsi, &cosPsi);
-        V3 r;
         const float uz2 = __fmaf_rn(v.x, v.x, v.y * v.y);
-        if (uz2 < 1e-20f) {
-            r = v3(sinTheta * cosPsi, sinTheta * sinPsi, v.z > 0.0f ? cosTheta : -cosTheta);
-        } else {
-            const float it = rsqrtf(uz2);
-            const float temp = uz2 * it;  // sqrt(1 - uz^2)
-            const float st = sinTheta * it;
-            r = v3(__fmaf_rn(st, __fmaf_rn(v.x * v.z, cosPsi, -v.y * sinPsi), v.x * cosTheta),
-                   __fmaf_rn(st, __fmaf_rn(v.y * v.z, cosPsi, v.x * sinPsi), v.y * cosTheta),
-                   __fmaf_rn(-sinTheta * cosPsi, temp, v.z * cosTheta));
-        }
+        const float it = rsqrtf(uz2);
+        const float temp = uz2 * it;  // sqrt(1 - uz^2)
+        const float st = sinTheta * it;
+        const float ax = sinTheta * cosPsi;
+        V3 r = v3(__fmaf_rn(st, __fmaf_rn(v.x * v.z, cosPsi, -v.y * sinPsi), v.x * cosTheta),
+                  __fmaf_rn(st, __fmaf_rn(v.y * v.z, cosPsi, v.x * sinPsi), v.y * cosTheta),
+                  __fmaf_rn(-ax, temp, v.z * cosTheta));
+        // the axial case by selects (it and temp are not finite there): a branch costs more
+        const bool axial = uz2 < 1e-20f;
+        r.x = axial ? ax : r.x;
+        r.y = axial ? sinTheta * sinPsi : r.y;
+        r.z = axial ? (v.z > 0.0f ? cosTheta : -cosTheta) : r.z;
         return fast_norm(r);
     }
 }
@@ -220,8 +237,9 @@ static __device__ __noinline__ void score_gradient(const KParams &P, const GradA
     }
 }
 
-// What an exit record needs of a photon, passed by value: a reference would take the photon's address out of the step loop, and every
-// step would then store it to local memory.
+// What an exit record needs of a photon, passed by value: a reference would take the
+// photon's address out of the step loop, and every step would then store it to local
+// memory.
 struct ExitState {
     float px, py, pz, vx, vy, vz, exit_w;
     int32_t last_tri;
@@ -229,7 +247,7 @@ struct ExitState {
 };
 __device__ __forceinline__ ExitState exit_state(const Photon &ph)
 {
-    return ExitState{ph.px, ph.py, ph.pz, ph.vx, ph.vy, ph.vz, ph.exit_w, ph.last_tri, ph.flags, ph.idx};
+    return ExitState{ph.px, ph.py, ph.pz, ph.vx, ph.vy, ph.vz, ph.unfin, ph.last_tri, ph.flags, ph.idx};
 }
 
 // The normal of the photon's last boundary event as the transport used it: the face's unit
@@ -309,7 +327,6 @@ static __device__ __noinline__ void finish_photon(const KParams &P, const ExitSt
 
 __device__ __forceinline__ void start_photon(const KParams &P, Photon &ph, uint32_t idx)
 {
-    const int64_t pid = P.first + (int64_t)idx;
     // PhotonClass::Init (.cl:344-389) with vStart[0] (.cl:429-467)
     ph.px = P.p0x; ph.py = P.p0y; ph.pz = P.p0z;
     ph.vx = P.v0x; ph.vy = P.v0y; ph.vz = P.v0z;
@@ -317,7 +334,7 @@ __device__ __forceinline__ void start_photon(const KParams &P, Photon &ph, uint3
         // fibre source (no reference counterpart), event 0: disk of radius src_radius in
         // the (eX, eY) plane, direction uniform in solid angle within the cone about eZ
         EventRng rng;
-        rng.draw((uint64_t)pid, 0u, P.stream, P.key0, P.key1);
+        rng.draw(P, idx, 0u);
         const V3 ex = v3(P.nxx, P.nxy, P.nxz), ey = v3(P.nyx, P.nyy, P.nyz), ez = v3(P.nzx, P.nzy, P.nzz);
         const float r = P.src_radius * sqrtf(rng.u0);
         const float phi = 2.0f * 3.14159265358979323846f * rng.u1;
@@ -335,11 +352,9 @@ __device__ __forceinline__ void start_photon(const KParams &P, Photon &ph, uint3
     ph.unfin = 0.0f;
     ph.absorbed = 0.0f;
     ph.last_tri = -1;
-    ph.exit_w = 0.0f;
     ph.curr = 0;
-    ph.refTri = -1;
     ph.steps = 0;
-    ph.flags = F_ROULETTE;
+    ph.flags = 0;
     ph.region_acc = 0;
     ph.idx = idx;
     ph.seg_len = 0.0f;
@@ -367,7 +382,7 @@ static __device__ __forceinline__ Photon boundary_event(const KParams &P, const 
     ph.px = ph.px + thit * ph.vx;
     ph.py = ph.py + thit * ph.vy;
     ph.pz = ph.pz + thit * ph.vz;
-    ph.refTri = -1;
+    ph.flags &= ~F_ON_FACE;
     if (tri < 0) {
         // the reference would read mediumIDs[-1] here; the photon leaves the model
         atomicAdd(s_cnt + 4, 1ull);
@@ -458,21 +473,24 @@ static __device__ __forceinline__ Photon boundary_event(const KParams &P, const 
             ph.py = __fmaf_rn(sp, nv.y, ph.py);
             ph.pz = __fmaf_rn(sp, nv.z, ph.pz);
         }
-        if (muaNew == 0.0f || musNew == 0.0f) {
+        float exit_w = 0.0f;
+        const bool leaves = muaNew == 0.0f || musNew == 0.0f;
+        if (leaves) {
             const float dist = fabsf(dot3(v3(P.nzx, P.nzy, P.nzz),
                                           v3(ph.px - P.poix, ph.py - P.poiy, ph.pz - P.poiz)));
             uint32_t kind;
             if (dist > P.distMin) kind = EXIT_TRANS;
             else kind = (ph.flags & F_FETAL) ? EXIT_SURF_FETAL : EXIT_SURF;
-            ph.exit_w = ph.w * P.exitScale;
+            exit_w = ph.w * P.exitScale;
             ph.flags = (ph.flags & ~(3u << EXIT_SHIFT)) | (kind << EXIT_SHIFT);
             ph.w = 0.0f;
         }
         const int prev = ph.curr;
         ph.curr = newID;
-        ph.refTri = tri;
+        ph.flags |= F_ON_FACE;
         if (newID == P.fetal_id) ph.flags |= F_FETAL;
         ph.unfin = Exact ? (step - thit) * m.mut : fmaxf(step - thit, 0.0f) * m.mut;
+        if (leaves) ph.unfin = exit_w;
         if (newID != prev) {
             if (ph.region_acc) atomicAdd(s_region + prev, ph.region_acc);
             ph.region_acc = 0;
@@ -510,31 +528,28 @@ enum : int { kStepEnded = 0, kStepClear = 1, kStepQuery = 2 };
 // lies within its reach (complete_step with tri = -1); kStepEnded: the photon ended
 // (debug build: a region id out of range).
 template <bool Exact>
-__device__ __forceinline__ int propose_step(const KParams &P, const Medium *s_media, Photon &ph, Counters &cnt,
-                                            Pending &pd)
+__device__ __forceinline__ int propose_step(const KParams &P, const Medium *s_media, Photon &ph, Pending &pd)
 {
     // The cell word is read on every step, its load issued before the Philox rounds so
     // that they hide its latency (reading it only when the carried bound is used up saves
     // loads but waits on them: 1.3 % slower on the 660 nm abdomen).
     const uint32_t word = cell_at(P, ph.px, ph.py, ph.pz);
     EventRng rng;
-    rng.draw((uint64_t)(P.first + (int64_t)ph.idx), ph.steps + 1u, P.stream, P.key0, P.key1);
+    rng.draw(P, ph.idx, ph.steps + 1u);
     [[maybe_unused]] unsigned long long *const dbg = P.counters ? P.counters + kBoundsCounter : nullptr;
     if (!LP_IN_RANGE(dbg, ph.curr, P.n_media)) {
         ph.w = 0.0f;
         return kStepEnded;
     }
-    const Medium m = s_media[ph.curr];
-    float step = 0.0f;
-    if (!m.ambient) {
-        if (ph.unfin == 0.0f) {
-            if (Exact) step = -logf(rng.u0) * P.factor / m.mut;
-            else step = -logf(rng.u0) * P.factor * m.inv_mut;
-        } else {
-            step = Exact ? ph.unfin / m.mut : ph.unfin * m.inv_mut;
-            ph.unfin = 0.0f;
-        }
-    }
+    const Medium &m = s_media[ph.curr];
+    const bool ambient = (m.kind & kAmbient) != 0;
+    // the residual of a step cut short by a boundary, or a new step; both are formed, and
+    // the select costs less than the branch
+    float step;
+    if (Exact) step = (ph.unfin == 0.0f) ? -logf(rng.u0) * P.factor / m.mut : ph.unfin / m.mut;
+    else step = (ph.unfin == 0.0f) ? -logf(rng.u0) * P.factor * m.inv_mut : ph.unfin * m.inv_mut;
+    if (ambient) step = 0.0f;
+    ph.unfin = 0.0f;
     pd.step = step;
     // reach: the production arithmetic also takes a face that lies up to a few rounding
     // units beyond the step as the step's boundary.  A hit computed just past the step
@@ -551,21 +566,12 @@ __device__ __forceinline__ int propose_step(const KParams &P, const Medium *s_me
     // after the step the bound shrinks by the step (plus the rounding of the move).
     pd.safe_here = ph.safe;
     pd.word = word;
-    if (m.ambient) return kStepQuery;
-    if (reach < pd.safe_here) {
-        cnt.skip++;
-        return kStepClear;
-    }
-    if (word & kCellEmpty) {
-        // a cell no triangle touches: its word holds a bound for all its points (the
-        // larger of two lower bounds is one too)
-        pd.safe_here = fmaxf(pd.safe_here, safe_distance(P, word));
-        if (reach < pd.safe_here) {
-            cnt.skip++;
-            return kStepClear;
-        }
-    }
-    return kStepQuery;
+    if (ambient) return kStepQuery;
+    if (reach < pd.safe_here) return kStepClear;
+    // a cell no triangle touches: its word holds a bound for all its points (the larger of
+    // two lower bounds is one too); safe_distance is 0 for the others
+    pd.safe_here = fmaxf(pd.safe_here, safe_distance(P, word));
+    return reach < pd.safe_here ? kStepClear : kStepQuery;
 }
 
 // The nearest triangle within the step's reach (-1: none) and its distance thit; updates
@@ -573,52 +579,53 @@ __device__ __forceinline__ int propose_step(const KParams &P, const Medium *s_me
 // whose step needs a query with `want`.
 template <int STACK>
 __device__ __forceinline__ int query_step(const KParams &P, const MeshView &M, const MeshView &SM, WarpQueue &Q,
-                                          const Medium *s_media, bool want, const Photon &ph, Counters &cnt, Pending &pd, float &thit)
+                                          const Medium *s_media, bool want, const Photon &ph, Counters &cnt,
+                                          Pending &pd, float &thit)
 {
     thit = kNoHit;
     if (!__any_sync(0xffffffffu, want)) return -1;
-    const bool ambient = want && s_media[ph.curr].ambient;
+    const bool ambient = want && (s_media[ph.curr].kind & kAmbient);
     bool used_bvh;
     // an empty cell: pd.safe_here holds its bound, which the step exceeds; a listed cell
     // raises it from the planes of its triangles when its list decides the step
     const int tri = warp_query<STACK>(P, M, SM, Q, want, v3(ph.px, ph.py, ph.pz), v3(ph.vx, ph.vy, ph.vz),
-                                      ph.refTri, ambient ? kNoHit : pd.reach, pd.word, thit, pd.safe_here, used_bvh);
+                                      (ph.flags & F_ON_FACE) ? ph.last_tri : -1, ambient ? kNoHit : pd.reach, pd.word,
+                                      thit, pd.safe_here, used_bvh);
     cnt.query += want ? 1u : 0u;
     cnt.bvh += used_bvh ? 1u : 0u;
     return tri;
 }
 
 // Returns false when the photon ends.  Agg: absorption deposits summed per cell across
-// the warp before the atomic adds.
+// the warp before the atomic adds.  rz_copy: first cell of the block's copy of the r-z
+// image (rz_copy_of).
 template <bool Exact, bool Grad, bool Agg = false>
 __device__ __forceinline__ bool complete_step(const KParams &P, const Medium *s_media, unsigned long long *s_region,
                                               unsigned long long *s_cnt, Photon &ph, Counters &cnt, GradAcc *ga,
-                                              const Pending &pd, int tri, float thit)
+                                              const Pending &pd, int tri, float thit, uint32_t rz_copy)
 {
-    const Medium m = s_media[ph.curr];
+    const Medium &m = s_media[ph.curr];
+    const bool ambient = (m.kind & kAmbient) != 0;
     const V3 v = v3(ph.vx, ph.vy, ph.vz);
-    float step = pd.step;
-    const float reach = pd.reach, safe_here = pd.safe_here;
-    if (m.ambient) step = thit;
-    const bool boundary = (tri >= 0) ? (thit <= (m.ambient ? step : reach)) : (kNoHit <= step);
+    const float step = ambient ? thit : pd.step;
+    // a query returns no hit beyond the step's reach
+    const bool boundary = tri >= 0 || kNoHit <= step;
     if (boundary) {
         cnt.boundary++;
         ph = boundary_event<Exact, Grad>(P, s_media, s_region, s_cnt, ph, Grad ? ga : nullptr, tri, thit, step, pd.u1);
     } else {
-        cnt.scatter++;
         ph.px = ph.px + step * ph.vx;
         ph.py = ph.py + step * ph.vy;
         ph.pz = ph.pz + step * ph.vz;
-        ph.refTri = -1;
-        ph.safe = fmaxf(safe_here - step - P.step_eps, 0.0f);
+        ph.flags &= ~F_ON_FACE;
+        ph.safe = fmaxf(pd.safe_here - step - P.step_eps, 0.0f);
         if (Grad) {
             ph.seg_len += step;
             ph.seg_k++;
         }
-        if (m.absorbs) {
-            ph.absorbed = ph.w * m.alb;
-            ph.w -= ph.absorbed;
-        }
+        const bool absorbs = (m.kind & kAbsorbs) != 0;
+        ph.absorbed = absorbs ? ph.w * m.alb : ph.absorbed;
+        ph.w = absorbs ? ph.w - ph.absorbed : ph.w;
         const V3 vn = scatter_direction<Exact>(v, m, pd.u1, pd.u2);
         ph.vx = vn.x; ph.vy = vn.y; ph.vz = vn.z;
         const V3 pr = v3(ph.px - P.poix, ph.py - P.poiy, ph.pz - P.poiz);
@@ -632,34 +639,35 @@ __device__ __forceinline__ bool complete_step(const KParams &P, const Medium *s_
         if (Exact) {
             const float rad = sqrtf(cx * cx + cy * cy) * sign_cl(cx) / P.dg[3];
             row = (int)floorf(cz / P.dg[2]);
-            col = (int)floorf(rad + (float)P.dimR);
+            col = (int)floorf(rad + P.f_dimR);
         } else {
             const float rad = copysignf(sqrtf(cx * cx + cy * cy), cx) * P.inv_dr;
             row = (int)floorf(cz * P.inv_dz);
-            col = (int)floorf(rad + (float)P.dimR);
+            col = (int)floorf(rad + P.f_dimR);
         }
-        const bool rz_in = row >= 0 && row < P.rz_nz && col >= 0 && col < P.rz_nr;
-        const unsigned long long fdm = (m.mua > 0.0f) ? fix32(Exact ? dw / m.mua : dw * m.inv_mua) : 0ull;
+        const bool rz_in = ((unsigned)row < (unsigned)P.rz_nz) & ((unsigned)col < (unsigned)P.rz_nr);
+        // inv_mua is 0 where mua is not positive
+        const unsigned long long fdm = Exact ? (m.mua > 0.0f ? fix32(dw / m.mua) : 0ull) : fix32(dw * m.inv_mua);
         int vox_key = -1;
         if (P.vox_nx > 0) {
             int ix, iy, iz;
             if (Exact) {
-                ix = (int)floorf(cx / P.vox_dx + 0.5f * (float)P.vox_nx);
-                iy = (int)floorf(cy / P.vox_dy + 0.5f * (float)P.vox_ny);
+                ix = (int)floorf(cx / P.vox_dx + P.half_vnx);
+                iy = (int)floorf(cy / P.vox_dy + P.half_vny);
                 iz = (int)floorf(cz / P.vox_dz);
             } else {
-                ix = (int)floorf(cx * P.inv_vdx + 0.5f * (float)P.vox_nx);
-                iy = (int)floorf(cy * P.inv_vdy + 0.5f * (float)P.vox_ny);
+                ix = (int)floorf(cx * P.inv_vdx + P.half_vnx);
+                iy = (int)floorf(cy * P.inv_vdy + P.half_vny);
                 iz = (int)floorf(cz * P.inv_vdz);
             }
-            if (ix >= 0 && ix < P.vox_nx && iy >= 0 && iy < P.vox_ny && iz >= 0 && iz < P.vox_nz)
-                vox_key = (iz * P.vox_ny + iy) * P.vox_nx + ix;
-            else
-                cnt.vox_drop++;
+            const bool vox_in = ((unsigned)ix < (unsigned)P.vox_nx) & ((unsigned)iy < (unsigned)P.vox_ny) &
+                                ((unsigned)iz < (unsigned)P.vox_nz);
+            vox_key = vox_in ? (iz * P.vox_ny + iy) * P.vox_nx + ix : -1;
+            cnt.vox_drop += vox_in ? 0u : 1u;
         }
-        if (!rz_in) cnt.rz_drop++;
+        cnt.rz_drop += rz_in ? 0u : 1u;
         const int rz_key = rz_in ? row * P.rz_nr + col : -1;
-        unsigned long long *const rz = P.rz_part + (int64_t)(blockIdx.x & P.rz_mask) * P.rz_stride;
+        unsigned long long *const rz = P.rz_part + 2 * (int64_t)rz_copy;
         if (Agg) {
             // warp-aggregated deposits: the lanes of this branch that hit the same cell
             // are matched, their fixed-point values summed exactly, and one leader per
@@ -695,18 +703,21 @@ __device__ __forceinline__ bool complete_step(const KParams &P, const Medium *s_
         cnt.roulette++;
         if (pd.u3 < P.chance) {
             ph.w /= P.chance;
-            ph.flags |= F_ROULETTE;
         } else {
             ph.w = 0.0f;
-            ph.flags &= ~F_ROULETTE;
         }
     }
     ph.steps++;
-    if (P.max_steps > 0 && (int64_t)ph.steps >= P.max_steps && ph.w > 0.0f) {
+    if (ph.steps >= P.step_cap && ph.w > 0.0f) {
         atomicAdd(s_cnt + 5, 1ull);
         ph.w = 0.0f;
     }
-    return ph.w > 0.0f && (ph.w > P.w_th || (ph.flags & F_ROULETTE));
+    return ph.w > 0.0f;
+}
+
+__device__ __forceinline__ uint32_t rz_copy_of(const KParams &P)
+{
+    return (blockIdx.x & P.rz_mask) * (uint32_t)(P.rz_stride >> 1);
 }
 
 // One iteration of the reference's do-while loop, the three parts in turn, for the warp's
@@ -714,16 +725,17 @@ __device__ __forceinline__ bool complete_step(const KParams &P, const Medium *s_
 // lane's photon ends.
 template <bool Exact, bool Grad, int STACK = kStackDepth, bool Agg = false>
 __device__ __forceinline__ bool step_photon(const KParams &P, const MeshView &M, const MeshView &SM, WarpQueue &Q,
-                                            const Medium *s_media, unsigned long long *s_region, unsigned long long *s_cnt, bool alive,
-                                            Photon &ph, Counters &cnt, GradAcc *ga)
+                                            const Medium *s_media, unsigned long long *s_region,
+                                            unsigned long long *s_cnt, bool alive, Photon &ph, Counters &cnt,
+                                            GradAcc *ga, uint32_t rz_copy)
 {
     Pending pd;
     int st = kStepEnded;
-    if (alive) st = propose_step<Exact>(P, s_media, ph, cnt, pd);
+    if (alive) st = propose_step<Exact>(P, s_media, ph, pd);
     float thit;
     const int tri = query_step<STACK>(P, M, SM, Q, s_media, st == kStepQuery, ph, cnt, pd, thit);
     if (st == kStepEnded) return false;
-    return complete_step<Exact, Grad, Agg>(P, s_media, s_region, s_cnt, ph, cnt, ga, pd, tri, thit);
+    return complete_step<Exact, Grad, Agg>(P, s_media, s_region, s_cnt, ph, cnt, ga, pd, tri, thit, rz_copy);
 }
 
 struct SmemLayout {
@@ -798,6 +810,7 @@ __global__ void __launch_bounds__(kBlock, LP_TRANSPORT_MIN_BLOCKS) transport_ker
 
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lt_mask = (1u << lane) - 1u;
+    const uint32_t rz_copy = rz_copy_of(P);
     Counters cnt = {};
     uint32_t photons = 0;
     Photon ph;
@@ -827,8 +840,9 @@ __global__ void __launch_bounds__(kBlock, LP_TRANSPORT_MIN_BLOCKS) transport_ker
             }
         }
         if (!__any_sync(0xffffffffu, alive)) break;
-        const bool more = step_photon<Exact, Grad, kStackDepth, Agg>(P, M, shared_view, queues[threadIdx.x >> 5], s_media, s_region,
-                                                                     s_cnt, alive, ph, cnt, &ga);
+        const bool more = step_photon<Exact, Grad, kStackDepth, Agg>(P, M, shared_view, queues[threadIdx.x >> 5],
+                                                                     s_media, s_region, s_cnt, alive, ph, cnt, &ga,
+                                                                     rz_copy);
         if (alive) {
             if (!more) {
                 if (ph.region_acc) atomicAdd(s_region + ph.curr, ph.region_acc);
@@ -837,13 +851,14 @@ __global__ void __launch_bounds__(kBlock, LP_TRANSPORT_MIN_BLOCKS) transport_ker
                     ga.k[ph.curr] += ph.seg_k;
                 }
                 finish_photon<Grad>(P, exit_state(ph), Grad ? &ga : nullptr);
+                cnt.steps += ph.steps;
                 photons++;
                 alive = false;
             }
         }
     }
     // block-level reduction of counters and region sums
-    const uint32_t cv[8] = {cnt.scatter, cnt.boundary, cnt.query, cnt.roulette, 0u, 0u, cnt.rz_drop, cnt.vox_drop};
+    const uint32_t cv[8] = {cnt.scatter(), cnt.boundary, cnt.query, cnt.roulette, 0u, 0u, cnt.rz_drop, cnt.vox_drop};
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         if (i == 4 || i == 5) continue;
@@ -855,7 +870,7 @@ __global__ void __launch_bounds__(kBlock, LP_TRANSPORT_MIN_BLOCKS) transport_ker
         unsigned long long x = photons;
         for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
         if (lane == 0 && x) atomicAdd(s_cnt + 8, x);
-        x = cnt.skip;
+        x = cnt.skip();
         for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
         if (lane == 0 && x) atomicAdd(s_cnt + 10, x);
         x = cnt.bvh;
