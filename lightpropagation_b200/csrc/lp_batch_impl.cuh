@@ -25,6 +25,7 @@ struct WarpSlot {
     KParams P;
     MeshView M;
     WarpQueue Q;
+    WarpDraws W;
     Medium media[kBatchMedia];
 };
 
@@ -81,7 +82,8 @@ __device__ __forceinline__ void zero_grad(GradAcc &ga, int n_media)
 template <bool Exact, bool Grad, int BLOCK, int MINB, int STACK>
 __global__ void __launch_bounds__(BLOCK, MINB) batch_kernel(const __grid_constant__ BatchParams B)
 {
-    __shared__ WarpSlot slots[BLOCK / 32];
+    extern __shared__ __align__(16) unsigned char smem[];
+    WarpSlot *const slots = reinterpret_cast<WarpSlot *>(smem);
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lt_mask = (1u << lane) - 1u;
     WarpSlot &S = slots[threadIdx.x >> 5];
@@ -89,6 +91,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_kernel(const __grid_constan
     uint32_t photons = 0;
     Photon ph;
     GradAcc ga;
+    uint32_t next_draw = 0;
+    ph.idx = ph.steps = 0;
     bool alive = false;
     int inst = -1;
     bool exhausted = true;   // the bound instance has no unclaimed photons (or none is bound)
@@ -123,6 +127,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_kernel(const __grid_constan
             inst = next;
             const unsigned long long n = (unsigned long long)S.P.n;
             exhausted = base + 32ull >= n;
+            next_draw = 0;
             const unsigned long long idx = base + lane;
             if (idx < n) {
                 start_photon(S.P, ph, (uint32_t)idx);
@@ -131,6 +136,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_kernel(const __grid_constan
             }
         } else if (need && !exhausted) {
             const int k = __popc(need);
+            next_draw = 0;
             unsigned long long base = 0;
             if (lane == 0) base = atomicAdd(B.claimed + inst, (unsigned long long)k);
             base = __shfl_sync(0xffffffffu, base, 0);
@@ -145,8 +151,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_kernel(const __grid_constan
                 }
             }
         }
-        const bool more = step_photon<Exact, Grad, STACK>(S.P, S.M, S.M, S.Q, S.media, S.P.region, S.P.counters, alive, ph,
-                                                          cnt, &ga, rz_copy_of(S.P));
+        const bool more = step_photon<Exact, Grad, STACK>(S.P, S.M, S.M, S.Q, S.media, S.P.region, S.P.counters,
+                                                          __ballot_sync(0xffffffffu, alive), alive, ph,
+                                                          cnt, &ga, S.W, next_draw, rz_copy_of(S.P));
         if (alive) {
             if (!more) {
                 if (ph.region_acc) atomicAdd(S.P.region + ph.curr, ph.region_acc);
@@ -167,15 +174,23 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_kernel(const __grid_constan
 template <bool Exact, bool Grad, int BLOCK, int MINB, int STACK>
 cudaError_t launch_batch_t(const BatchParams &B, int grid, cudaStream_t s)
 {
-    batch_kernel<Exact, Grad, BLOCK, MINB, STACK><<<grid, BLOCK, 0, s>>>(B);
+    const int smem = BLOCK / 32 * (int)sizeof(WarpSlot);
+    cudaError_t e = cudaFuncSetAttribute(batch_kernel<Exact, Grad, BLOCK, MINB, STACK>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    batch_kernel<Exact, Grad, BLOCK, MINB, STACK><<<grid, BLOCK, smem, s>>>(B);
     return cudaGetLastError();
 }
 
 template <bool Exact, bool Grad, int BLOCK, int MINB, int STACK>
 cudaError_t batch_occupancy_t(int *blocks_per_sm)
 {
+    const int smem = BLOCK / 32 * (int)sizeof(WarpSlot);
+    cudaError_t e = cudaFuncSetAttribute(batch_kernel<Exact, Grad, BLOCK, MINB, STACK>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, batch_kernel<Exact, Grad, BLOCK, MINB, STACK>,
-                                                         BLOCK, 0);
+                                                         BLOCK, smem);
 }
 
 }  // namespace lp

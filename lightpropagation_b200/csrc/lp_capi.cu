@@ -543,6 +543,7 @@ void fill_params(lp_ctx *c, KParams &P, int64_t first, int64_t n, int nodes_smem
     P.f_dimR = (float)g.dimR;
     P.half_vnx = 0.5f * (float)c->vox_n[0];
     P.half_vny = 0.5f * (float)c->vox_n[1];
+    P.vox_on = c->vox_n[0] > 0 ? 1u : 0u;
     P.sft = c->sft.p; P.rtd = c->rtd.p; P.rz = c->rz.p; P.vox = c->vox.p; P.rbins = c->rbins.p;
     P.region = c->region.p; P.det = c->det.p; P.counters = c->counters.p;
     const int copies = rz_copies(rz_values(c));

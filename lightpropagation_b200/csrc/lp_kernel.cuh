@@ -61,6 +61,7 @@ struct KParams {
     float dg[6];
     float inv_dr, inv_dz, inv_vdx, inv_vdy, inv_vdz;   // reciprocals for the fast mode
     float f_dimR, half_vnx, half_vny;                  // dimR, vox_nx / 2, vox_ny / 2
+    uint32_t vox_on;                                   // 1 with a voxel grid
     // tallies (fixed point, 2^32 per unit weight)
     unsigned long long *sft, *rtd, *rz, *vox, *rbins, *region, *det, *counters;
     // where the r-z deposits go: rz_mask + 1 (a power of two) copies of the image, each of

@@ -18,16 +18,19 @@
 // At the end of a photon its exit record (.cl:1583-1594) is binned on the device into
 // the reference's SFT and RTd images (CalculatePropagation.cpp:1553-1626).
 //
-// What bounds it: the instructions of one step, about 500 of them in one chain that
-// branches on its own results.  A warp with one photon left issues one every 4.7 cycles
-// (fixed latencies and the special-function unit, 2,600 cycles a step), so short runs
-// and the ends of long ones wait for their longest photon; full warps (24 per SM at 80
-// registers) issue two cycles of three.  Hence the form of the step: selects instead of
-// branches where both sides are a few operations, round keys and derived constants in
-// the kernel's parameters, 32-bit indices, one 16-byte load for a medium's factors, and
-// no counter that another one implies.  Against the same step without these: slab, 1e6
-// photons, 114 -> 99 ms; curved abdomen at 660 nm, 3e6 photons, 201 -> 181 ms; 1e5
-// photons 40 -> 34 ms.
+// What bounds it: the instructions of one step, 400 to 500 of them in one chain that
+// branches on its own results.  A warp with one photon left issues one every 4 to 5
+// cycles (fixed latencies and the special-function unit), so short runs and the ends of
+// long ones wait for their longest photon; full warps (24 per SM at 80 registers) issue
+// two cycles of three.  Hence the form of the step: selects instead of branches where both
+// sides are a few operations, round keys and derived constants in the kernel's parameters,
+// 32-bit indices, two 16-byte loads for a medium's factors, no counter that another one
+// implies; no branch between the move and the deposits (square roots without a slow path,
+// no test for a voxel grid), so that the chains of direction, tallies and the next cell
+// word overlap; and random numbers drawn several events ahead once lanes are idle
+// (next_draws).  One photon alone takes 0.79 us a step on the slab (1.20 before these),
+// 0.89 on the curved abdomen (1.36); slab, 1e6 photons, 114 -> 97 ms; abdomen at 660 nm,
+// 3e6 photons, 201 -> 181 ms; 1e5 photons 40 -> 29 ms.
 //
 // Exact = true  keeps the reference's arithmetic operation by operation (compiled
 //               with --fmad=false): a photon follows the oracle's trajectory for the
@@ -67,6 +70,7 @@ struct Photon {
     float seg_len;           // differentiation: path length and interactions in the
     uint32_t seg_k;          // current region since the photon entered it
     float safe;              // lower bound of the distance from the position to any triangle
+    uint32_t word;           // cell word at the position (cell_at)
 };
 
 // Per-photon, per-region path lengths and interaction counts of a differentiated run
@@ -118,14 +122,124 @@ __device__ __forceinline__ V3 rotate(V3 vec, V3 axis, float c, float s)
     return add3(add3(scl3(nDx, axis), scl3(c, nXxXn)), scl3(s, nXx));
 }
 
+// 1 / sqrt(x) of the special-function unit, for normal x (rsqrtf without its handling of
+// denormals: the same bits).
+__device__ __forceinline__ float rsqrt_normal(float x)
+{
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// The correctly rounded square root for x >= 1e-30, 0 below: one Newton correction of
+// x / sqrt(x) with fused multiply-adds (Markstein, IBM J. Res. Dev. 34, 1990).  Compared
+// with sqrtf for every float from 1e-30 to 3e38.  Unlike sqrtf it has no branch to a slow
+// path, which would cut the step's straight line of code.
+__device__ __forceinline__ float sqrt_normal(float x)
+{
+    const float y = rsqrt_normal(x), s = x * y;
+    const float r = __fmaf_rn(__fmaf_rn(-s, s, x), 0.5f * y, s);
+    return x >= 1e-30f ? r : 0.0f;
+}
+
 __device__ __forceinline__ V3 fast_norm(V3 v)
 {
-    const float r = rsqrtf(__fmaf_rn(v.x, v.x, __fmaf_rn(v.y, v.y, v.z * v.z)));
+    const float r = rsqrt_normal(__fmaf_rn(v.x, v.x, __fmaf_rn(v.y, v.y, v.z * v.z)));
     return v3(v.x * r, v.y * r, v.z * r);
 }
 
+// Cosine and sine of the azimuth of the uniform xp.
 template <bool Exact>
-__device__ __forceinline__ V3 scatter_direction(V3 v, const Medium &m, float xt, float xp)
+__device__ __forceinline__ void azimuth(float xp, float &cosPsi, float &sinPsi)
+{
+    if (Exact) {
+        const float psi = 2.0f * 3.14159265358979323846f * xp;
+        cosPsi = cosf(psi);
+        sinPsi = sqrtf(1.0f - cosPsi * cosPsi);
+        if (psi > 3.14159265358979323846f) sinPsi *= -1.0f;
+    } else {
+        sincospif(2.0f * xp, &sinPsi, &cosPsi);
+    }
+}
+
+// What a step takes from its event's random numbers (EventRng): -log of the first, the
+// second (polar angle or Fresnel), the azimuth of the third, the fourth (roulette).  None
+// of it depends on the photon's state, only on its index and step number.
+struct Draws {
+    float neg_log, u1, cos_psi, sin_psi, u3;
+};
+template <bool Exact>
+__device__ __forceinline__ Draws make_draws(const KParams &P, uint32_t idx, uint32_t event)
+{
+    EventRng rng;
+    rng.draw(P, idx, event);
+    Draws d;
+    d.neg_log = -logf(rng.u0);
+    d.u1 = rng.u1;
+    azimuth<Exact>(rng.u2, d.cos_psi, d.sin_psi);
+    d.u3 = rng.u3;
+    return d;
+}
+
+// The warp's draws.  A warp of 17 to 32 photons draws one event for each, every lane its
+// own.  With fewer photons the idle lanes draw the following events: each of k photons
+// gets `span` lanes (the largest power of two with k span <= 32), the draws of its next
+// `span` events go through shared memory, and the warp draws again when those are used
+// up.  Philox, logarithm and azimuth are a quarter of a step's instructions; the end of a
+// run, when each warp waits for its last photons, and short runs pay for them once in up
+// to 32 steps.
+struct WarpDraws {
+    float v[5][32];
+};
+// next: the lane's next column of WarpDraws, plus 256 times the events drawn and not used
+// yet (the same for the whole warp; below 256 the warp has to draw, 0 to begin with).
+template <bool Exact>
+__device__ __forceinline__ Draws next_draws(const KParams &P, WarpDraws &W, unsigned live, bool alive, uint32_t idx,
+                                            uint32_t steps, uint32_t &next)
+{
+    Draws d;
+    if (next < 256u) {
+        const unsigned lane = threadIdx.x & 31u;
+        const int span_log = __clz(max(__popc(live), 1) - 1) - 27;   // 5 for one photon (clz(0) = 32), 0 from 17 on
+        uint32_t event = steps + 1u;
+        next = 0;
+        if (span_log > 0) {
+            const unsigned rank = __popc(live & ((1u << lane) - 1u));
+            next = (256u << span_log) + ((rank << span_log) & 31u);
+            __syncwarp();
+            if (alive) {
+                W.v[0][rank] = __uint_as_float(idx);
+                W.v[1][rank] = __uint_as_float(event);
+            }
+            __syncwarp();
+            idx = __float_as_uint(W.v[0][lane >> span_log]);
+            event = __float_as_uint(W.v[1][lane >> span_log]) + (lane & ((1u << span_log) - 1u));
+            __syncwarp();
+        }
+        d = make_draws<Exact>(P, idx, event);
+        if (span_log > 0) {
+            W.v[0][lane] = d.neg_log;
+            W.v[1][lane] = d.u1;
+            W.v[2][lane] = d.cos_psi;
+            W.v[3][lane] = d.sin_psi;
+            W.v[4][lane] = d.u3;
+            __syncwarp();
+        }
+    }
+    if (next >= 256u) {
+        const uint32_t s = next & 31u;
+        next += 1u - 256u;
+        d.neg_log = W.v[0][s];
+        d.u1 = W.v[1][s];
+        d.cos_psi = W.v[2][s];
+        d.sin_psi = W.v[3][s];
+        d.u3 = W.v[4][s];
+    }
+    return d;
+}
+
+template <bool Exact>
+__device__ __forceinline__ V3 scatter_direction(V3 v, const Medium &m, float xt, float cosPsi, float sinPsi)
 {
     const float cosTheta = hg_cos_theta<Exact>(m, xt);
     if (Exact) {
@@ -142,21 +256,15 @@ __device__ __forceinline__ V3 scatter_direction(V3 v, const Medium &m, float xt,
         }
         e_rot = norm3(e_rot);
         const float sinTheta = sqrtf(1.0f - cosTheta * cosTheta);
-        const float psi = 2.0f * 3.14159265358979323846f * xp;
-        const float cosPsi = cosf(psi);
-        float sinPsi = sqrtf(1.0f - cosPsi * cosPsi);
-        if (psi > 3.14159265358979323846f) sinPsi *= -1.0f;
         const V3 rot_theta = norm3(rotate(v, e_rot, cosTheta, sinTheta));
         return norm3(rotate(rot_theta, v, cosPsi, sinPsi));
     } else {
         // direction-cosine update (Wang, Jacques & Zheng, MCML 1995).  1 - uz^2 is taken
         // as ux^2 + uy^2 (|v| = 1), which keeps its precision near the z axis where the
         // difference form cancels; the axial case scatters about z with uz' = sign(uz) cos.
-        const float sinTheta = sqrtf(fmaxf(0.0f, __fmaf_rn(-cosTheta, cosTheta, 1.0f)));
-        float sinPsi, cosPsi;
-        sincospif(2.0f * xp, &sinPsi, &cosPsi);
+        const float sinTheta = sqrt_normal(fmaxf(0.0f, __fmaf_rn(-cosTheta, cosTheta, 1.0f)));
         const float uz2 = __fmaf_rn(v.x, v.x, v.y * v.y);
-        const float it = rsqrtf(uz2);
+        const float it = rsqrt_normal(uz2);
         const float temp = uz2 * it;  // sqrt(1 - uz^2)
         const float st = sinTheta * it;
         const float ax = sinTheta * cosPsi;
@@ -360,6 +468,7 @@ __device__ __forceinline__ void start_photon(const KParams &P, Photon &ph, uint3
     ph.seg_len = 0.0f;
     ph.seg_k = 0;
     ph.safe = 0.0f;
+    ph.word = cell_at(P, ph.px, ph.py, ph.pz);
 }
 
 // A boundary event (.cl:1443-1465 with TransmitOrReflect, .cl:921-1018): the photon moves
@@ -509,8 +618,8 @@ static __device__ __forceinline__ Photon boundary_event(const KParams &P, const 
     return ph;
 }
 
-// A step in three parts: propose_step draws the event's random numbers and the step
-// length and decides whether the step can reach a triangle; query_step finds the nearest
+// A step in three parts: propose_step forms the step length from the event's draws and
+// decides whether the step can reach a triangle; query_step finds the nearest
 // triangle within reach; complete_step moves the photon (boundary event, or absorption and
 // scattering), scores it and plays roulette.  One call of each in turn is one iteration of
 // the reference's do-while loop (.cl:1388-1600).  (Letting the lanes whose step needs a
@@ -519,8 +628,6 @@ static __device__ __forceinline__ Photon boundary_event(const KParams &P, const 
 // the shared queries save.)
 struct Pending {
     float step, reach, safe_here;   // step length, its reach, distance bound at the position
-    float u1, u2, u3;               // the event's uniforms after the step length's
-    uint32_t word;                  // cell word at the position
 };
 enum : int { kStepEnded = 0, kStepClear = 1, kStepQuery = 2 };
 
@@ -528,14 +635,9 @@ enum : int { kStepEnded = 0, kStepClear = 1, kStepQuery = 2 };
 // lies within its reach (complete_step with tri = -1); kStepEnded: the photon ended
 // (debug build: a region id out of range).
 template <bool Exact>
-__device__ __forceinline__ int propose_step(const KParams &P, const Medium *s_media, Photon &ph, Pending &pd)
+__device__ __forceinline__ int propose_step(const KParams &P, const Medium *s_media, float neg_log, Photon &ph,
+                                            Pending &pd)
 {
-    // The cell word is read on every step, its load issued before the Philox rounds so
-    // that they hide its latency (reading it only when the carried bound is used up saves
-    // loads but waits on them: 1.3 % slower on the 660 nm abdomen).
-    const uint32_t word = cell_at(P, ph.px, ph.py, ph.pz);
-    EventRng rng;
-    rng.draw(P, ph.idx, ph.steps + 1u);
     [[maybe_unused]] unsigned long long *const dbg = P.counters ? P.counters + kBoundsCounter : nullptr;
     if (!LP_IN_RANGE(dbg, ph.curr, P.n_media)) {
         ph.w = 0.0f;
@@ -546,8 +648,8 @@ __device__ __forceinline__ int propose_step(const KParams &P, const Medium *s_me
     // the residual of a step cut short by a boundary, or a new step; both are formed, and
     // the select costs less than the branch
     float step;
-    if (Exact) step = (ph.unfin == 0.0f) ? -logf(rng.u0) * P.factor / m.mut : ph.unfin / m.mut;
-    else step = (ph.unfin == 0.0f) ? -logf(rng.u0) * P.factor * m.inv_mut : ph.unfin * m.inv_mut;
+    if (Exact) step = (ph.unfin == 0.0f) ? neg_log * P.factor / m.mut : ph.unfin / m.mut;
+    else step = (ph.unfin == 0.0f) ? neg_log * P.factor * m.inv_mut : ph.unfin * m.inv_mut;
     if (ambient) step = 0.0f;
     ph.unfin = 0.0f;
     pd.step = step;
@@ -558,19 +660,15 @@ __device__ __forceinline__ int propose_step(const KParams &P, const Medium *s_me
     // on the face (and is moved off it, see boundary_event) with no residual step.
     const float reach = Exact ? step : step + P.boundary_push + 1e-6f * step;
     pd.reach = reach;
-    pd.u1 = rng.u1;
-    pd.u2 = rng.u2;
-    pd.u3 = rng.u3;
     // safe_here: lower bound of the distance from p to every triangle.  A step shorter
     // than it cannot reach one, so its bounded query would return "no hit" and is skipped;
     // after the step the bound shrinks by the step (plus the rounding of the move).
     pd.safe_here = ph.safe;
-    pd.word = word;
     if (ambient) return kStepQuery;
     if (reach < pd.safe_here) return kStepClear;
     // a cell no triangle touches: its word holds a bound for all its points (the larger of
     // two lower bounds is one too); safe_distance is 0 for the others
-    pd.safe_here = fmaxf(pd.safe_here, safe_distance(P, word));
+    pd.safe_here = fmaxf(pd.safe_here, safe_distance(P, ph.word));
     return reach < pd.safe_here ? kStepClear : kStepQuery;
 }
 
@@ -589,7 +687,7 @@ __device__ __forceinline__ int query_step(const KParams &P, const MeshView &M, c
     // an empty cell: pd.safe_here holds its bound, which the step exceeds; a listed cell
     // raises it from the planes of its triangles when its list decides the step
     const int tri = warp_query<STACK>(P, M, SM, Q, want, v3(ph.px, ph.py, ph.pz), v3(ph.vx, ph.vy, ph.vz),
-                                      (ph.flags & F_ON_FACE) ? ph.last_tri : -1, ambient ? kNoHit : pd.reach, pd.word,
+                                      (ph.flags & F_ON_FACE) ? ph.last_tri : -1, ambient ? kNoHit : pd.reach, ph.word,
                                       thit, pd.safe_here, used_bvh);
     cnt.query += want ? 1u : 0u;
     cnt.bvh += used_bvh ? 1u : 0u;
@@ -602,7 +700,7 @@ __device__ __forceinline__ int query_step(const KParams &P, const MeshView &M, c
 template <bool Exact, bool Grad, bool Agg = false>
 __device__ __forceinline__ bool complete_step(const KParams &P, const Medium *s_media, unsigned long long *s_region,
                                               unsigned long long *s_cnt, Photon &ph, Counters &cnt, GradAcc *ga,
-                                              const Pending &pd, int tri, float thit, uint32_t rz_copy)
+                                              const Pending &pd, const Draws &d, int tri, float thit, uint32_t rz_copy)
 {
     const Medium &m = s_media[ph.curr];
     const bool ambient = (m.kind & kAmbient) != 0;
@@ -612,11 +710,14 @@ __device__ __forceinline__ bool complete_step(const KParams &P, const Medium *s_
     const bool boundary = tri >= 0 || kNoHit <= step;
     if (boundary) {
         cnt.boundary++;
-        ph = boundary_event<Exact, Grad>(P, s_media, s_region, s_cnt, ph, Grad ? ga : nullptr, tri, thit, step, pd.u1);
+        ph = boundary_event<Exact, Grad>(P, s_media, s_region, s_cnt, ph, Grad ? ga : nullptr, tri, thit, step, d.u1);
+        ph.word = cell_at(P, ph.px, ph.py, ph.pz);
     } else {
         ph.px = ph.px + step * ph.vx;
         ph.py = ph.py + step * ph.vy;
         ph.pz = ph.pz + step * ph.vz;
+        // the next step's cell word: its load is in flight during the rest of this step
+        ph.word = cell_at(P, ph.px, ph.py, ph.pz);
         ph.flags &= ~F_ON_FACE;
         ph.safe = fmaxf(pd.safe_here - step - P.step_eps, 0.0f);
         if (Grad) {
@@ -626,7 +727,7 @@ __device__ __forceinline__ bool complete_step(const KParams &P, const Medium *s_
         const bool absorbs = (m.kind & kAbsorbs) != 0;
         ph.absorbed = absorbs ? ph.w * m.alb : ph.absorbed;
         ph.w = absorbs ? ph.w - ph.absorbed : ph.w;
-        const V3 vn = scatter_direction<Exact>(v, m, pd.u1, pd.u2);
+        const V3 vn = scatter_direction<Exact>(v, m, d.u1, d.cos_psi, d.sin_psi);
         ph.vx = vn.x; ph.vy = vn.y; ph.vz = vn.z;
         const V3 pr = v3(ph.px - P.poix, ph.py - P.poiy, ph.pz - P.poiz);
         const float cx = dot3(v3(P.nxx, P.nxy, P.nxz), pr);
@@ -641,30 +742,28 @@ __device__ __forceinline__ bool complete_step(const KParams &P, const Medium *s_
             row = (int)floorf(cz / P.dg[2]);
             col = (int)floorf(rad + P.f_dimR);
         } else {
-            const float rad = copysignf(sqrtf(cx * cx + cy * cy), cx) * P.inv_dr;
+            const float rad = copysignf(sqrt_normal(cx * cx + cy * cy), cx) * P.inv_dr;
             row = (int)floorf(cz * P.inv_dz);
             col = (int)floorf(rad + P.f_dimR);
         }
         const bool rz_in = ((unsigned)row < (unsigned)P.rz_nz) & ((unsigned)col < (unsigned)P.rz_nr);
         // inv_mua is 0 where mua is not positive
         const unsigned long long fdm = Exact ? (m.mua > 0.0f ? fix32(dw / m.mua) : 0ull) : fix32(dw * m.inv_mua);
-        int vox_key = -1;
-        if (P.vox_nx > 0) {
-            int ix, iy, iz;
-            if (Exact) {
-                ix = (int)floorf(cx / P.vox_dx + P.half_vnx);
-                iy = (int)floorf(cy / P.vox_dy + P.half_vny);
-                iz = (int)floorf(cz / P.vox_dz);
-            } else {
-                ix = (int)floorf(cx * P.inv_vdx + P.half_vnx);
-                iy = (int)floorf(cy * P.inv_vdy + P.half_vny);
-                iz = (int)floorf(cz * P.inv_vdz);
-            }
-            const bool vox_in = ((unsigned)ix < (unsigned)P.vox_nx) & ((unsigned)iy < (unsigned)P.vox_ny) &
-                                ((unsigned)iz < (unsigned)P.vox_nz);
-            vox_key = vox_in ? (iz * P.vox_ny + iy) * P.vox_nx + ix : -1;
-            cnt.vox_drop += vox_in ? 0u : 1u;
+        int ix, iy, iz;
+        if (Exact) {
+            ix = (int)floorf(cx / P.vox_dx + P.half_vnx);
+            iy = (int)floorf(cy / P.vox_dy + P.half_vny);
+            iz = (int)floorf(cz / P.vox_dz);
+        } else {
+            ix = (int)floorf(cx * P.inv_vdx + P.half_vnx);
+            iy = (int)floorf(cy * P.inv_vdy + P.half_vny);
+            iz = (int)floorf(cz * P.inv_vdz);
         }
+        // never in without a voxel grid (vox_nx = 0), and then no drop either
+        const bool vox_in = ((unsigned)ix < (unsigned)P.vox_nx) & ((unsigned)iy < (unsigned)P.vox_ny) &
+                            ((unsigned)iz < (unsigned)P.vox_nz);
+        const int vox_key = vox_in ? (iz * P.vox_ny + iy) * P.vox_nx + ix : -1;
+        cnt.vox_drop += vox_in ? 0u : P.vox_on;
         cnt.rz_drop += rz_in ? 0u : 1u;
         const int rz_key = rz_in ? row * P.rz_nr + col : -1;
         unsigned long long *const rz = P.rz_part + 2 * (int64_t)rz_copy;
@@ -690,18 +789,19 @@ __device__ __forceinline__ bool complete_step(const KParams &P, const Medium *s_
                 if (a && lane == (unsigned)(__ffs(g_vox) - 1)) atomicAdd(P.vox + vox_key, a);
             }
         } else {
+            // a weight that rounds to 0 is rare, and adding it is cheaper than the test
             if (rz_key >= 0) {
                 unsigned long long *c = rz + 2 * (int64_t)rz_key;
-                if (fdw) atomicAdd(c, fdw);
-                if (fdm) atomicAdd(c + 1, fdm);
+                atomicAdd(c, fdw);
+                atomicAdd(c + 1, fdm);
             }
-            if (vox_key >= 0 && fdw) atomicAdd(P.vox + vox_key, fdw);
+            if (vox_key >= 0) atomicAdd(P.vox + vox_key, fdw);
         }
         ph.region_acc += fdw;
     }
     if (ph.w < P.w_th && ph.w > 0.0f) {
         cnt.roulette++;
-        if (pd.u3 < P.chance) {
+        if (d.u3 < P.chance) {
             ph.w /= P.chance;
         } else {
             ph.w = 0.0f;
@@ -721,21 +821,22 @@ __device__ __forceinline__ uint32_t rz_copy_of(const KParams &P)
 }
 
 // One iteration of the reference's do-while loop, the three parts in turn, for the warp's
-// photons (the whole warp calls it, `alive` lanes have one).  Returns false when the
+// photons (the whole warp calls it; `live` has the lanes with one, `alive` is the lane's bit).  Returns false when the
 // lane's photon ends.
 template <bool Exact, bool Grad, int STACK = kStackDepth, bool Agg = false>
 __device__ __forceinline__ bool step_photon(const KParams &P, const MeshView &M, const MeshView &SM, WarpQueue &Q,
                                             const Medium *s_media, unsigned long long *s_region,
-                                            unsigned long long *s_cnt, bool alive, Photon &ph, Counters &cnt,
-                                            GradAcc *ga, uint32_t rz_copy)
+                                            unsigned long long *s_cnt, unsigned live, bool alive, Photon &ph, Counters &cnt,
+                                            GradAcc *ga, WarpDraws &W, uint32_t &next, uint32_t rz_copy)
 {
+    const Draws d = next_draws<Exact>(P, W, live, alive, ph.idx, ph.steps, next);
     Pending pd;
     int st = kStepEnded;
-    if (alive) st = propose_step<Exact>(P, s_media, ph, pd);
+    if (alive) st = propose_step<Exact>(P, s_media, d.neg_log, ph, pd);
     float thit;
     const int tri = query_step<STACK>(P, M, SM, Q, s_media, st == kStepQuery, ph, cnt, pd, thit);
     if (st == kStepEnded) return false;
-    return complete_step<Exact, Grad, Agg>(P, s_media, s_region, s_cnt, ph, cnt, ga, pd, tri, thit, rz_copy);
+    return complete_step<Exact, Grad, Agg>(P, s_media, s_region, s_cnt, ph, cnt, ga, pd, d, tri, thit, rz_copy);
 }
 
 struct SmemLayout {
@@ -794,6 +895,7 @@ __global__ void __launch_bounds__(kBlock, LP_TRANSPORT_MIN_BLOCKS) transport_ker
 {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ WarpQueue queues[kBlock / 32];
+    __shared__ WarpDraws draws[kBlock / 32];
     const SmemLayout L = smem_layout(P.nodes_smem, P.tris_smem);
     Medium *s_media = reinterpret_cast<Medium *>(smem + L.off_media);
     unsigned long long *s_region = reinterpret_cast<unsigned long long *>(smem + L.off_region);
@@ -815,12 +917,16 @@ __global__ void __launch_bounds__(kBlock, LP_TRANSPORT_MIN_BLOCKS) transport_ker
     uint32_t photons = 0;
     Photon ph;
     GradAcc ga;
+    uint32_t next = 0;
     bool alive = false;
     bool exhausted = false;
+    ph.idx = ph.steps = 0;
     for (;;) {
-        const unsigned need = __ballot_sync(0xffffffffu, !alive);
-        if (need && !exhausted) {
+        unsigned live = __ballot_sync(0xffffffffu, alive);
+        if (live != 0xffffffffu && !exhausted) {
+            const unsigned need = ~live;
             const int k = __popc(need);
+            next = 0;   // the new photons' events are to be drawn
             unsigned long long base = 0;
             if (lane == 0) base = atomicAdd(P.work, (unsigned long long)k);
             base = __shfl_sync(0xffffffffu, base, 0);
@@ -838,11 +944,12 @@ __global__ void __launch_bounds__(kBlock, LP_TRANSPORT_MIN_BLOCKS) transport_ker
                     alive = true;
                 }
             }
+            live = __ballot_sync(0xffffffffu, alive);
         }
-        if (!__any_sync(0xffffffffu, alive)) break;
+        if (!live) break;
         const bool more = step_photon<Exact, Grad, kStackDepth, Agg>(P, M, shared_view, queues[threadIdx.x >> 5],
-                                                                     s_media, s_region, s_cnt, alive, ph, cnt, &ga,
-                                                                     rz_copy);
+                                                                     s_media, s_region, s_cnt, live, alive, ph, cnt, &ga,
+                                                                     draws[threadIdx.x >> 5], next, rz_copy);
         if (alive) {
             if (!more) {
                 if (ph.region_acc) atomicAdd(s_region + ph.curr, ph.region_acc);
