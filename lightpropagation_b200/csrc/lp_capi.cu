@@ -1101,7 +1101,6 @@ int lp_run_async(lp_ctx *c, int64_t first, int64_t n)
     c->st_tris_smem = tris_smem;
     c->st_smem = smem;
     c->st_per_sm = per_sm;
-    c->st_grid = c->num_sms * per_sm;
     // The kernel indexes the photons of one launch with 32 bits: a longer range runs as
     // several launches in order (the same photon ids, so the same tallies).  Exit records
     // (at most 2^30 slots, indexed from the range's first photon) all come from the first.
@@ -1113,10 +1112,13 @@ int lp_run_async(lp_ctx *c, int64_t first, int64_t n)
             P.exit_rec = nullptr;
             P.exit_cap = 0;
         }
+        int grid;
+        lp::plan_launch(P, lp::block_size(), c->num_sms, per_sm, grid);
+        c->st_grid = grid;
         LP_CUDA(c, cudaMemsetAsync(c->work.p, 0, 8, c->stream));
         c->h2d_bytes += (int64_t)sizeof(KParams);
-        LP_CUDA(c, c->exact ? lp::launch_transport_exact(P, c->num_sms * per_sm, smem, c->stream)
-                            : lp::launch_transport_fast(P, c->num_sms * per_sm, smem, c->stream));
+        LP_CUDA(c, c->exact ? lp::launch_transport_exact(P, grid, smem, c->stream)
+                            : lp::launch_transport_fast(P, grid, smem, c->stream));
     }
     const int copies = rz_copies(rz_values(c));
     if (copies > 1)
@@ -1622,7 +1624,7 @@ int prepare_plain(lp_batch *b)
         LP_BCUDA(b, b->grad_on ? lp::transport_occupancy_fast_grad(L.smem, &per_sm)
                                : lp::transport_occupancy_fast(L.smem, &per_sm));
         if (per_sm < 1) return bfail(b, LP_ERR_CUDA, "batch: transport kernel does not fit on an SM");
-        L.grid = b->num_sms * per_sm;
+        lp::plan_launch(L.P, lp::block_size(), b->num_sms, per_sm, L.grid);
     }
     return LP_OK;
 }

@@ -105,7 +105,27 @@ struct KParams {
     int32_t agg_tallies;
     // scratch: photon work counter
     unsigned long long *work;
+    uint32_t lane_mask;   // lanes of a warp that carry photons (plan_launch)
 };
+
+// Blocks of a transport launch and the lanes of a warp that carry photons.  A short run
+// lasts as long as its longest photon (many times the mean), and a photon's step takes
+// the longer the more others share its warp (each of them may have a query or a boundary
+// event) and its SM.  So up to the lanes of two blocks per SM the photons are spread evenly
+// over the warps of two, and up to twice as many take turns on them.  Against full warps
+// on three blocks (slab / curved abdomen at 660 nm): 1,000 photons 17.9 -> 12.2 / 15.3 ->
+// 10.1 ms, 10,000 20.8 -> 16.6 / 20.3 -> 18.1, 30,000 25.0 -> 20.5 / 23.5 -> 20.1, 100,000
+// 31.2 -> 29.6 / 28.6 -> 27.3; at 300,000 three blocks win on the slab (43.7 against 47.7)
+// and lose on the abdomen (42.8 against 40.2).
+inline void plan_launch(KParams &P, int block, int num_sms, int per_sm, int &grid)
+{
+    const int few = per_sm < 2 ? per_sm : 2;
+    const int64_t warps = (int64_t)num_sms * few * (block / 32);
+    int64_t lanes = (P.n + warps - 1) / warps;
+    lanes = lanes < 1 ? 1 : lanes > 32 ? 32 : lanes;
+    P.lane_mask = lanes == 32 ? 0xffffffffu : (1u << lanes) - 1u;
+    grid = num_sms * (P.n <= 64 * warps ? few : per_sm);
+}
 
 // A batch: many instances (one KParams each) traced by one persistent launch.
 constexpr int kBatchMedia = kGradRegions;   // regions per instance in a batch

@@ -24,6 +24,7 @@
 
 namespace lp {
 int smem_bytes(int nodes_smem, int tris_smem);
+int block_size();
 cudaError_t launch_transport_exact(const KParams &P, int grid, int smem, cudaStream_t s);
 cudaError_t transport_occupancy_exact(int smem, int *blocks_per_sm);
 void set_thread_error(const char *msg);
@@ -355,7 +356,9 @@ extern "C" int lp_run_noalloc(const lp_noalloc_args *a, void *stream)
         std::lock_guard<std::mutex> lk(lp::launch_mutex());
         if ((e = transport_occupancy_exact(smem, &per_sm)) != cudaSuccess || per_sm < 1)
             return reject(LP_ERR_CUDA, "lp_run_noalloc: occupancy query failed");
-        if ((e = launch_transport_exact(P, sms * per_sm, smem, s)) != cudaSuccess)
+        int grid;
+        plan_launch(P, block_size(), sms, per_sm, grid);
+        if ((e = launch_transport_exact(P, grid, smem, s)) != cudaSuccess)
             return reject(LP_ERR_CUDA, "lp_run_noalloc: transport launch failed");
     }
     if (a->counters) {

@@ -923,15 +923,15 @@ __global__ void __launch_bounds__(kBlock, LP_TRANSPORT_MIN_BLOCKS) transport_ker
     ph.idx = ph.steps = 0;
     for (;;) {
         unsigned live = __ballot_sync(0xffffffffu, alive);
-        if (live != 0xffffffffu && !exhausted) {
-            const unsigned need = ~live;
+        if (live != P.lane_mask && !exhausted) {
+            const unsigned need = P.lane_mask & ~live;
             const int k = __popc(need);
             next = 0;   // the new photons' events are to be drawn
             unsigned long long base = 0;
             if (lane == 0) base = atomicAdd(P.work, (unsigned long long)k);
             base = __shfl_sync(0xffffffffu, base, 0);
             if (base + (unsigned long long)k >= (unsigned long long)P.n) exhausted = true;
-            if (!alive) {
+            if ((need >> lane) & 1u) {
                 const unsigned long long idx = base + __popc(need & lt_mask);
                 if (idx < (unsigned long long)P.n) {
                     start_photon(P, ph, (uint32_t)idx);
