@@ -330,18 +330,18 @@ int64_t n_vox(const lp_ctx *c)
     return c->vox_n[0] > 0 ? (int64_t)c->vox_n[0] * c->vox_n[1] * c->vox_n[2] : 0;
 }
 
-// Copies of an r-z image of n values for the deposits of a launch, `images` of them at
-// once.  Every scatter event adds to its cell of the r-z image, and as all photons start
-// at one point, a few cells near it take most of the adds: the L2 works them off one
-// after the other.  On the curved abdomen at 660 nm (3e6 photons, 1.2 MB image) one copy
-// takes 400 ms, two 277, four 217 and eight or more 216; without the deposits it is 215.
-// Sixteen leave room for a faster step.  The limit keeps the copies of one image within a
-// quarter of the L2 (a larger image has finer cells, so fewer adds to each), the second
-// one those of a batch within a few percent of the device memory.
+// Copies of an r-z image of n values for the deposits of a launch.  Every scatter event
+// adds to its cell of the r-z image, and as all photons start at one point, a few cells
+// near it take most of the adds: the L2 works them off one after the other.  On the curved
+// abdomen at 660 nm (3e6 photons, 1.2 MB image, the step as it was then) one copy took
+// 400 ms, two 277, four 217 and eight or more 216; without the deposits it was 215.
+// Sixteen leave room for a faster step.  The limit keeps the copies within a quarter of the
+// L2 (a larger image has finer cells, so fewer adds to each).  The instances of a batch
+// launch run side by side, each with an image of its own, and share out the sixteen.
 int rz_copies(size_t n, size_t images = 1)
 {
     size_t k = 16;
-    while (k > 1 && (k * n * 8 > (size_t(32) << 20) || k * n * images * 8 > (size_t(4) << 30))) k /= 2;
+    while (k > 1 && (k * n * 8 > (size_t(32) << 20) || k * images > 16)) k /= 2;
     return (int)k;
 }
 
@@ -1113,7 +1113,7 @@ int lp_run_async(lp_ctx *c, int64_t first, int64_t n)
             P.exit_cap = 0;
         }
         int grid;
-        lp::plan_launch(P, lp::block_size(), c->num_sms, per_sm, grid);
+        lp::plan_launch(m, lp::block_size(), c->num_sms, per_sm, grid, P.lane_mask);
         c->st_grid = grid;
         LP_CUDA(c, cudaMemsetAsync(c->work.p, 0, 8, c->stream));
         c->h2d_bytes += (int64_t)sizeof(KParams);
@@ -1444,10 +1444,12 @@ struct lp_batch {
     DevBuf<double> grad;
     DevBuf<Medium> media;
     DevBuf<KParams> params;
-    DevBuf<int32_t> frontier;
+    DevBuf<int64_t> cum;       // BatchParams::cum
+    int64_t n_batch = 0;       // photons of the batch launch
     bool grad_on = false;
     int config = -1;
     int grid = 0;
+    uint32_t lane_mask = 0xffffffffu;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     // Instances of at least plain_min photons (plain_min > 0) run as a persistent transport
@@ -1581,7 +1583,13 @@ int upload_instances(lp_batch *b)
         LP_BCUDA(b, b->plain_work.ensure(b->plain.size()));
         for (size_t k = 0; k < b->plain.size(); ++k) b->plain[k].P.work = b->plain_work.p + k;
     }
+    std::vector<int64_t> cum(I + 1, 0);
+    for (size_t i = 0; i < I; ++i) cum[i + 1] = cum[i] + P[i].n;
+    // the graph's launch was planned for the photons it had then
+    if (b->n_batch != cum[I]) drop_graph(b);
+    b->n_batch = cum[I];
     if (I) {
+        LP_BCUDA(b, cudaMemcpyAsync(b->cum.p, cum.data(), (I + 1) * 8, cudaMemcpyHostToDevice, b->stream));
         LP_BCUDA(b, cudaMemcpyAsync(b->params.p, P.data(), I * sizeof(KParams), cudaMemcpyHostToDevice, b->stream));
         LP_BCUDA(b, cudaMemcpyAsync(b->media.p, M.data(), M.size() * sizeof(Medium), cudaMemcpyHostToDevice,
                                     b->stream));
@@ -1605,7 +1613,6 @@ int enqueue_zero(lp_batch *b)
     LP_BCUDA(b, cudaMemsetAsync(b->counters.p, 0, I * LP_NCOUNTERS * 8, s));
     LP_BCUDA(b, cudaMemsetAsync(b->grad.p, 0, I * grad_stride(b) * 8, s));
     LP_BCUDA(b, cudaMemsetAsync(b->claimed.p, 0, I * 8, s));
-    LP_BCUDA(b, cudaMemsetAsync(b->frontier.p, 0, 4, s));
     if (!b->plain.empty()) LP_BCUDA(b, cudaMemsetAsync(b->plain_work.p, 0, b->plain.size() * 8, s));
     for (size_t k = 0; k < b->plain.size(); ++k) {
         LP_BCUDA(b, cudaMemsetAsync(b->own[k]->rz.p, 0, b->n_rz * 8, s));
@@ -1624,7 +1631,7 @@ int prepare_plain(lp_batch *b)
         LP_BCUDA(b, b->grad_on ? lp::transport_occupancy_fast_grad(L.smem, &per_sm)
                                : lp::transport_occupancy_fast(L.smem, &per_sm));
         if (per_sm < 1) return bfail(b, LP_ERR_CUDA, "batch: transport kernel does not fit on an SM");
-        lp::plan_launch(L.P, lp::block_size(), b->num_sms, per_sm, L.grid);
+        lp::plan_launch(L.P.n, lp::block_size(), b->num_sms, per_sm, L.grid, L.P.lane_mask);
     }
     return LP_OK;
 }
@@ -1647,7 +1654,9 @@ int prepare_grid(lp_batch *b, int config)
     int per_sm = 0;
     LP_BCUDA(b, lp::batch_occupancy(config, b->grad_on, &per_sm));
     if (per_sm < 1) return bfail(b, LP_ERR_CUDA, "batch configuration %d does not fit on an SM", config);
-    b->grid = b->num_sms * per_sm;
+    int block, minb, stack;
+    lp::batch_config_info(config, &block, &minb, &stack);
+    lp::plan_launch(b->n_batch, block, b->num_sms, per_sm, b->grid, b->lane_mask);
     return LP_OK;
 }
 
@@ -1656,8 +1665,9 @@ int enqueue_launch(lp_batch *b, int config)
     lp::BatchParams B;
     B.inst = b->params.p;
     B.claimed = b->claimed.p;
-    B.frontier = b->frontier.p;
+    B.cum = b->cum.p;
     B.n_inst = (int32_t)b->inst.size();
+    B.lane_mask = b->lane_mask;
     LP_BCUDA(b, lp::launch_batch(config, b->grad_on, B, b->grid, b->stream));
     const int copies = rz_copies(b->n_rz, b->inst.size());
     if (copies > 1)
@@ -1762,7 +1772,6 @@ int lp_batch_create(lp_batch **out, int32_t n_ctx, lp_ctx *const *ctxs)
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&b->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&b->ev1);
-    if (e == cudaSuccess) e = b->frontier.ensure(1);
     if (e != cudaSuccess) {
         int r = fail(nullptr, LP_ERR_CUDA, "lp_batch_create: %s", cudaGetErrorString(e));
         lp_batch_destroy(b);
@@ -1825,6 +1834,7 @@ int lp_batch_set_instances(lp_batch *b, int32_t n_inst, const lp_instance *in)
         LP_BCUDA(b, b->counters.ensure(J * LP_NCOUNTERS));
         LP_BCUDA(b, b->grad.ensure(J * grad_stride(b)));
         LP_BCUDA(b, b->claimed.ensure(J));
+        LP_BCUDA(b, b->cum.ensure(J + 1));
         LP_BCUDA(b, b->media.ensure(J * lp::kBatchMedia));
         LP_BCUDA(b, b->params.ensure(J));
     }

@@ -117,14 +117,15 @@ struct KParams {
 // 10.1 ms, 10,000 20.8 -> 16.6 / 20.3 -> 18.1, 30,000 25.0 -> 20.5 / 23.5 -> 20.1, 100,000
 // 31.2 -> 29.6 / 28.6 -> 27.3; at 300,000 three blocks win on the slab (43.7 against 47.7)
 // and lose on the abdomen (42.8 against 40.2).
-inline void plan_launch(KParams &P, int block, int num_sms, int per_sm, int &grid)
+inline void plan_launch(int64_t n, int block, int num_sms, int per_sm, int &grid, uint32_t &lane_mask)
 {
-    const int few = per_sm < 2 ? per_sm : 2;
+    const int two = 512 / block > 1 ? 512 / block : 1;   // 16 warps, two blocks of the transport kernel
+    const int few = per_sm < two ? per_sm : two;
     const int64_t warps = (int64_t)num_sms * few * (block / 32);
-    int64_t lanes = (P.n + warps - 1) / warps;
+    int64_t lanes = (n + warps - 1) / warps;
     lanes = lanes < 1 ? 1 : lanes > 32 ? 32 : lanes;
-    P.lane_mask = lanes == 32 ? 0xffffffffu : (1u << lanes) - 1u;
-    grid = num_sms * (P.n <= 64 * warps ? few : per_sm);
+    lane_mask = lanes == 32 ? 0xffffffffu : (1u << lanes) - 1u;
+    grid = num_sms * (n <= 64 * warps ? few : per_sm);
 }
 
 // A batch: many instances (one KParams each) traced by one persistent launch.
@@ -132,8 +133,9 @@ constexpr int kBatchMedia = kGradRegions;   // regions per instance in a batch
 struct BatchParams {
     const KParams *inst;             // [n_inst] per-instance parameters (device memory)
     unsigned long long *claimed;     // [n_inst] photon indices handed out so far
-    int32_t *frontier;               // lowest instance that may still have unclaimed photons
+    const int64_t *cum;              // [n_inst + 1] photons of the instances before each
     int32_t n_inst;
+    uint32_t lane_mask;              // lanes of a warp that carry photons (plan_launch)
 };
 
 // Bounds checks of the debug build (compiled with -DLP_DEBUG into liblpcuda_debug.so):

@@ -357,7 +357,7 @@ extern "C" int lp_run_noalloc(const lp_noalloc_args *a, void *stream)
         if ((e = transport_occupancy_exact(smem, &per_sm)) != cudaSuccess || per_sm < 1)
             return reject(LP_ERR_CUDA, "lp_run_noalloc: occupancy query failed");
         int grid;
-        plan_launch(P, block_size(), sms, per_sm, grid);
+        plan_launch(P.n, block_size(), sms, per_sm, grid, P.lane_mask);
         if ((e = launch_transport_exact(P, grid, smem, s)) != cudaSuccess)
             return reject(LP_ERR_CUDA, "lp_run_noalloc: transport launch failed");
     }
