@@ -61,10 +61,10 @@ __device__ __forceinline__ void warp_load_slot(WarpSlot &S, const KParams *inst,
     if (lane == 0) {
         MeshView &M = S.M;
         M.na = S.P.node_a; M.nb = S.P.node_b; M.nc = S.P.node_c; M.nd = S.P.node_d;
-        M.ta = S.P.tri_a; M.tb = S.P.tri_b; M.tc = S.P.tri_c;
+        M.tri = S.P.tri;
         M.s_na = M.s_nb = M.s_nc = nullptr;
         M.s_nd = nullptr;
-        M.s_ta = M.s_tb = M.s_tc = nullptr;
+        M.s_tri = nullptr;
         M.nodes_smem = 0;
         M.tris_smem = 0;
         M.n_nodes = S.P.n_nodes;

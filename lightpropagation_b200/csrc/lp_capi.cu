@@ -235,7 +235,7 @@ struct lp_ctx {
     float fiber_radius = 0.0f, fiber_na = 0.0f;
     lp_geometry geo{};
     // device buffers
-    DevBuf<float4> node_a, node_b, node_c, tri_a, tri_b, tri_c, attr;
+    DevBuf<float4> node_a, node_b, node_c, tri, attr;
     DevBuf<int4> node_d;
     DevBuf<Medium> media;
     DevBuf<unsigned long long> sft, rtd, rz, vox, rbins, region, det, counters, work;
@@ -394,18 +394,14 @@ int upload_mesh(lp_ctx *c)
     LP_CUDA(c, c->node_b.ensure(nn));
     LP_CUDA(c, c->node_c.ensure(nn));
     LP_CUDA(c, c->node_d.ensure(nn));
-    LP_CUDA(c, c->tri_a.ensure(nt));
-    LP_CUDA(c, c->tri_b.ensure(nt));
-    LP_CUDA(c, c->tri_c.ensure(nt));
+    LP_CUDA(c, c->tri.ensure(3 * nt));
     LP_CUDA(c, c->attr.ensure(nt));
     cudaStream_t s = c->stream;
     LP_CUDA(c, cudaMemcpyAsync(c->node_a.p, b.node_a.data(), nn * 16, cudaMemcpyHostToDevice, s));
     LP_CUDA(c, cudaMemcpyAsync(c->node_b.p, b.node_b.data(), nn * 16, cudaMemcpyHostToDevice, s));
     LP_CUDA(c, cudaMemcpyAsync(c->node_c.p, b.node_c.data(), nn * 16, cudaMemcpyHostToDevice, s));
     LP_CUDA(c, cudaMemcpyAsync(c->node_d.p, b.node_d.data(), nn * 16, cudaMemcpyHostToDevice, s));
-    LP_CUDA(c, cudaMemcpyAsync(c->tri_a.p, b.tri_a.data(), nt * 16, cudaMemcpyHostToDevice, s));
-    LP_CUDA(c, cudaMemcpyAsync(c->tri_b.p, b.tri_b.data(), nt * 16, cudaMemcpyHostToDevice, s));
-    LP_CUDA(c, cudaMemcpyAsync(c->tri_c.p, b.tri_c.data(), nt * 16, cudaMemcpyHostToDevice, s));
+    LP_CUDA(c, cudaMemcpyAsync(c->tri.p, b.tri.data(), nt * 48, cudaMemcpyHostToDevice, s));
     LP_CUDA(c, cudaMemcpyAsync(c->attr.p, c->tri_attr.data(), nt * 16, cudaMemcpyHostToDevice, s));
     c->h2d_bytes += (int64_t)(nn * 64 + nt * 64);
     c->mesh_dirty = false;
@@ -499,7 +495,7 @@ void fill_params(lp_ctx *c, KParams &P, int64_t first, int64_t n, int nodes_smem
 {
     std::memset(&P, 0, sizeof P);
     P.node_a = c->node_a.p; P.node_b = c->node_b.p; P.node_c = c->node_c.p; P.node_d = c->node_d.p;
-    P.tri_a = c->tri_a.p; P.tri_b = c->tri_b.p; P.tri_c = c->tri_c.p; P.tri_attr = c->attr.p;
+    P.tri = c->tri.p; P.tri_attr = c->attr.p;
     P.n_nodes = (int32_t)c->bvh.node_a.size();
     P.n_tri = (int32_t)c->n_tri;
     P.nodes_smem = nodes_smem;
@@ -648,7 +644,7 @@ int build_safety_grid(lp_ctx *c)
     KParams P;
     std::memset(&P, 0, sizeof P);
     P.node_a = c->node_a.p; P.node_b = c->node_b.p; P.node_c = c->node_c.p; P.node_d = c->node_d.p;
-    P.tri_a = c->tri_a.p; P.tri_b = c->tri_b.p; P.tri_c = c->tri_c.p;
+    P.tri = c->tri.p;
     P.g_ox = c->g_origin[0]; P.g_oy = c->g_origin[1]; P.g_oz = c->g_origin[2];
     P.g_nx = c->g_n[0]; P.g_ny = c->g_n[1]; P.g_nz = c->g_n[2];
     P.g_unit = c->g_unit;
@@ -783,7 +779,7 @@ void lp_destroy(lp_ctx *c)
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     c->node_a.release(); c->node_b.release(); c->node_c.release(); c->node_d.release();
-    c->tri_a.release(); c->tri_b.release(); c->tri_c.release(); c->attr.release();
+    c->tri.release(); c->attr.release();
     c->media.release();
     c->sft.release(); c->rtd.release(); c->rz.release(); c->vox.release(); c->rbins.release();
     c->region.release(); c->det.release(); c->counters.release(); c->work.release();

@@ -34,7 +34,7 @@ struct KParams {
     // mesh (see lp_bvh.hpp)
     const float4 *node_a, *node_b, *node_c;
     const int4 *node_d;
-    const float4 *tri_a, *tri_b, *tri_c;
+    const float4 *tri;        // three per triangle in BVH order: tri_a, tri_b, tri_c of lp_bvh.hpp
     const float4 *tri_attr;   // by original index: unit normal, (inner | outer << 16) bits
     int32_t n_nodes, n_tri, nodes_smem, tris_smem;
     // media
@@ -310,10 +310,10 @@ __device__ __forceinline__ int trunc_sat_d(double q)
 struct MeshView {
     const float4 *na, *nb, *nc;
     const int4 *nd;
-    const float4 *ta, *tb, *tc;
+    const float4 *tri;
     const float4 *s_na, *s_nb, *s_nc;
     const int4 *s_nd;
-    const float4 *s_ta, *s_tb, *s_tc;
+    const float4 *s_tri;
     int32_t nodes_smem, tris_smem;
     int32_t n_nodes, n_tri;          // array sizes for the debug build's bounds checks
     // barycentric tolerance of the hit test: 0 is the reference's test; a few 1e-6 (the
@@ -323,19 +323,14 @@ struct MeshView {
     unsigned long long *dbg;         // its counter of skipped accesses (may be null)
 };
 
-// A triangle record in BVH order: staged in shared memory or read from the mesh arrays.
+// A triangle record in BVH order, 48 bytes in one piece (two sectors; three apart would be
+// three).
 struct TriRec {
     float4 a, b, c;
 };
-__device__ __forceinline__ TriRec load_tri(const MeshView &M, int j)
+__device__ __forceinline__ TriRec load_tri(const float4 *tri, int j)
 {
-    TriRec T;
-    if (j < M.tris_smem) {
-        T.a = M.s_ta[j]; T.b = M.s_tb[j]; T.c = M.s_tc[j];
-    } else {
-        T.a = __ldg(M.ta + j); T.b = __ldg(M.tb + j); T.c = __ldg(M.tc + j);
-    }
-    return T;
+    return TriRec{__ldg(tri + 3 * j), __ldg(tri + 3 * j + 1), __ldg(tri + 3 * j + 2)};
 }
 
 // The reference's ray/triangle test (.cl:1047-1083) of the ray (p, v), with G = p - M,
@@ -369,7 +364,9 @@ __device__ __forceinline__ void test_tri(const MeshView &M, int j, V3 p, V3 v, i
                                          int &bid)
 {
     if (!LP_IN_RANGE(M.dbg, j, M.n_tri)) return;
-    const TriRec T = load_tri(M, j);
+    TriRec T;
+    if (j < M.tris_smem) T = TriRec{M.s_tri[3 * j], M.s_tri[3 * j + 1], M.s_tri[3 * j + 2]};
+    else T = load_tri(M.tri, j);
     const int o = __float_as_int(T.c.y);
     if (o == ref_tri) return;
     const V3 E = v3(T.a.w, T.b.x, T.b.y), F = v3(T.b.z, T.b.w, T.c.x);
@@ -536,42 +533,55 @@ __device__ __forceinline__ int warp_query(const KParams &P, const MeshView &M, c
         const bool mine = ((todo >> lane) & 1u) && rank < kQueue;
         float s = 0.0f, limit = fminf(bound, kNoHit);
         int cells = 0;
-        bool first = true, own = false;
+        bool own = false;
+        uint32_t cnt = 0, off = 0;   // each query's next list
         if (mine) {
+            // the cell it starts in
+            const float reach = P.g_margin + cell_face_distance(P, p.x, p.y, p.z) - P.g_eps;
             Q.ray0[rank] = make_float4(p.x, p.y, p.z, v.x);
             Q.ray1[rank] = make_float4(v.y, v.z, limit, __int_as_float(ref_tri));
             Q.best[rank] = ((unsigned long long)__float_as_uint(limit) << 32) | kNoTri;
-        }
-        for (;;) {
-            // each query's next list
-            uint32_t cnt = 0, off = 0;
-            while (mine && !bvh && cnt == 0 && s <= limit) {
-                const V3 q = v3(p.x + s * v.x, p.y + s * v.y, p.z + s * v.z);
-                const uint32_t w = first ? word : cell_at(P, q.x, q.y, q.z);
-                float reach = P.g_margin + cell_face_distance(P, q.x, q.y, q.z) - P.g_eps;
-                if (w & kCellEmpty) {
-                    if (w & kCellOutside) {
-                        // just inside the box: its outermost cells hold no triangle
-                        const float t = grid_entry(P, q, v);
-                        reach = t < kNoHit ? t + 0.25f * P.g_h : 4.0f * kNoHit;
-                    } else {
-                        reach = fmaxf(reach, safe_distance(P, w));
-                    }
-                } else {
-                    cnt = (w >> 24) & 127u;
-                    off = w & 0xffffffu;
-                    bvh = cnt == kCellDense;
-                    own = first && bound <= reach && !bvh;
-                    if (first) Q.safe[rank] = __float_as_uint(ref_tri < 0 ? fmaxf(reach, 0.0f) : 0.0f);
-                    if (!LP_IN_RANGE(M.dbg, (int64_t)off + cnt - 1, P.n_cell_refs)) {
-                        cnt = 0;
-                        Q.safe[rank] = 0u;
-                    }
+            Q.safe[rank] = __float_as_uint(ref_tri < 0 ? fmaxf(reach, 0.0f) : 0.0f);
+            if (!(word & kCellEmpty)) {
+                cnt = (word >> 24) & 127u;
+                off = word & 0xffffffu;
+                bvh = cnt == kCellDense;
+                own = bound <= reach && !bvh;
+                s = 0.9375f * reach;
+                if (!LP_IN_RANGE(M.dbg, (int64_t)off + cnt - 1, P.n_cell_refs)) {
+                    cnt = 0;
+                    Q.safe[rank] = 0u;
                 }
-                first = false;
-                if (++cells > kMarchMax || !(reach > 0.125f * P.g_h)) bvh = bvh || !own;
-                s = own ? 2.0f * kNoHit : s + 0.9375f * reach;
+                if (!own && !(reach > 0.125f * P.g_h)) bvh = true;
                 if (bvh) cnt = 0;
+            }
+        }
+        const bool march = mine && !own;
+        const bool marching = __any_sync(0xffffffffu, march);
+        for (;;) {
+            if (marching) {
+                while (march && !bvh && cnt == 0 && s <= limit) {
+                    const V3 q = v3(p.x + s * v.x, p.y + s * v.y, p.z + s * v.z);
+                    const uint32_t w = cell_at(P, q.x, q.y, q.z);
+                    float reach = P.g_margin + cell_face_distance(P, q.x, q.y, q.z) - P.g_eps;
+                    if (w & kCellEmpty) {
+                        if (w & kCellOutside) {
+                            // just inside the box: its outermost cells hold no triangle
+                            const float t = grid_entry(P, q, v);
+                            reach = t < kNoHit ? t + 0.25f * P.g_h : 4.0f * kNoHit;
+                        } else {
+                            reach = fmaxf(reach, safe_distance(P, w));
+                        }
+                    } else {
+                        cnt = (w >> 24) & 127u;
+                        off = w & 0xffffffu;
+                        bvh = cnt == kCellDense;
+                        if (!LP_IN_RANGE(M.dbg, (int64_t)off + cnt - 1, P.n_cell_refs)) cnt = 0;
+                    }
+                    s += 0.9375f * reach;
+                    if (++cells > kMarchMax || !(reach > 0.125f * P.g_h)) bvh = true;
+                    if (bvh) cnt = 0;
+                }
             }
             const unsigned segs = __ballot_sync(0xffffffffu, cnt > 0);
             if (!segs) break;
@@ -596,7 +606,7 @@ __device__ __forceinline__ int warp_query(const KParams &P, const MeshView &M, c
                     const uint32_t k = sg >> 27;
                     const int j = __ldg(P.cell_refs + ((sg & 0x7ffffffu) - kSegBias + item));
                     if (LP_IN_RANGE(M.dbg, j, M.n_tri)) {
-                        const TriRec T = load_tri(M, j);
+                        const TriRec T = load_tri(P.tri, j);
                         const float4 r0 = Q.ray0[k], r1 = Q.ray1[k];
                         const V3 E = v3(T.a.w, T.b.x, T.b.y), F = v3(T.b.z, T.b.w, T.c.x);
                         const V3 G = sub3(v3(r0.x, r0.y, r0.z), v3(T.a.x, T.a.y, T.a.z));
@@ -604,9 +614,11 @@ __device__ __forceinline__ int warp_query(const KParams &P, const MeshView &M, c
                         const float t0 = dot3(GE, F);
                         const float d = fabsf(t0) * T.c.z - T.c.w * (fabsf(G.x) + fabsf(G.y) + fabsf(G.z));
                         atomicMin(&Q.safe[k], __float_as_uint(fmaxf(d, 0.0f)));
+                        // most triangles' planes lie beyond the step (d bounds the distance
+                        // from below, rounding included): nothing to hit
                         const int o = __float_as_int(T.c.y);
                         float t;
-                        if (o != __float_as_int(r1.w) &&
+                        if (d <= r1.z && o != __float_as_int(r1.w) &&
                             tri_hit(M, E, F, G, GE, t0, v3(r0.w, r1.x, r1.y), r1.z, t) && t <= r1.z)
                             atomicMin(&Q.best[k], ((unsigned long long)__float_as_uint(t) << 32) | (unsigned)o);
                     } else {
@@ -615,7 +627,9 @@ __device__ __forceinline__ int warp_query(const KParams &P, const MeshView &M, c
                 }
             }
             __syncwarp();
-            if (mine) limit = __uint_as_float((uint32_t)(Q.best[rank] >> 32));
+            if (!marching) break;
+            cnt = 0;
+            if (march) limit = __uint_as_float((uint32_t)(Q.best[rank] >> 32));
         }
         if (mine && !bvh) {
             const unsigned long long b = Q.best[rank];

@@ -49,14 +49,12 @@ constexpr size_t OFF_NODE_A = OFF_MEDIA + LP_NOALLOC_MAX_MEDIA * sizeof(Medium);
 constexpr size_t OFF_NODE_B = OFF_NODE_A + kMaxNodes * 16;
 constexpr size_t OFF_NODE_C = OFF_NODE_B + kMaxNodes * 16;
 constexpr size_t OFF_NODE_D = OFF_NODE_C + kMaxNodes * 16;
-constexpr size_t OFF_TRI_A = OFF_NODE_D + kMaxNodes * 16;
-constexpr size_t OFF_TRI_B = OFF_TRI_A + LP_NOALLOC_MAX_TRI * 16;
-constexpr size_t OFF_TRI_C = OFF_TRI_B + LP_NOALLOC_MAX_TRI * 16;
-constexpr size_t OFF_ATTR = OFF_TRI_C + LP_NOALLOC_MAX_TRI * 16;
+constexpr size_t OFF_TRI = OFF_NODE_D + kMaxNodes * 16;
+constexpr size_t OFF_ATTR = OFF_TRI + LP_NOALLOC_MAX_TRI * 48;
 constexpr size_t OFF_BOX = OFF_ATTR + LP_NOALLOC_MAX_TRI * 16;   // leaf and node boxes, 6 floats each
 constexpr size_t OFF_END = OFF_BOX + (size_t)(kMaxLeaves + kMaxNodes) * 24;
 static_assert(OFF_END <= LP_NOALLOC_SCRATCH_BYTES, "scratch layout exceeds the static array");
-static_assert(OFF_NODE_A % 16 == 0 && OFF_TRI_A % 16 == 0 && OFF_ATTR % 16 == 0, "float4 alignment");
+static_assert(OFF_NODE_A % 16 == 0 && OFF_TRI % 16 == 0 && OFF_ATTR % 16 == 0, "float4 alignment");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[LP_NOALLOC_SCRATCH_BYTES];
 
@@ -82,8 +80,7 @@ __global__ void __launch_bounds__(256) noalloc_setup_kernel(const float *tri, co
     float4 *na = reinterpret_cast<float4 *>(s + OFF_NODE_A), *nb = reinterpret_cast<float4 *>(s + OFF_NODE_B);
     float4 *nc = reinterpret_cast<float4 *>(s + OFF_NODE_C);
     int4 *nd = reinterpret_cast<int4 *>(s + OFF_NODE_D);
-    float4 *ta = reinterpret_cast<float4 *>(s + OFF_TRI_A), *tb = reinterpret_cast<float4 *>(s + OFF_TRI_B);
-    float4 *tc = reinterpret_cast<float4 *>(s + OFF_TRI_C), *at = reinterpret_cast<float4 *>(s + OFF_ATTR);
+    float4 *trec = reinterpret_cast<float4 *>(s + OFF_TRI), *at = reinterpret_cast<float4 *>(s + OFF_ATTR);
     float *box = reinterpret_cast<float *>(s + OFF_BOX);
     const int tid = threadIdx.x, bd = blockDim.x;
     for (int i = tid; i < mp.n; i += bd) {
@@ -111,9 +108,9 @@ __global__ void __launch_bounds__(256) noalloc_setup_kernel(const float *tri, co
         const float *t = tri + 9 * (int64_t)j;
         const float Ex = __fsub_rn(t[0], t[6]), Ey = __fsub_rn(t[1], t[7]), Ez = __fsub_rn(t[2], t[8]);
         const float Fx = __fsub_rn(t[3], t[6]), Fy = __fsub_rn(t[4], t[7]), Fz = __fsub_rn(t[5], t[8]);
-        ta[j] = make_float4(t[6], t[7], t[8], Ex);
-        tb[j] = make_float4(Ey, Ez, Fx, Fy);
-        tc[j] = make_float4(Fz, __int_as_float(j), 0.0f, 0.0f);
+        trec[3 * j] = make_float4(t[6], t[7], t[8], Ex);
+        trec[3 * j + 1] = make_float4(Ey, Ez, Fx, Fy);
+        trec[3 * j + 2] = make_float4(Fz, __int_as_float(j), 0.0f, 0.0f);
         float x = nrm[3 * (int64_t)j], y = nrm[3 * (int64_t)j + 1], z = nrm[3 * (int64_t)j + 2];
         const float l = __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)), __fmul_rn(z, z)));
         if (l != 0.0f) {
@@ -296,9 +293,7 @@ extern "C" int lp_run_noalloc(const lp_noalloc_args *a, void *stream)
     P.node_b = reinterpret_cast<const float4 *>(sb + OFF_NODE_B);
     P.node_c = reinterpret_cast<const float4 *>(sb + OFF_NODE_C);
     P.node_d = reinterpret_cast<const int4 *>(sb + OFF_NODE_D);
-    P.tri_a = reinterpret_cast<const float4 *>(sb + OFF_TRI_A);
-    P.tri_b = reinterpret_cast<const float4 *>(sb + OFF_TRI_B);
-    P.tri_c = reinterpret_cast<const float4 *>(sb + OFF_TRI_C);
+    P.tri = reinterpret_cast<const float4 *>(sb + OFF_TRI);
     P.tri_attr = reinterpret_cast<const float4 *>(sb + OFF_ATTR);
     P.n_nodes = NI;
     P.n_tri = (int32_t)a->n_tri;

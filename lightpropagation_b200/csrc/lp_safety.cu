@@ -80,7 +80,8 @@ __device__ float nearest_dist2(const KParams &P, V3 p, float cap2)
             if (ref[s] < 0) {
                 const int e = ~ref[s], f = e >> 3, cnt = (e & 7) + 1;
                 for (int j = f; j < f + cnt; ++j) {
-                    const float4 ta = __ldg(P.tri_a + j), tb = __ldg(P.tri_b + j), tc = __ldg(P.tri_c + j);
+                    const TriRec T = load_tri(P.tri, j);
+                    const float4 ta = T.a, tb = T.b, tc = T.c;
                     const float q = point_triangle_dist2(p, v3(ta.x, ta.y, ta.z), v3(ta.w, tb.x, tb.y),
                                                          v3(tb.z, tb.w, tc.x));
                     best = fminf(best, q);
@@ -234,7 +235,8 @@ __global__ void __launch_bounds__(256) cell_lists_kernel(const __grid_constant__
     const int lane = threadIdx.x & 31;
     const int n_warps = (gridDim.x * blockDim.x) >> 5;
     for (int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < n_tri; j += n_warps) {
-        const float4 ta = __ldg(P.tri_a + j), tb = __ldg(P.tri_b + j), tc = __ldg(P.tri_c + j);
+        const TriRec T = load_tri(P.tri, j);
+        const float4 ta = T.a, tb = T.b, tc = T.c;
         const V3 a = v3(ta.x, ta.y, ta.z);
         const V3 b = add3(a, v3(ta.w, tb.x, tb.y)), d = add3(a, v3(tb.z, tb.w, tc.x));
         const float lo[3] = {fminf(a.x, fminf(b.x, d.x)), fminf(a.y, fminf(b.y, d.y)), fminf(a.z, fminf(b.z, d.z))};

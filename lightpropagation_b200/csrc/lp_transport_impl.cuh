@@ -840,7 +840,7 @@ __device__ __forceinline__ bool step_photon(const KParams &P, const MeshView &M,
 }
 
 struct SmemLayout {
-    int off_media, off_region, off_cnt, off_na, off_nb, off_nc, off_nd, off_ta, off_tb, off_tc, bytes;
+    int off_media, off_region, off_cnt, off_na, off_nb, off_nc, off_nd, off_tri, bytes;
 };
 
 __host__ __device__ inline SmemLayout smem_layout(int nodes_smem, int tris_smem)
@@ -854,9 +854,7 @@ __host__ __device__ inline SmemLayout smem_layout(int nodes_smem, int tris_smem)
     L.off_nb = o; o += nodes_smem * 16;
     L.off_nc = o; o += nodes_smem * 16;
     L.off_nd = o; o += nodes_smem * 16;
-    L.off_ta = o; o += tris_smem * 16;
-    L.off_tb = o; o += tris_smem * 16;
-    L.off_tc = o; o += tris_smem * 16;
+    L.off_tri = o; o += tris_smem * 48;
     L.bytes = o;
     return L;
 }
@@ -865,22 +863,18 @@ __device__ __forceinline__ MeshView stage_mesh(const KParams &P, unsigned char *
 {
     MeshView M;
     M.na = P.node_a; M.nb = P.node_b; M.nc = P.node_c; M.nd = P.node_d;
-    M.ta = P.tri_a; M.tb = P.tri_b; M.tc = P.tri_c;
+    M.tri = P.tri;
     float4 *sa = reinterpret_cast<float4 *>(smem + L.off_na);
     float4 *sb = reinterpret_cast<float4 *>(smem + L.off_nb);
     float4 *sc = reinterpret_cast<float4 *>(smem + L.off_nc);
     int4 *sd = reinterpret_cast<int4 *>(smem + L.off_nd);
-    float4 *ta = reinterpret_cast<float4 *>(smem + L.off_ta);
-    float4 *tb = reinterpret_cast<float4 *>(smem + L.off_tb);
-    float4 *tc = reinterpret_cast<float4 *>(smem + L.off_tc);
+    float4 *tri = reinterpret_cast<float4 *>(smem + L.off_tri);
     for (int i = threadIdx.x; i < P.nodes_smem; i += blockDim.x) {
         sa[i] = P.node_a[i]; sb[i] = P.node_b[i]; sc[i] = P.node_c[i]; sd[i] = P.node_d[i];
     }
-    for (int i = threadIdx.x; i < P.tris_smem; i += blockDim.x) {
-        ta[i] = P.tri_a[i]; tb[i] = P.tri_b[i]; tc[i] = P.tri_c[i];
-    }
+    for (int i = threadIdx.x; i < 3 * P.tris_smem; i += blockDim.x) tri[i] = P.tri[i];
     M.s_na = sa; M.s_nb = sb; M.s_nc = sc; M.s_nd = sd;
-    M.s_ta = ta; M.s_tb = tb; M.s_tc = tc;
+    M.s_tri = tri;
     M.nodes_smem = P.nodes_smem;
     M.tris_smem = P.tris_smem;
     M.n_nodes = P.n_nodes;
