@@ -116,6 +116,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_kernel(const __grid_constan
     GradAcc ga;
     uint32_t next_draw = 0;
     ph.idx = ph.steps = 0;
+    ph.curr = 0;
     bool alive = false;
     const unsigned lanes = __popc(B.lane_mask);
     int inst = -1, from;   // from: where the search for the next instance begins

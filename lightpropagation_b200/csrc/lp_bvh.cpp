@@ -381,7 +381,6 @@ void build_bvh(const float *tri, int64_t n, Bvh &out, int leaf_target, int threa
     out.tri_a.resize((size_t)n);
     out.tri_b.resize((size_t)n);
     out.tri_c.resize((size_t)n);
-    out.tri.resize((size_t)n * 3);
     for (int64_t j = 0; j < n; ++j) {
         const int32_t oi = pr[(size_t)j].id;
         const float *t = tri + 9 * (int64_t)oi;
@@ -406,9 +405,6 @@ void build_bvh(const float *tri, int64_t n, Bvh &out, int leaf_target, int threa
         out.tri_a[j] = {t[6], t[7], t[8], Ex};
         out.tri_b[j] = {Ey, Ez, Fx, Fy};
         out.tri_c[j] = {Fz, ob, inv_n, kappa};
-        out.tri[3 * j] = out.tri_a[j];
-        out.tri[3 * j + 1] = out.tri_b[j];
-        out.tri[3 * j + 2] = out.tri_c[j];
     }
 }
 

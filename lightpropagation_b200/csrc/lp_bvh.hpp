@@ -32,7 +32,6 @@ struct Bvh {
     std::vector<F4> node_a, node_b, node_c;
     std::vector<I4> node_d;
     std::vector<F4> tri_a, tri_b, tri_c;
-    std::vector<F4> tri;   // the three of each triangle together, as the device reads them
     int32_t depth = 0;
     float margin = 0.0f;
     float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};

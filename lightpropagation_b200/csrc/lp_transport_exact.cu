@@ -51,6 +51,13 @@ __global__ void __launch_bounds__(kBlock) query_kernel(const __grid_constant__ K
     }
 }
 
+// out[3 i + k] = soa[k n + i], k < 3.
+__global__ void __launch_bounds__(256) interleave_kernel(const float4 *soa, int64_t n, float4 *out)
+{
+    for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < 3 * n; x += (int64_t)gridDim.x * blockDim.x)
+        out[x] = soa[(x % 3) * n + x / 3];
+}
+
 // dst[k][i] += the sum of part[k][0..copies)[i], and the copies are left at zero for the
 // next launch.  k < images, i < n.  Bound by the bytes of the copies (HBM or L2).
 __global__ void __launch_bounds__(256) fold_kernel(unsigned long long *dst, unsigned long long *part, int copies,
@@ -129,6 +136,13 @@ cudaError_t launch_query(const KParams &P, int smem, int64_t n, const float *ori
     int grid = (int)std::min<int64_t>((n + kBlock - 1) / kBlock, 148 * 8);
     if (grid < 1) grid = 1;
     query_kernel<<<grid, kBlock, smem, s>>>(P, n, orig, dir, ref, tmax, id_out, t_out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_interleave(const float4 *soa, int64_t n, float4 *out, cudaStream_t s)
+{
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((3 * n + 255) / 256, 148 * 8));
+    interleave_kernel<<<grid, 256, 0, s>>>(soa, n, out);
     return cudaGetLastError();
 }
 

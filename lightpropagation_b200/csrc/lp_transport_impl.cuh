@@ -28,9 +28,10 @@
 // implies; no branch between the move and the deposits (square roots without a slow path,
 // no test for a voxel grid), so that the chains of direction, tallies and the next cell
 // word overlap; and random numbers drawn several events ahead once lanes are idle
-// (next_draws).  One photon alone takes 0.79 us a step on the slab (1.20 before these),
-// 0.89 on the curved abdomen (1.36); slab, 1e6 photons, 114 -> 97 ms; abdomen at 660 nm,
-// 3e6 photons, 201 -> 181 ms; 1e5 photons 40 -> 29 ms.
+// (next_draws); the lanes without a photon run along, and rare ends (roulette, step cap)
+// share one branch.  One photon alone takes 0.65 us a step on the slab (1.20 before these),
+// 0.73 on the curved abdomen (1.36); slab, 1e6 photons, 114 -> 90 ms; abdomen at 660 nm,
+// 3e6 photons, 201 -> 175 ms; 1e5 photons 40 -> 24 ms.
 //
 // Exact = true  keeps the reference's arithmetic operation by operation (compiled
 //               with --fmad=false): a photon follows the oracle's trajectory for the
@@ -226,15 +227,17 @@ __device__ __forceinline__ Draws next_draws(const KParams &P, WarpDraws &W, unsi
             __syncwarp();
         }
     }
-    if (next >= 256u) {
-        const uint32_t s = next & 31u;
-        next += 1u - 256u;
-        d.neg_log = W.v[0][s];
-        d.u1 = W.v[1][s];
-        d.cos_psi = W.v[2][s];
-        d.sin_psi = W.v[3][s];
-        d.u3 = W.v[4][s];
-    }
+    // read and selected on every step: cheaper for the last photons than a branch (1000 slab
+    // photons 10.5 -> 9.9 ms), and as good for full warps
+    const uint32_t s = next & 31u;
+    const bool shared = next >= 256u;
+    const Draws e = {W.v[0][s], W.v[1][s], W.v[2][s], W.v[3][s], W.v[4][s]};
+    next += shared ? 1u - 256u : 0u;
+    d.neg_log = shared ? e.neg_log : d.neg_log;
+    d.u1 = shared ? e.u1 : d.u1;
+    d.cos_psi = shared ? e.cos_psi : d.cos_psi;
+    d.sin_psi = shared ? e.sin_psi : d.sin_psi;
+    d.u3 = shared ? e.u3 : d.u3;
     return d;
 }
 
@@ -618,59 +621,10 @@ static __device__ __forceinline__ Photon boundary_event(const KParams &P, const 
     return ph;
 }
 
-// A step in three parts: propose_step forms the step length from the event's draws and
-// decides whether the step can reach a triangle; query_step finds the nearest
-// triangle within reach; complete_step moves the photon (boundary event, or absorption and
-// scattering), scores it and plays roulette.  One call of each in turn is one iteration of
-// the reference's do-while loop (.cl:1388-1600).  (Letting the lanes whose step needs a
-// query wait until several of a warp do, and running their queries together, measured
-// slower on every batch size: the waiting lanes cost more steps per warp iteration than
-// the shared queries save.)
+// The step a photon is on: its length and reach, and the distance bound at the position.
 struct Pending {
-    float step, reach, safe_here;   // step length, its reach, distance bound at the position
+    float step, reach, safe_here;
 };
-enum : int { kStepEnded = 0, kStepClear = 1, kStepQuery = 2 };
-
-// kStepQuery: the step may reach a triangle and needs a query; kStepClear: no triangle
-// lies within its reach (complete_step with tri = -1); kStepEnded: the photon ended
-// (debug build: a region id out of range).
-template <bool Exact>
-__device__ __forceinline__ int propose_step(const KParams &P, const Medium *s_media, float neg_log, Photon &ph,
-                                            Pending &pd)
-{
-    [[maybe_unused]] unsigned long long *const dbg = P.counters ? P.counters + kBoundsCounter : nullptr;
-    if (!LP_IN_RANGE(dbg, ph.curr, P.n_media)) {
-        ph.w = 0.0f;
-        return kStepEnded;
-    }
-    const Medium &m = s_media[ph.curr];
-    const bool ambient = (m.kind & kAmbient) != 0;
-    // the residual of a step cut short by a boundary, or a new step; both are formed, and
-    // the select costs less than the branch
-    float step;
-    if (Exact) step = (ph.unfin == 0.0f) ? neg_log * P.factor / m.mut : ph.unfin / m.mut;
-    else step = (ph.unfin == 0.0f) ? neg_log * P.factor * m.inv_mut : ph.unfin * m.inv_mut;
-    if (ambient) step = 0.0f;
-    ph.unfin = 0.0f;
-    pd.step = step;
-    // reach: the production arithmetic also takes a face that lies up to a few rounding
-    // units beyond the step as the step's boundary.  A hit computed just past the step
-    // although it lies just within it would otherwise let the photon end its step on the
-    // far side of the face, outside the region it is labelled with.  The photon then stops
-    // on the face (and is moved off it, see boundary_event) with no residual step.
-    const float reach = Exact ? step : step + P.boundary_push + 1e-6f * step;
-    pd.reach = reach;
-    // safe_here: lower bound of the distance from p to every triangle.  A step shorter
-    // than it cannot reach one, so its bounded query would return "no hit" and is skipped;
-    // after the step the bound shrinks by the step (plus the rounding of the move).
-    pd.safe_here = ph.safe;
-    if (ambient) return kStepQuery;
-    if (reach < pd.safe_here) return kStepClear;
-    // a cell no triangle touches: its word holds a bound for all its points (the larger of
-    // two lower bounds is one too); safe_distance is 0 for the others
-    pd.safe_here = fmaxf(pd.safe_here, safe_distance(P, ph.word));
-    return reach < pd.safe_here ? kStepClear : kStepQuery;
-}
 
 // The nearest triangle within the step's reach (-1: none) and its distance thit; updates
 // the distance bound the query establishes.  Every lane of the warp calls it, the ones
@@ -694,125 +648,100 @@ __device__ __forceinline__ int query_step(const KParams &P, const MeshView &M, c
     return tri;
 }
 
-// Returns false when the photon ends.  Agg: absorption deposits summed per cell across
-// the warp before the atomic adds.  rz_copy: first cell of the block's copy of the r-z
-// image (rz_copy_of).
-template <bool Exact, bool Grad, bool Agg = false>
-__device__ __forceinline__ bool complete_step(const KParams &P, const Medium *s_media, unsigned long long *s_region,
-                                              unsigned long long *s_cnt, Photon &ph, Counters &cnt, GradAcc *ga,
-                                              const Pending &pd, const Draws &d, int tri, float thit, uint32_t rz_copy)
+// A scatter event: moves the photon by `step`, absorbs, scatters and adds the deposit to the
+// tallies.  Agg: deposits summed per cell across the warp before the atomic adds.  rz_copy:
+// first cell of the block's copy of the r-z image (rz_copy_of).
+template <bool Exact, bool Grad, bool Agg>
+__device__ __forceinline__ void scatter_event(const KParams &P, const Medium &m, unsigned long long *s_cnt, Photon &ph,
+                                              Counters &cnt, float step, float safe_here, const Draws &d,
+                                              uint32_t rz_copy)
 {
-    const Medium &m = s_media[ph.curr];
-    const bool ambient = (m.kind & kAmbient) != 0;
     const V3 v = v3(ph.vx, ph.vy, ph.vz);
-    const float step = ambient ? thit : pd.step;
-    // a query returns no hit beyond the step's reach
-    const bool boundary = tri >= 0 || kNoHit <= step;
-    if (boundary) {
-        cnt.boundary++;
-        ph = boundary_event<Exact, Grad>(P, s_media, s_region, s_cnt, ph, Grad ? ga : nullptr, tri, thit, step, d.u1);
-        ph.word = cell_at(P, ph.px, ph.py, ph.pz);
+    ph.px = ph.px + step * ph.vx;
+    ph.py = ph.py + step * ph.vy;
+    ph.pz = ph.pz + step * ph.vz;
+    // the next step's cell word: its load is in flight during the rest of this step
+    ph.word = cell_at(P, ph.px, ph.py, ph.pz);
+    ph.flags &= ~F_ON_FACE;
+    ph.safe = fmaxf(safe_here - step - P.step_eps, 0.0f);
+    if (Grad) {
+        ph.seg_len += step;
+        ph.seg_k++;
+    }
+    const bool absorbs = (m.kind & kAbsorbs) != 0;
+    ph.absorbed = absorbs ? ph.w * m.alb : ph.absorbed;
+    ph.w = absorbs ? ph.w - ph.absorbed : ph.w;
+    const V3 vn = scatter_direction<Exact>(v, m, d.u1, d.cos_psi, d.sin_psi);
+    ph.vx = vn.x; ph.vy = vn.y; ph.vz = vn.z;
+    const V3 pr = v3(ph.px - P.poix, ph.py - P.poiy, ph.pz - P.poiz);
+    const float cx = dot3(v3(P.nxx, P.nxy, P.nxz), pr);
+    const float cy = dot3(v3(P.nyx, P.nyy, P.nyz), pr);
+    const float cz = dot3(v3(P.nzx, P.nzy, P.nzz), pr);
+    const float dw = ph.absorbed;
+    const unsigned long long fdw = fix32(dw);
+    // r-z grid (RecordAbsorbtionRZ, .cl:254-271, with atomic adds and z rows)
+    int row, col;
+    if (Exact) {
+        const float rad = sqrtf(cx * cx + cy * cy) * sign_cl(cx) / P.dg[3];
+        row = (int)floorf(cz / P.dg[2]);
+        col = (int)floorf(rad + P.f_dimR);
     } else {
-        ph.px = ph.px + step * ph.vx;
-        ph.py = ph.py + step * ph.vy;
-        ph.pz = ph.pz + step * ph.vz;
-        // the next step's cell word: its load is in flight during the rest of this step
-        ph.word = cell_at(P, ph.px, ph.py, ph.pz);
-        ph.flags &= ~F_ON_FACE;
-        ph.safe = fmaxf(pd.safe_here - step - P.step_eps, 0.0f);
-        if (Grad) {
-            ph.seg_len += step;
-            ph.seg_k++;
-        }
-        const bool absorbs = (m.kind & kAbsorbs) != 0;
-        ph.absorbed = absorbs ? ph.w * m.alb : ph.absorbed;
-        ph.w = absorbs ? ph.w - ph.absorbed : ph.w;
-        const V3 vn = scatter_direction<Exact>(v, m, d.u1, d.cos_psi, d.sin_psi);
-        ph.vx = vn.x; ph.vy = vn.y; ph.vz = vn.z;
-        const V3 pr = v3(ph.px - P.poix, ph.py - P.poiy, ph.pz - P.poiz);
-        const float cx = dot3(v3(P.nxx, P.nxy, P.nxz), pr);
-        const float cy = dot3(v3(P.nyx, P.nyy, P.nyz), pr);
-        const float cz = dot3(v3(P.nzx, P.nzy, P.nzz), pr);
-        const float dw = ph.absorbed;
-        const unsigned long long fdw = fix32(dw);
-        // r-z grid (RecordAbsorbtionRZ, .cl:254-271, with atomic adds and z rows)
-        int row, col;
-        if (Exact) {
-            const float rad = sqrtf(cx * cx + cy * cy) * sign_cl(cx) / P.dg[3];
-            row = (int)floorf(cz / P.dg[2]);
-            col = (int)floorf(rad + P.f_dimR);
-        } else {
-            const float rad = copysignf(sqrt_normal(cx * cx + cy * cy), cx) * P.inv_dr;
-            row = (int)floorf(cz * P.inv_dz);
-            col = (int)floorf(rad + P.f_dimR);
-        }
-        const bool rz_in = ((unsigned)row < (unsigned)P.rz_nz) & ((unsigned)col < (unsigned)P.rz_nr);
-        // inv_mua is 0 where mua is not positive
-        const unsigned long long fdm = Exact ? (m.mua > 0.0f ? fix32(dw / m.mua) : 0ull) : fix32(dw * m.inv_mua);
-        int ix, iy, iz;
-        if (Exact) {
-            ix = (int)floorf(cx / P.vox_dx + P.half_vnx);
-            iy = (int)floorf(cy / P.vox_dy + P.half_vny);
-            iz = (int)floorf(cz / P.vox_dz);
-        } else {
-            ix = (int)floorf(cx * P.inv_vdx + P.half_vnx);
-            iy = (int)floorf(cy * P.inv_vdy + P.half_vny);
-            iz = (int)floorf(cz * P.inv_vdz);
-        }
-        // never in without a voxel grid (vox_nx = 0), and then no drop either
-        const bool vox_in = ((unsigned)ix < (unsigned)P.vox_nx) & ((unsigned)iy < (unsigned)P.vox_ny) &
-                            ((unsigned)iz < (unsigned)P.vox_nz);
-        const int vox_key = vox_in ? (iz * P.vox_ny + iy) * P.vox_nx + ix : -1;
-        cnt.vox_drop += vox_in ? 0u : P.vox_on;
-        cnt.rz_drop += rz_in ? 0u : 1u;
-        const int rz_key = rz_in ? row * P.rz_nr + col : -1;
-        unsigned long long *const rz = P.rz_part + 2 * (int64_t)rz_copy;
-        if (Agg) {
-            // warp-aggregated deposits: the lanes of this branch that hit the same cell
-            // are matched, their fixed-point values summed exactly, and one leader per
-            // cell issues the atomic add (integer sums: same tallies as the plain form)
-            const unsigned lane = threadIdx.x & 31u;
-            const unsigned act = __activemask();
-            const unsigned g_rz = __match_any_sync(act, rz_key);
-            if (rz_key >= 0) {
-                const unsigned long long a = group_sum_u64(g_rz, fdw), b = group_sum_u64(g_rz, fdm);
-                if (lane == (unsigned)(__ffs(g_rz) - 1)) {
-                    unsigned long long *c = rz + 2 * (int64_t)rz_key;
-                    if (a) atomicAdd(c, a);
-                    if (b) atomicAdd(c + 1, b);
-                    atomicAdd(s_cnt + 15, 1ull);   // leaders: 1 - leaders / deposits is the match rate
-                }
-            }
-            const unsigned g_vox = __match_any_sync(act, vox_key);
-            if (vox_key >= 0) {
-                const unsigned long long a = group_sum_u64(g_vox, fdw);
-                if (a && lane == (unsigned)(__ffs(g_vox) - 1)) atomicAdd(P.vox + vox_key, a);
-            }
-        } else {
-            // a weight that rounds to 0 is rare, and adding it is cheaper than the test
-            if (rz_key >= 0) {
+        const float rad = copysignf(sqrt_normal(cx * cx + cy * cy), cx) * P.inv_dr;
+        row = (int)floorf(cz * P.inv_dz);
+        col = (int)floorf(rad + P.f_dimR);
+    }
+    const bool rz_in = ((unsigned)row < (unsigned)P.rz_nz) & ((unsigned)col < (unsigned)P.rz_nr);
+    // inv_mua is 0 where mua is not positive
+    const unsigned long long fdm = Exact ? (m.mua > 0.0f ? fix32(dw / m.mua) : 0ull) : fix32(dw * m.inv_mua);
+    int ix, iy, iz;
+    if (Exact) {
+        ix = (int)floorf(cx / P.vox_dx + P.half_vnx);
+        iy = (int)floorf(cy / P.vox_dy + P.half_vny);
+        iz = (int)floorf(cz / P.vox_dz);
+    } else {
+        ix = (int)floorf(cx * P.inv_vdx + P.half_vnx);
+        iy = (int)floorf(cy * P.inv_vdy + P.half_vny);
+        iz = (int)floorf(cz * P.inv_vdz);
+    }
+    // never in without a voxel grid (vox_nx = 0), and then no drop either
+    const bool vox_in = ((unsigned)ix < (unsigned)P.vox_nx) & ((unsigned)iy < (unsigned)P.vox_ny) &
+                        ((unsigned)iz < (unsigned)P.vox_nz);
+    const int vox_key = vox_in ? (iz * P.vox_ny + iy) * P.vox_nx + ix : -1;
+    cnt.vox_drop += vox_in ? 0u : P.vox_on;
+    cnt.rz_drop += rz_in ? 0u : 1u;
+    const int rz_key = rz_in ? row * P.rz_nr + col : -1;
+    unsigned long long *const rz = P.rz_part + 2 * (int64_t)rz_copy;
+    if (Agg) {
+        // warp-aggregated deposits: the lanes of this branch that hit the same cell
+        // are matched, their fixed-point values summed exactly, and one leader per
+        // cell issues the atomic add (integer sums: same tallies as the plain form)
+        const unsigned lane = threadIdx.x & 31u;
+        const unsigned act = __activemask();
+        const unsigned g_rz = __match_any_sync(act, rz_key);
+        if (rz_key >= 0) {
+            const unsigned long long a = group_sum_u64(g_rz, fdw), b = group_sum_u64(g_rz, fdm);
+            if (lane == (unsigned)(__ffs(g_rz) - 1)) {
                 unsigned long long *c = rz + 2 * (int64_t)rz_key;
-                atomicAdd(c, fdw);
-                atomicAdd(c + 1, fdm);
+                if (a) atomicAdd(c, a);
+                if (b) atomicAdd(c + 1, b);
+                atomicAdd(s_cnt + 15, 1ull);   // leaders: 1 - leaders / deposits is the match rate
             }
-            if (vox_key >= 0) atomicAdd(P.vox + vox_key, fdw);
         }
-        ph.region_acc += fdw;
-    }
-    if (ph.w < P.w_th && ph.w > 0.0f) {
-        cnt.roulette++;
-        if (d.u3 < P.chance) {
-            ph.w /= P.chance;
-        } else {
-            ph.w = 0.0f;
+        const unsigned g_vox = __match_any_sync(act, vox_key);
+        if (vox_key >= 0) {
+            const unsigned long long a = group_sum_u64(g_vox, fdw);
+            if (a && lane == (unsigned)(__ffs(g_vox) - 1)) atomicAdd(P.vox + vox_key, a);
         }
+    } else {
+        // a weight that rounds to 0 is rare, and adding it is cheaper than the test
+        if (rz_key >= 0) {
+            unsigned long long *c = rz + 2 * (int64_t)rz_key;
+            atomicAdd(c, fdw);
+            atomicAdd(c + 1, fdm);
+        }
+        if (vox_key >= 0) atomicAdd(P.vox + vox_key, fdw);
     }
-    ph.steps++;
-    if (ph.steps >= P.step_cap && ph.w > 0.0f) {
-        atomicAdd(s_cnt + 5, 1ull);
-        ph.w = 0.0f;
-    }
-    return ph.w > 0.0f;
+    ph.region_acc += fdw;
 }
 
 __device__ __forceinline__ uint32_t rz_copy_of(const KParams &P)
@@ -820,23 +749,72 @@ __device__ __forceinline__ uint32_t rz_copy_of(const KParams &P)
     return (blockIdx.x & P.rz_mask) * (uint32_t)(P.rz_stride >> 1);
 }
 
-// One iteration of the reference's do-while loop, the three parts in turn, for the warp's
-// photons (the whole warp calls it; `live` has the lanes with one, `alive` is the lane's bit).  Returns false when the
-// lane's photon ends.
+// One iteration of the reference's do-while loop (.cl:1388-1600) for the warp's photons
+// (the whole warp calls it; `live` has the lanes with one, `alive` is the lane's bit): step
+// length, query if the step may reach a triangle, boundary event or scatter event, roulette.
+// Returns false when the lane's photon ends.  Lanes without a photon compute the step length
+// too: a branch around it costs every step more.  (Letting the lanes whose step needs a
+// query wait until several of a warp do, and running their queries together, measured
+// slower on every batch size: the waiting lanes cost more steps than the shared queries
+// save.)
 template <bool Exact, bool Grad, int STACK = kStackDepth, bool Agg = false>
 __device__ __forceinline__ bool step_photon(const KParams &P, const MeshView &M, const MeshView &SM, WarpQueue &Q,
                                             const Medium *s_media, unsigned long long *s_region,
-                                            unsigned long long *s_cnt, unsigned live, bool alive, Photon &ph, Counters &cnt,
-                                            GradAcc *ga, WarpDraws &W, uint32_t &next, uint32_t rz_copy)
+                                            unsigned long long *s_cnt, unsigned live, bool alive, Photon &ph,
+                                            Counters &cnt, GradAcc *ga, WarpDraws &W, uint32_t &next, uint32_t rz_copy)
 {
     const Draws d = next_draws<Exact>(P, W, live, alive, ph.idx, ph.steps, next);
+    [[maybe_unused]] unsigned long long *const dbg = P.counters ? P.counters + kBoundsCounter : nullptr;
+    // debug build: a region id out of range ends the photon
+    if (alive && !LP_IN_RANGE(dbg, ph.curr, P.n_media)) {
+        ph.w = 0.0f;
+        ph.curr = 0;
+        alive = false;
+    }
+    const Medium &m = s_media[ph.curr];
+    const bool ambient = (m.kind & kAmbient) != 0;
+    // the residual of a step cut short by a boundary, or a new step
     Pending pd;
-    int st = kStepEnded;
-    if (alive) st = propose_step<Exact>(P, s_media, d.neg_log, ph, pd);
+    const float optical = (ph.unfin == 0.0f) ? d.neg_log * P.factor : ph.unfin;
+    pd.step = Exact ? optical / m.mut : optical * m.inv_mut;
+    if (ambient) pd.step = 0.0f;
+    ph.unfin = alive ? 0.0f : ph.unfin;
+    // reach: the production arithmetic also takes a face that lies up to a few rounding
+    // units beyond the step as the step's boundary.  A hit computed just past the step
+    // although it lies just within it would otherwise let the photon end its step on the
+    // far side of the face, outside the region it is labelled with.  The photon then stops
+    // on the face (and is moved off it, see boundary_event) with no residual step.
+    pd.reach = Exact ? pd.step : pd.step + P.boundary_push + 1e-6f * pd.step;
+    // safe_here: lower bound of the distance from p to every triangle, the larger of the
+    // carried one and that of a cell no triangle touches (safe_distance is 0 for the others).
+    // A step shorter than it cannot reach a triangle, so its bounded query would return "no
+    // hit" and is skipped; after the step the bound shrinks by the step (plus the rounding of
+    // the move).
+    pd.safe_here = fmaxf(ph.safe, safe_distance(P, ph.word));
+    const bool want = alive && (ambient || !(pd.reach < pd.safe_here));
     float thit;
-    const int tri = query_step<STACK>(P, M, SM, Q, s_media, st == kStepQuery, ph, cnt, pd, thit);
-    if (st == kStepEnded) return false;
-    return complete_step<Exact, Grad, Agg>(P, s_media, s_region, s_cnt, ph, cnt, ga, pd, d, tri, thit, rz_copy);
+    const int tri = query_step<STACK>(P, M, SM, Q, s_media, want, ph, cnt, pd, thit);
+    const float step = ambient ? thit : pd.step;
+    // a query returns no hit beyond the step's reach
+    if (alive && (tri >= 0 || kNoHit <= step)) {
+        cnt.boundary++;
+        ph = boundary_event<Exact, Grad>(P, s_media, s_region, s_cnt, ph, Grad ? ga : nullptr, tri, thit, step, d.u1);
+        ph.word = cell_at(P, ph.px, ph.py, ph.pz);
+    } else if (alive) {
+        scatter_event<Exact, Grad, Agg>(P, m, s_cnt, ph, cnt, step, pd.safe_here, d, rz_copy);
+    }
+    ph.steps += alive ? 1u : 0u;
+    if (alive && (ph.w < P.w_th || ph.steps >= P.step_cap)) {
+        if (ph.w < P.w_th && ph.w > 0.0f) {
+            cnt.roulette++;
+            ph.w = d.u3 < P.chance ? ph.w / P.chance : 0.0f;
+        }
+        if (ph.steps >= P.step_cap && ph.w > 0.0f) {
+            atomicAdd(s_cnt + 5, 1ull);
+            ph.w = 0.0f;
+        }
+    }
+    return ph.w > 0.0f;
 }
 
 struct SmemLayout {
@@ -915,6 +893,7 @@ __global__ void __launch_bounds__(kBlock, LP_TRANSPORT_MIN_BLOCKS) transport_ker
     bool alive = false;
     bool exhausted = false;
     ph.idx = ph.steps = 0;
+    ph.curr = 0;
     for (;;) {
         unsigned live = __ballot_sync(0xffffffffu, alive);
         if (live != P.lane_mask && !exhausted) {
