@@ -39,12 +39,10 @@ cudaError_t launch_query(const KParams &P, int smem, int64_t n, const float *ori
                          cudaStream_t s);
 cudaError_t launch_philox(const uint32_t *ctr, const uint32_t *key, int64_t n, uint32_t *out,
                           cudaStream_t s);
-cudaError_t launch_safety_grid(const KParams &P, float h, float half_diag, float eps, float cap, float *const *levels,
-                               int n_levels, uint16_t *out, cudaStream_t s);
 cudaError_t launch_cell_lists(const KParams &P, int n_tri, float h, float eps, uint32_t *count, const uint32_t *start,
                               int32_t *refs, cudaStream_t s);
-cudaError_t launch_cell_words(int64_t n, const uint16_t *safe, const uint32_t *count, const uint32_t *start, bool lists,
-                              uint32_t *word, cudaStream_t s);
+cudaError_t launch_cell_words(const KParams &P, float m, const uint32_t *count, const uint32_t *start, bool lists,
+                              uint8_t *gap, float *d2, uint32_t *word, cudaStream_t s);
 cudaError_t launch_interleave(const float4 *soa, int64_t n, float4 *out, cudaStream_t s);
 cudaError_t launch_fold(unsigned long long *dst, unsigned long long *part, int copies, int64_t n, int64_t images,
                         cudaStream_t s);
@@ -255,7 +253,10 @@ struct lp_ctx {
     int64_t n_cell_refs = 0;
     float g_origin[3] = {0, 0, 0}, g_h = 0, g_unit = 0, g_eps = 0, g_step_eps = 0, g_push = 0;
     // lists hold the triangles touching each cell widened by cell_margin cells on every side
+    // by default half a cell, or three quarters where the triangles are large (build_safety_grid)
     float cell_margin = 0.5f;
+    bool margin_set = false;   // lp_set_cell_margin
+    float grid_margin = 0.5f;  // the built grid's
     bool agg_tallies = false;   // lp_set_tally_aggregation
     int32_t g_n[3] = {0, 0, 0};
     float grid_ms = 0;
@@ -587,7 +588,7 @@ void fill_params(lp_ctx *c, KParams &P, int64_t first, int64_t n, int nodes_smem
     P.g_ny = grid ? c->g_n[1] : 0;
     P.g_nz = grid ? c->g_n[2] : 0;
     P.g_h = c->g_h;
-    P.g_margin = c->cell_margin * c->g_h;
+    P.g_margin = c->grid_margin * c->g_h;
     P.step_eps = c->g_step_eps;
     P.boundary_push = c->exact ? 0.0f : c->g_push;
     P.tri_eps = c->exact ? 0.0f : 2e-6f;
@@ -595,21 +596,20 @@ void fill_params(lp_ctx *c, KParams &P, int64_t first, int64_t n, int nodes_smem
 }
 
 // Cell grid over the mesh bounds padded by one cell: cubic cells of size h chosen so
-// the grid has at most grid_max_cells cells; safety bounds in units of h / 256.
-//   1. safety_level_kernel: per cell, a lower bound of the distance to the nearest
-//      triangle, from blocks of 8, 4 and 2 cells per edge down to cells;
-//   2. cell_lists_kernel (count pass): per cell, the triangles touching it;
-//   3. exclusive scan of the counts: each cell's first slot in cell_refs;
-//   4. cell_lists_kernel (fill pass): the triangle indices;
-//   5. cell_word_kernel: one word per cell (KParams::cell_word).
+// the grid has at most grid_max_cells cells; distance bounds in units of h / 256.
+//   1. cell_lists_kernel (count pass): per cell, the triangles touching it;
+//   2. exclusive scan of the counts: each cell's first slot in cell_refs;
+//   3. cell_lists_kernel (fill pass): the triangle indices;
+//   4. launch_cell_words: the distance bounds of the empty cells, and one word per cell
+//      (KParams::cell_word).
 int build_safety_grid(lp_ctx *c)
 {
     Phase phase("lp cell grid build");
-    c->grid_dirty = false;
     c->n_cell_refs = 0;
     if (c->grid_max_cells <= 0 || c->n_tri == 0) {
         c->cell_word.release();
         c->cell_refs.release();
+        c->grid_dirty = false;
         return LP_OK;
     }
     const lp::Bvh &b = c->bvh;
@@ -641,12 +641,18 @@ int build_safety_grid(lp_ctx *c)
     // component; 5e-7 * scale is about 4 ulp (2^-23 = 1.19e-7)
     c->g_step_eps = (float)(5e-7 * scale);
     for (int a = 0; a < 3; ++a) c->g_origin[a] = (float)(b.lo[a] - h);
-    DevBuf<uint16_t> safe;
-    DevBuf<float> level[4];   // block distances of the safety grid's levels 1..3
-    DevBuf<uint32_t> count, start;
-    DevBuf<unsigned char> scan_tmp;
-    LP_CUDA(c, safe.ensure((size_t)cells));
+    // scratch of the build, in one allocation: counts, offsets, bounds, row gaps, scan
+    size_t tmp_bytes = 0;
+    cudaStream_t s = c->stream;
+    LP_CUDA(c, cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, (uint32_t *)nullptr, (uint32_t *)nullptr, cells, s));
+    const size_t n_cells = ((size_t)cells + 255) & ~(size_t)255;
     LP_CUDA(c, c->cell_word.ensure((size_t)cells));
+    DevBuf<unsigned char> scratch;
+    LP_CUDA(c, scratch.ensure(n_cells * 13 + tmp_bytes));
+    uint32_t *const count = reinterpret_cast<uint32_t *>(scratch.p), *const start = count + n_cells;
+    float *const d2 = reinterpret_cast<float *>(start + n_cells);
+    uint8_t *const gap = reinterpret_cast<uint8_t *>(d2 + n_cells);
+    void *const scan_tmp = gap + n_cells;
     KParams P;
     std::memset(&P, 0, sizeof P);
     P.node_a = c->node_a.p; P.node_b = c->node_b.p; P.node_c = c->node_c.p; P.node_d = c->node_d.p;
@@ -655,62 +661,51 @@ int build_safety_grid(lp_ctx *c)
     P.g_nx = c->g_n[0]; P.g_ny = c->g_n[1]; P.g_nz = c->g_n[2];
     P.g_unit = c->g_unit;
     P.g_inv_h = 1.0f / c->g_h;
-    // eps: far above the few-ulp overreach of the ray/triangle test at this scale
-    const float eps = (float)(1e-4 * scale);
-    cudaStream_t s = c->stream;
+    P.g_h = c->g_h;
+    P.g_eps = c->g_eps;
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventRecord(e0, s);
-    // levels of blocks of 2, 4 and 8 cells per edge above the cells (fewer on small grids)
-    int n_levels = 0;
-    cudaError_t e = cudaSuccess;
-    float *lv[4] = {nullptr, nullptr, nullptr, nullptr};
-    while (n_levels < 3 && e == cudaSuccess) {
-        const int L = n_levels + 1;
-        const int64_t nb = (int64_t)((c->g_n[0] + (1 << L) - 1) >> L) * ((c->g_n[1] + (1 << L) - 1) >> L) *
-                           ((c->g_n[2] + (1 << L) - 1) >> L);
-        if (nb < 512) break;
-        e = level[L].ensure((size_t)nb);
-        lv[L] = level[L].p;
-        ++n_levels;
-    }
-    if (e == cudaSuccess)
-        e = lp::launch_safety_grid(P, (float)h, (float)(h * std::sqrt(3.0) / 2.0), eps, (float)(64.0 * h), lv, n_levels,
-                                   safe.p, s);
     bool lists = false;
+    const int nt = (int)c->bvh.tri_a.size();
+    c->grid_margin = c->cell_margin;
     // every list holds the triangles that touch its cell widened by the margin plus g_eps
-    const float list_eps = c->cell_margin * c->g_h + c->g_eps;
-    if (e == cudaSuccess && c->cell_lists) {
-        const int nt = (int)c->bvh.tri_a.size();
-        size_t tmp_bytes = 0;
-        if ((e = count.ensure((size_t)cells)) == cudaSuccess && (e = start.ensure((size_t)cells)) == cudaSuccess &&
-            (e = cudaMemsetAsync(count.p, 0, (size_t)cells * 4, s)) == cudaSuccess &&
-            (e = lp::launch_cell_lists(P, nt, c->g_h, list_eps, count.p, nullptr, nullptr, s)) == cudaSuccess &&
-            (e = cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, count.p, start.p, cells, s)) == cudaSuccess &&
-            (e = scan_tmp.ensure(tmp_bytes)) == cudaSuccess &&
-            (e = cub::DeviceScan::ExclusiveSum(scan_tmp.p, tmp_bytes, count.p, start.p, cells, s)) == cudaSuccess) {
-            uint32_t last[2] = {0, 0};
-            if ((e = cudaMemcpyAsync(&last[0], start.p + cells - 1, 4, cudaMemcpyDeviceToHost, s)) == cudaSuccess &&
-                (e = cudaMemcpyAsync(&last[1], count.p + cells - 1, 4, cudaMemcpyDeviceToHost, s)) == cudaSuccess &&
-                (e = cudaStreamSynchronize(s)) == cudaSuccess) {
-                const int64_t total = (int64_t)last[0] + last[1];
-                // cells past 2^24 list entries are marked dense (BVH); beyond 2^28 lists are off
-                if (total > 0 && total <= (int64_t(1) << 28)) {
-                    if ((e = c->cell_refs.ensure((size_t)total)) == cudaSuccess &&
-                        (e = cudaMemsetAsync(count.p, 0, (size_t)cells * 4, s)) == cudaSuccess &&
-                        (e = lp::launch_cell_lists(P, nt, c->g_h, list_eps, count.p, start.p, c->cell_refs.p, s)) ==
-                            cudaSuccess) {
-                        lists = true;
-                        c->n_cell_refs = total;
-                    }
-                }
-            }
+    auto list_eps = [c]() { return c->grid_margin * c->g_h + c->g_eps; };
+    // counts, their scan and the number of entries
+    auto count_lists = [&](int64_t &total) {
+        cudaError_t r = cudaMemsetAsync(count, 0, (size_t)cells * 4, s);
+        if (r == cudaSuccess) r = lp::launch_cell_lists(P, nt, c->g_h, list_eps(), count, nullptr, nullptr, s);
+        if (r != cudaSuccess || !c->cell_lists) return r;
+        uint32_t last[2] = {0, 0};
+        if ((r = cub::DeviceScan::ExclusiveSum(scan_tmp, tmp_bytes, count, start, cells, s)) == cudaSuccess &&
+            (r = cudaMemcpyAsync(&last[0], start + cells - 1, 4, cudaMemcpyDeviceToHost, s)) == cudaSuccess &&
+            (r = cudaMemcpyAsync(&last[1], count + cells - 1, 4, cudaMemcpyDeviceToHost, s)) == cudaSuccess)
+            r = cudaStreamSynchronize(s);
+        total = (int64_t)last[0] + last[1];
+        return r;
+    };
+    int64_t total = 0;
+    cudaError_t e = count_lists(total);
+    // Triangles of many cells make short lists, which a wider margin lengthens by little while
+    // the queries get fewer: slab (32 triangles), 1e6 photons, 98 -> 91 ms with three quarters
+    // of a cell.  On the abdomen with 25,600 triangles (about 100 cells each) 71.6 -> 71.2, with
+    // 202,500 (about 30) 73.2 -> 74.5.
+    if (e == cudaSuccess && !c->margin_set && total >= 64 * (int64_t)nt && total <= (int64_t(1) << 22)) {
+        c->grid_margin = 0.75f;
+        e = count_lists(total);
+    }
+    // cells past 2^24 list entries are marked dense (BVH); beyond 2^28 lists are off
+    if (e == cudaSuccess && total > 0 && total <= (int64_t(1) << 28)) {
+        if ((e = c->cell_refs.ensure((size_t)total)) == cudaSuccess &&
+            (e = cudaMemsetAsync(count, 0, (size_t)cells * 4, s)) == cudaSuccess &&
+            (e = lp::launch_cell_lists(P, nt, c->g_h, list_eps(), count, start, c->cell_refs.p, s)) == cudaSuccess) {
+            lists = true;
+            c->n_cell_refs = total;
         }
     }
     if (e == cudaSuccess)
-        e = lp::launch_cell_words(cells, safe.p, lists ? count.p : nullptr, lists ? start.p : nullptr, lists,
-                                  c->cell_word.p, s);
+        e = lp::launch_cell_words(P, c->grid_margin, count, start, lists, gap, d2, c->cell_word.p, s);
     cudaEventRecord(e1, s);
     cudaEventSynchronize(e1);
     cudaEventElapsedTime(&c->grid_ms, e0, e1);
@@ -718,6 +713,7 @@ int build_safety_grid(lp_ctx *c)
     cudaEventDestroy(e1);
     if (e != cudaSuccess) return cuda_fail(c, e, "cell grid");
     if (!lists) c->cell_refs.release();
+    c->grid_dirty = false;   // a build that failed is tried again by the next run
     return LP_OK;
 }
 
@@ -959,8 +955,9 @@ int lp_set_cell_margin(lp_ctx *c, float cells)
 {
     if (!c) return LP_ERR_INVALID;
     if (!(cells >= 0.0f && cells <= 4.0f)) return fail(c, LP_ERR_INVALID, "lp_set_cell_margin: %g cells", (double)cells);
-    if (cells != c->cell_margin) {
+    if (!c->margin_set || cells != c->cell_margin) {
         c->cell_margin = cells;
+        c->margin_set = true;
         c->grid_dirty = true;
     }
     return LP_OK;

@@ -498,10 +498,11 @@ __device__ __forceinline__ float grid_entry(const KParams &P, V3 p, V3 v)
 //     bound; the march goes on from 15/16 of the larger;
 //   * outside the grid: on to the grid's box, or the end when the ray does not meet it.
 // It ends when s has passed the bound or the nearest hit so far.  Most queries are
-// decided by the list they start in (bound <= g_margin + d - g_eps); for those `safe`
-// (coming in with a lower bound already known, the photon's carried one) is raised to a
-// lower bound of the distance from p to every triangle: g_margin + d - g_eps for the
-// unlisted ones, the distance to their plane for the listed ones, |(G x E) . F| / |E x F|
+// decided by the list they start in (bound <= g_margin + d - g_eps).  For those, and for
+// starts in an empty cell, `safe` (coming in with a lower bound already known, the photon's
+// carried one) is raised to a lower bound of the distance from p to every triangle: g_margin
+// + d - g_eps for the unlisted ones (or the empty cell's bound, if larger), the distance to
+// their plane for the listed ones, |(G x E) . F| / |E x F|
 // less a bound of the rounding of that product (tri_c.z = 1 / |E x F|, tri_c.w = the
 // rounding factor per unit |G|, see lp_bvh.hpp), 0 on a triangle (ref_tri >= 0).
 // Dense cells, marches past kMarchMax cells or stuck (lists without a margin), and a mesh
@@ -554,6 +555,11 @@ __device__ __forceinline__ int warp_query(const KParams &P, const MeshView &M, c
                 }
                 if (!own && !(reach > 0.125f * P.g_h)) bvh = true;
                 if (bvh) cnt = 0;
+            } else if (!(word & kCellOutside)) {
+                // no triangle within g_margin + d - g_eps, nor within the word's bound
+                const float clear = fmaxf(reach, safe_distance(P, word));
+                safe = fmaxf(safe, clear);
+                s = 0.9375f * clear;
             }
         }
         const bool march = mine && !own;

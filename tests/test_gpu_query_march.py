@@ -4,7 +4,7 @@ edges of the march."""
 import numpy as np
 import pytest
 
-from lightpropagation_b200 import Simulation, meshes
+from lightpropagation_b200 import Simulation, meshes, workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -42,3 +42,24 @@ def test_march_equals_bvh(margin, cells, n):
     assert np.array_equal(got[0][1].view(np.uint32), got[1][1].view(np.uint32))
     if n > 1000:
         assert (got[0][0] >= 0).mean() > 0.1
+
+
+@pytest.mark.parametrize("mesh", ["slab", "abdomen"])
+@pytest.mark.parametrize("margin,cells", [(0.5, 1 << 24), (0.0, 1 << 20), (0.3, 1 << 16), (2.5, 1 << 20), (0.5, 1 << 6)])
+def test_distance_bounds_change_no_tally(mesh, margin, cells):
+    """The empty cells' distance bounds follow from the lists and their margin: with any
+    margin and cell size, with and without the lists, the tallies are those of a run that
+    queries every step."""
+    w = workloads.plain_slab() if mesh == "slab" else workloads.curved_abdomen(freq=10)
+    got = []
+    for n_cells, lists in ((0, False), (cells, False), (cells, True)):
+        with w.apply(Simulation(0), seed=77) as s:
+            s.set_safety_grid(n_cells)
+            s.set_cell_margin(margin)
+            s.set_cell_lists(lists)
+            s.zero()
+            s.run(3000)
+            got.append(s.tallies())
+    for t in got[1:]:
+        for k in ("sft", "rtd", "rz", "vox", "region"):
+            assert np.array_equal(got[0][k], t[k]), k
