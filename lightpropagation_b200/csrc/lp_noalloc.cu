@@ -25,8 +25,8 @@
 namespace lp {
 int smem_bytes(int nodes_smem, int tris_smem);
 int block_size();
-cudaError_t launch_transport_exact(const KParams &P, int grid, int smem, cudaStream_t s);
-cudaError_t transport_occupancy_exact(int smem, int *blocks_per_sm);
+cudaError_t launch_transport_no_grid(const KParams &P, int grid, int smem, cudaStream_t s);
+cudaError_t transport_occupancy_no_grid(int smem, int *blocks_per_sm);
 void set_thread_error(const char *msg);
 float rspecular_of(const float *nmuasg, int n_media);
 std::mutex &launch_mutex();
@@ -43,6 +43,7 @@ constexpr size_t OFF_CNT = 8;                       // 16 counters -> 136 bytes 
 // set as the work counter when the mesh fails the device-side check: every photon index
 // handed out is then past the range, so the transport kernel traces nothing
 constexpr unsigned long long kRejectAll = 1ull << 62;
+constexpr size_t OFF_EPS = 192;                     // KParams::mesh_eps, two floats
 constexpr size_t HEADER = 256;                      // cleared at every call
 constexpr size_t OFF_MEDIA = HEADER;
 constexpr size_t OFF_NODE_A = OFF_MEDIA + LP_NOALLOC_MAX_MEDIA * sizeof(Medium);
@@ -110,7 +111,18 @@ __global__ void __launch_bounds__(256) noalloc_setup_kernel(const float *tri, co
         const float Fx = __fsub_rn(t[3], t[6]), Fy = __fsub_rn(t[4], t[7]), Fz = __fsub_rn(t[5], t[8]);
         trec[3 * j] = make_float4(t[6], t[7], t[8], Ex);
         trec[3 * j + 1] = make_float4(Ey, Ez, Fx, Fy);
-        trec[3 * j + 2] = make_float4(Fz, __int_as_float(j), 0.0f, 0.0f);
+        // plane-distance factors as in build_bvh
+        const double nx = (double)Ey * Fz - (double)Ez * Fy, ny = (double)Ez * Fx - (double)Ex * Fz,
+                     nz = (double)Ex * Fy - (double)Ey * Fx;
+        const double nl = sqrt(nx * nx + ny * ny + nz * nz);
+        const double el = sqrt((double)Ex * Ex + (double)Ey * Ey + (double)Ez * Ez);
+        const double fl = sqrt((double)Fx * Fx + (double)Fy * Fy + (double)Fz * Fz);
+        float inv_n = 0.0f, kappa = 0.0f;
+        if (nl > 1e-30 * (el * fl + 1e-300) && isfinite(nl)) {
+            inv_n = (float)((1.0 / nl) * (1.0 - 1e-6));
+            kappa = (float)fmin(1e-5 * el * fl / nl, 1e30);
+        }
+        trec[3 * j + 2] = make_float4(Fz, __int_as_float(j), inv_n, kappa);
         float x = nrm[3 * (int64_t)j], y = nrm[3 * (int64_t)j + 1], z = nrm[3 * (int64_t)j + 2];
         const float l = __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)), __fmul_rn(z, z)));
         if (l != 0.0f) {
@@ -143,6 +155,13 @@ __global__ void __launch_bounds__(256) noalloc_setup_kernel(const float *tri, co
     }
     const float ext = fmaxf(fmaxf(s_b[3][0] - s_b[0][0], s_b[4][0] - s_b[1][0]), s_b[5][0] - s_b[2][0]);
     const float margin = 1e-5f * fmaxf(ext, s_abs[0]) + 1e-30f;
+    if (tid == 0) {
+        // allowances of the distance bounds: far above the few-ulp overreach of the
+        // ray/triangle test and the rounding of one position update at this scale
+        float *eps = reinterpret_cast<float *>(s + OFF_EPS);
+        eps[0] = 1e-4f * fmaxf(ext, s_abs[0]);
+        eps[1] = 5e-7f * fmaxf(ext, s_abs[0]);
+    }
     // leaf boxes
     const int L = (n_tri + kLeafTris - 1) / kLeafTris;
     for (int leaf = tid; leaf < L; leaf += bd) {
@@ -341,7 +360,8 @@ extern "C" int lp_run_noalloc(const lp_noalloc_args *a, void *stream)
     P.region = reinterpret_cast<unsigned long long *>(a->region);
     P.counters = reinterpret_cast<unsigned long long *>(sb + OFF_CNT);
     P.work = reinterpret_cast<unsigned long long *>(sb + OFF_WORK);
-    // voxel grid, radial bins, rings, exit records and the safety grid stay off
+    P.mesh_eps = reinterpret_cast<const float *>(sb + OFF_EPS);
+    // voxel grid, radial bins, rings, exit records and the cell grid stay off
     const int smem = smem_bytes(P.nodes_smem, P.tris_smem);
     int per_sm = 0, sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -349,11 +369,11 @@ extern "C" int lp_run_noalloc(const lp_noalloc_args *a, void *stream)
         // the kernel's shared-memory attribute is process-wide: lp_run on another thread
         // sets it too, so the setting and the launch are made under the same lock
         std::lock_guard<std::mutex> lk(lp::launch_mutex());
-        if ((e = transport_occupancy_exact(smem, &per_sm)) != cudaSuccess || per_sm < 1)
+        if ((e = transport_occupancy_no_grid(smem, &per_sm)) != cudaSuccess || per_sm < 1)
             return reject(LP_ERR_CUDA, "lp_run_noalloc: occupancy query failed");
         int grid;
         plan_launch(P.n, block_size(), sms, per_sm, grid, P.lane_mask);
-        if ((e = launch_transport_exact(P, grid, smem, s)) != cudaSuccess)
+        if ((e = launch_transport_no_grid(P, grid, smem, s)) != cudaSuccess)
             return reject(LP_ERR_CUDA, "lp_run_noalloc: transport launch failed");
     }
     if (a->counters) {

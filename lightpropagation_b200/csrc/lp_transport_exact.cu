@@ -15,6 +15,23 @@ cudaError_t transport_occupancy_exact(int smem, int *blocks_per_sm)
     return transport_occupancy_t<true, false>(smem, blocks_per_sm);
 }
 
+// The transport of lp_run_noalloc: reference arithmetic, no cell grid, distance bounds from
+// the mesh itself (P.mesh_eps set).
+cudaError_t launch_transport_no_grid(const KParams &P, int grid, int smem, cudaStream_t s)
+{
+    transport_kernel<true, false, false, true><<<grid, kBlock, smem, s>>>(P);
+    return cudaGetLastError();
+}
+
+cudaError_t transport_occupancy_no_grid(int smem, int *blocks_per_sm)
+{
+    cudaError_t e = cudaFuncSetAttribute(transport_kernel<true, false, false, true>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, transport_kernel<true, false, false, true>, kBlock,
+                                                         smem);
+}
+
 cudaError_t transport_occupancy_exact_grad(int smem, int *blocks_per_sm)
 {
     return transport_occupancy_t<true, true>(smem, blocks_per_sm);

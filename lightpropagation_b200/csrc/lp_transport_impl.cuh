@@ -629,7 +629,7 @@ struct Pending {
 // The nearest triangle within the step's reach (-1: none) and its distance thit; updates
 // the distance bound the query establishes.  Every lane of the warp calls it, the ones
 // whose step needs a query with `want`.
-template <int STACK>
+template <int STACK, bool NoGrid>
 __device__ __forceinline__ int query_step(const KParams &P, const MeshView &M, const MeshView &SM, WarpQueue &Q,
                                           const Medium *s_media, bool want, const Photon &ph, Counters &cnt,
                                           Pending &pd, float &thit)
@@ -638,6 +638,13 @@ __device__ __forceinline__ int query_step(const KParams &P, const MeshView &M, c
     if (!__any_sync(0xffffffffu, want)) return -1;
     const bool ambient = want && (s_media[ph.curr].kind & kAmbient);
     bool used_bvh;
+    if (NoGrid) {
+        cnt.query += want ? 1u : 0u;
+        cnt.bvh += want ? 1u : 0u;
+        return mesh_query<STACK>(P, SM, want, v3(ph.px, ph.py, ph.pz), v3(ph.vx, ph.vy, ph.vz),
+                                 (ph.flags & F_ON_FACE) ? ph.last_tri : -1, ambient ? kNoHit : pd.reach, thit,
+                                 pd.safe_here);
+    }
     // an empty cell: pd.safe_here holds its bound, which the step exceeds; a listed cell
     // raises it from the planes of its triangles when its list decides the step
     const int tri = warp_query<STACK>(P, M, SM, Q, want, v3(ph.px, ph.py, ph.pz), v3(ph.vx, ph.vy, ph.vz),
@@ -651,7 +658,7 @@ __device__ __forceinline__ int query_step(const KParams &P, const MeshView &M, c
 // A scatter event: moves the photon by `step`, absorbs, scatters and adds the deposit to the
 // tallies.  Agg: deposits summed per cell across the warp before the atomic adds.  rz_copy:
 // first cell of the block's copy of the r-z image (rz_copy_of).
-template <bool Exact, bool Grad, bool Agg>
+template <bool Exact, bool Grad, bool Agg, bool NoGrid>
 __device__ __forceinline__ void scatter_event(const KParams &P, const Medium &m, unsigned long long *s_cnt, Photon &ph,
                                               Counters &cnt, float step, float safe_here, const Draws &d,
                                               uint32_t rz_copy)
@@ -661,9 +668,9 @@ __device__ __forceinline__ void scatter_event(const KParams &P, const Medium &m,
     ph.py = ph.py + step * ph.vy;
     ph.pz = ph.pz + step * ph.vz;
     // the next step's cell word: its load is in flight during the rest of this step
-    ph.word = cell_at(P, ph.px, ph.py, ph.pz);
+    if (!NoGrid) ph.word = cell_at(P, ph.px, ph.py, ph.pz);
     ph.flags &= ~F_ON_FACE;
-    ph.safe = fmaxf(safe_here - step - P.step_eps, 0.0f);
+    ph.safe = fmaxf(safe_here - step - (NoGrid ? __ldg(P.mesh_eps + 1) : P.step_eps), 0.0f);
     if (Grad) {
         ph.seg_len += step;
         ph.seg_k++;
@@ -757,7 +764,7 @@ __device__ __forceinline__ uint32_t rz_copy_of(const KParams &P)
 // query wait until several of a warp do, and running their queries together, measured
 // slower on every batch size: the waiting lanes cost more steps than the shared queries
 // save.)
-template <bool Exact, bool Grad, int STACK = kStackDepth, bool Agg = false>
+template <bool Exact, bool Grad, int STACK = kStackDepth, bool Agg = false, bool NoGrid = false>
 __device__ __forceinline__ bool step_photon(const KParams &P, const MeshView &M, const MeshView &SM, WarpQueue &Q,
                                             const Medium *s_media, unsigned long long *s_region,
                                             unsigned long long *s_cnt, unsigned live, bool alive, Photon &ph,
@@ -793,15 +800,15 @@ __device__ __forceinline__ bool step_photon(const KParams &P, const MeshView &M,
     pd.safe_here = fmaxf(ph.safe, safe_distance(P, ph.word));
     const bool want = alive && (ambient || !(pd.reach < pd.safe_here));
     float thit;
-    const int tri = query_step<STACK>(P, M, SM, Q, s_media, want, ph, cnt, pd, thit);
+    const int tri = query_step<STACK, NoGrid>(P, M, SM, Q, s_media, want, ph, cnt, pd, thit);
     const float step = ambient ? thit : pd.step;
     // a query returns no hit beyond the step's reach
     if (alive && (tri >= 0 || kNoHit <= step)) {
         cnt.boundary++;
         ph = boundary_event<Exact, Grad>(P, s_media, s_region, s_cnt, ph, Grad ? ga : nullptr, tri, thit, step, d.u1);
-        ph.word = cell_at(P, ph.px, ph.py, ph.pz);
+        if (!NoGrid) ph.word = cell_at(P, ph.px, ph.py, ph.pz);
     } else if (alive) {
-        scatter_event<Exact, Grad, Agg>(P, m, s_cnt, ph, cnt, step, pd.safe_here, d, rz_copy);
+        scatter_event<Exact, Grad, Agg, NoGrid>(P, m, s_cnt, ph, cnt, step, pd.safe_here, d, rz_copy);
     }
     ph.steps += alive ? 1u : 0u;
     if (alive && (ph.w < P.w_th || ph.steps >= P.step_cap)) {
@@ -862,7 +869,8 @@ __device__ __forceinline__ MeshView stage_mesh(const KParams &P, unsigned char *
     return M;
 }
 
-template <bool Exact, bool Grad, bool Agg = false>
+// NoGrid: the mesh has no cell grid (mesh_query).
+template <bool Exact, bool Grad, bool Agg = false, bool NoGrid = false>
 __global__ void __launch_bounds__(kBlock, LP_TRANSPORT_MIN_BLOCKS) transport_kernel(const __grid_constant__ KParams P)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -920,7 +928,7 @@ __global__ void __launch_bounds__(kBlock, LP_TRANSPORT_MIN_BLOCKS) transport_ker
             live = __ballot_sync(0xffffffffu, alive);
         }
         if (!live) break;
-        const bool more = step_photon<Exact, Grad, kStackDepth, Agg>(P, M, shared_view, queues[threadIdx.x >> 5],
+        const bool more = step_photon<Exact, Grad, kStackDepth, Agg, NoGrid>(P, M, shared_view, queues[threadIdx.x >> 5],
                                                                      s_media, s_region, s_cnt, live, alive, ph, cnt, &ga,
                                                                      draws[threadIdx.x >> 5], next, rz_copy);
         if (alive) {
