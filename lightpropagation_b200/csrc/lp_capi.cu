@@ -1112,7 +1112,7 @@ int lp_run_async(lp_ctx *c, int64_t first, int64_t n)
             P.exit_cap = 0;
         }
         int grid;
-        lp::plan_launch(m, lp::block_size(), c->num_sms, per_sm, grid, P.lane_mask);
+        lp::plan_launch(m, lp::block_size(), c->num_sms, per_sm, grid, P.lane_mask, P.few_blocks);
         c->st_grid = grid;
         LP_CUDA(c, cudaMemsetAsync(c->work.p, 0, 8, c->stream));
         c->h2d_bytes += (int64_t)sizeof(KParams);
@@ -1630,7 +1630,8 @@ int prepare_plain(lp_batch *b)
         LP_BCUDA(b, b->grad_on ? lp::transport_occupancy_fast_grad(L.smem, &per_sm)
                                : lp::transport_occupancy_fast(L.smem, &per_sm));
         if (per_sm < 1) return bfail(b, LP_ERR_CUDA, "batch: transport kernel does not fit on an SM");
-        lp::plan_launch(L.P.n, lp::block_size(), b->num_sms, per_sm, L.grid, L.P.lane_mask);
+        lp::plan_launch(L.P.n, lp::block_size(), b->num_sms, per_sm, L.grid, L.P.lane_mask, L.P.few_blocks);
+        L.P.few_blocks = 0;   // that instance sets its shared-memory attribute at the launch, here a capture
     }
     return LP_OK;
 }
@@ -1655,7 +1656,8 @@ int prepare_grid(lp_batch *b, int config)
     if (per_sm < 1) return bfail(b, LP_ERR_CUDA, "batch configuration %d does not fit on an SM", config);
     int block, minb, stack;
     lp::batch_config_info(config, &block, &minb, &stack);
-    lp::plan_launch(b->n_batch, block, b->num_sms, per_sm, b->grid, b->lane_mask);
+    uint32_t few;
+    lp::plan_launch(b->n_batch, block, b->num_sms, per_sm, b->grid, b->lane_mask, few);
     return LP_OK;
 }
 

@@ -110,26 +110,31 @@ struct KParams {
     // scratch: photon work counter
     unsigned long long *work;
     uint32_t lane_mask;   // lanes of a warp that carry photons (plan_launch)
+    // host side: the kernel instance for 16 warps per SM runs (plan_launch)
+    uint32_t few_blocks;
 };
 
 // Blocks of a transport launch and the lanes of a warp that carry photons.  A short run
 // lasts as long as its longest photon (many times the mean), and a photon's step takes
 // the longer the more others share its warp (each of them may have a query or a boundary
-// event) and its SM.  So up to the lanes of two blocks per SM the photons are spread evenly
-// over the warps of two, and up to twice as many take turns on them.  Against full warps
-// on three blocks (slab / curved abdomen at 660 nm): 1,000 photons 17.9 -> 12.2 / 15.3 ->
-// 10.1 ms, 10,000 20.8 -> 16.6 / 20.3 -> 18.1, 30,000 25.0 -> 20.5 / 23.5 -> 20.1, 100,000
-// 31.2 -> 29.6 / 28.6 -> 27.3; at 300,000 three blocks win on the slab (43.7 against 47.7)
-// and lose on the abdomen (42.8 against 40.2).
-inline void plan_launch(int64_t n, int block, int num_sms, int per_sm, int &grid, uint32_t &lane_mask)
+// event) and its SM.  So up to the lanes of 16 warps per SM the photons are spread evenly
+// over those warps, and up to twice as many take turns on them.  Against full warps, 24 per
+// SM (slab / curved abdomen at 660 nm): 1,000 photons 17.9 -> 12.2 / 15.3 -> 10.1 ms, 10,000
+// 20.8 -> 16.6 / 20.3 -> 18.1, 30,000 25.0 -> 20.5 / 23.5 -> 20.1, 100,000 31.2 -> 29.6 / 28.6
+// -> 27.3; at 300,000 more warps win on the slab (43.7 against 47.7) and lose on the abdomen
+// (42.8 against 40.2).
+// few: the launch has no more than those warps, so the kernel instance compiled for them runs
+// (106 registers instead of 95): 30,000 slab photons 16.7 -> 15.7 ms, 50,000 on 25,600
+// triangles 17.3 -> 16.4, 1e5 on the abdomen 23.7 -> 23.0.
+inline void plan_launch(int64_t n, int block, int num_sms, int per_sm, int &grid, uint32_t &lane_mask, uint32_t &few)
 {
-    const int two = 512 / block > 1 ? 512 / block : 1;   // 16 warps, two blocks of the transport kernel
-    const int few = per_sm < two ? per_sm : two;
-    const int64_t warps = (int64_t)num_sms * few * (block / 32);
+    const int blocks = per_sm * block < 512 ? per_sm : 512 / block > 1 ? 512 / block : 1;
+    const int64_t warps = (int64_t)num_sms * blocks * (block / 32);
     int64_t lanes = (n + warps - 1) / warps;
     lanes = lanes < 1 ? 1 : lanes > 32 ? 32 : lanes;
     lane_mask = lanes == 32 ? 0xffffffffu : (1u << lanes) - 1u;
-    grid = num_sms * (n <= 64 * warps ? few : per_sm);
+    few = n <= 64 * warps ? 1u : 0u;
+    grid = num_sms * (few ? blocks : per_sm);
 }
 
 // A batch: many instances (one KParams each) traced by one persistent launch.

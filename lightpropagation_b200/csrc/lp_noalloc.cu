@@ -317,7 +317,7 @@ extern "C" int lp_run_noalloc(const lp_noalloc_args *a, void *stream)
     P.n_nodes = NI;
     P.n_tri = (int32_t)a->n_tri;
     const int base_smem = smem_bytes(0, 0);
-    int room = 64 * 1024 - base_smem;
+    int room = 36 * 1024 - base_smem;   // five blocks per SM
     P.nodes_smem = std::min(NI, room / 64);
     room -= P.nodes_smem * 64;
     P.tris_smem = std::min((int)a->n_tri, room / 48);
@@ -372,7 +372,7 @@ extern "C" int lp_run_noalloc(const lp_noalloc_args *a, void *stream)
         if ((e = transport_occupancy_no_grid(smem, &per_sm)) != cudaSuccess || per_sm < 1)
             return reject(LP_ERR_CUDA, "lp_run_noalloc: occupancy query failed");
         int grid;
-        plan_launch(P.n, block_size(), sms, per_sm, grid, P.lane_mask);
+        plan_launch(P.n, block_size(), sms, per_sm, grid, P.lane_mask, P.few_blocks);
         if ((e = launch_transport_no_grid(P, grid, smem, s)) != cudaSuccess)
             return reject(LP_ERR_CUDA, "lp_run_noalloc: transport launch failed");
     }

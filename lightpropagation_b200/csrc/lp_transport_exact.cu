@@ -19,8 +19,8 @@ cudaError_t transport_occupancy_exact(int smem, int *blocks_per_sm)
 // the mesh itself (P.mesh_eps set).
 cudaError_t launch_transport_no_grid(const KParams &P, int grid, int smem, cudaStream_t s)
 {
-    transport_kernel<true, false, false, true><<<grid, kBlock, smem, s>>>(P);
-    return cudaGetLastError();
+    if (P.few_blocks) return launch_instance<true, false, false, true, kFewBlocks>(P, grid, smem, s);
+    return launch_instance<true, false, false, true, LP_TRANSPORT_MIN_BLOCKS>(P, grid, smem, s);
 }
 
 cudaError_t transport_occupancy_no_grid(int smem, int *blocks_per_sm)

@@ -21,7 +21,7 @@
 // What bounds it: the instructions of one step, 400 to 500 of them in one chain that
 // branches on its own results.  A warp with one photon left issues one every 4 to 5
 // cycles (fixed latencies and the special-function unit), so short runs and the ends of
-// long ones wait for their longest photon; full warps (24 per SM at 80 registers) issue
+// long ones wait for their longest photon; full warps (20 per SM at 96 registers) issue
 // two cycles of three.  Hence the form of the step: selects instead of branches where both
 // sides are a few operations, round keys and derived constants in the kernel's parameters,
 // 32-bit indices, two 16-byte loads for a medium's factors, no counter that another one
@@ -50,12 +50,16 @@
 
 namespace lp {
 
-constexpr int kBlock = 256;
+constexpr int kBlock = 128;
 // Resident blocks per SM the single-instance kernel is compiled for (register budget
-// 65536 / (kBlock x this)); the batched kernel's configurations are autotuned instead.
+// 65536 / (kBlock x this)); the batched kernel's configurations are autotuned instead.  Five
+// of 128 threads leave 96 registers, 20 warps per SM.  Slab 1e6 photons / curved abdomen 660
+// nm 3e6 and 5e5, ms: 83.5 / 170 / 45.2; three of 256 (80 registers, 24 warps, spills) 86.2 /
+// 173 / 49.0; eleven of 64 (88) 87.9 / 180 / 49.8.  Short runs use four (128, no spills).
 #ifndef LP_TRANSPORT_MIN_BLOCKS
-#define LP_TRANSPORT_MIN_BLOCKS 3
+#define LP_TRANSPORT_MIN_BLOCKS 5
 #endif
+constexpr int kFewBlocks = 4;   // 16 warps, as plan_launch
 
 struct Photon {
     float px, py, pz, vx, vy, vz;
@@ -870,8 +874,9 @@ __device__ __forceinline__ MeshView stage_mesh(const KParams &P, unsigned char *
 }
 
 // NoGrid: the mesh has no cell grid (mesh_query).
-template <bool Exact, bool Grad, bool Agg = false, bool NoGrid = false>
-__global__ void __launch_bounds__(kBlock, LP_TRANSPORT_MIN_BLOCKS) transport_kernel(const __grid_constant__ KParams P)
+// MinBlocks: resident blocks per SM it is compiled for.
+template <bool Exact, bool Grad, bool Agg = false, bool NoGrid = false, int MinBlocks = LP_TRANSPORT_MIN_BLOCKS>
+__global__ void __launch_bounds__(kBlock, MinBlocks) transport_kernel(const __grid_constant__ KParams P)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ WarpQueue queues[kBlock / 32];
@@ -971,22 +976,31 @@ __global__ void __launch_bounds__(kBlock, LP_TRANSPORT_MIN_BLOCKS) transport_ker
         if (s_region[i]) atomicAdd(P.region + i, s_region[i]);
 }
 
+template <bool Exact, bool Grad, bool Agg, bool NoGrid, int MinBlocks>
+cudaError_t launch_instance(const KParams &P, int grid, int smem, cudaStream_t s)
+{
+    cudaError_t e = cudaFuncSetAttribute(transport_kernel<Exact, Grad, Agg, NoGrid, MinBlocks>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    transport_kernel<Exact, Grad, Agg, NoGrid, MinBlocks><<<grid, kBlock, smem, s>>>(P);
+    return cudaGetLastError();
+}
+
 // P.grad selects the differentiating instantiation.
 // The warp-aggregated form exists for the production arithmetic without differentiation
-// only (P.agg_tallies is ignored otherwise).
+// only (P.agg_tallies is ignored otherwise).  The instance for few blocks sets its own
+// shared-memory attribute; the occupancy query has set the other's (prepare_plain outside of
+// stream capture).
 template <bool Exact>
 cudaError_t launch_transport_t(const KParams &P, int grid, int smem, cudaStream_t s)
 {
-    if (!Exact && !P.grad && P.agg_tallies) {
-        cudaError_t e = cudaFuncSetAttribute(transport_kernel<false, false, true>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return e;
-        transport_kernel<false, false, true><<<grid, kBlock, smem, s>>>(P);
-    } else if (P.grad) {
-        transport_kernel<Exact, true><<<grid, kBlock, smem, s>>>(P);
-    } else {
-        transport_kernel<Exact, false><<<grid, kBlock, smem, s>>>(P);
-    }
+    if (!Exact && !P.grad && P.agg_tallies)
+        return launch_instance<false, false, true, false, LP_TRANSPORT_MIN_BLOCKS>(P, grid, smem, s);
+    if (P.few_blocks)
+        return P.grad ? launch_instance<Exact, true, false, false, kFewBlocks>(P, grid, smem, s)
+                      : launch_instance<Exact, false, false, false, kFewBlocks>(P, grid, smem, s);
+    if (P.grad) transport_kernel<Exact, true><<<grid, kBlock, smem, s>>>(P);
+    else transport_kernel<Exact, false><<<grid, kBlock, smem, s>>>(P);
     return cudaGetLastError();
 }
 
