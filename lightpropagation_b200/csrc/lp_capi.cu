@@ -427,7 +427,9 @@ void media_table(const float *nmuasg, int n_media, std::vector<Medium> &m)
         m[i].g = q[3];
         m[i].mut = q[1] + q[2];
         m[i].alb = q[1] / (q[1] + q[2]);
-        m[i].kind = (q[1] > 0.0f && q[2] > 0.0f ? lp::kAbsorbs : 0u) | (q[1] == 0.0f && q[2] == 0.0f ? lp::kAmbient : 0u);
+        m[i].kind = (q[1] > 0.0f && q[2] > 0.0f ? lp::kAbsorbs : 0u) |
+                    (q[1] == 0.0f && q[2] == 0.0f ? lp::kAmbient : 0u) |
+                    lp::plain_div_of(q[1], q[1] + q[2], q[3]);
         m[i].inv_mut = (q[1] + q[2]) > 0.0f ? 1.0f / (q[1] + q[2]) : 0.0f;
         m[i].inv_mua = q[1] > 0.0f ? 1.0f / q[1] : 0.0f;
         const float g = q[3];
@@ -547,6 +549,11 @@ void fill_params(lp_ctx *c, KParams &P, int64_t first, int64_t n, int nodes_smem
     P.half_vnx = 0.5f * (float)c->vox_n[0];
     P.half_vny = 0.5f * (float)c->vox_n[1];
     P.vox_on = c->vox_n[0] > 0 ? 1u : 0u;
+    P.plain_div = lp::div_range(c->det_grid[2]) && lp::div_range(c->det_grid[3]) &&
+                          (!P.vox_on || (lp::div_range(c->vox_d[0]) && lp::div_range(c->vox_d[1]) &&
+                                         lp::div_range(c->vox_d[2])))
+                      ? 0u
+                      : 1u;
     P.sft = c->sft.p; P.rtd = c->rtd.p; P.rz = c->rz.p; P.vox = c->vox.p; P.rbins = c->rbins.p;
     P.region = c->region.p; P.det = c->det.p; P.counters = c->counters.p;
     const int copies = rz_copies(rz_values(c));

@@ -29,6 +29,16 @@ struct alignas(16) Medium {
 };
 constexpr uint32_t kAbsorbs = 1u;  // mua > 0 && mus > 0  (Absorb, .cl:841-847)
 constexpr uint32_t kAmbient = 2u;  // mua == 0 && mus == 0 (step = distance to boundary, .cl:1405-1410)
+constexpr uint32_t kPlainDiv = 4u; // a divisor outside of div_range: the plain operator divides
+
+// Divisors for which div_rn needs no care for overflow and underflow.
+__host__ __device__ __forceinline__ bool div_range(float x) { return x >= 1e-12f && x <= 1e12f; }
+// Those of a medium: mua, mut, 2 g and 1 - g + 2 g xi.
+__host__ __device__ __forceinline__ uint32_t plain_div_of(float mua, float mut, float g)
+{
+    const float a = g < 0.0f ? -g : g;
+    return div_range(mua) && div_range(mut) && (g == 0.0f || (a >= 1e-6f && 1.0f - a >= 1e-6f)) ? 0u : kPlainDiv;
+}
 
 struct KParams {
     // mesh (see lp_bvh.hpp)
@@ -62,6 +72,7 @@ struct KParams {
     float inv_dr, inv_dz, inv_vdx, inv_vdy, inv_vdz;   // reciprocals for the fast mode
     float f_dimR, half_vnx, half_vny;                  // dimR, vox_nx / 2, vox_ny / 2
     uint32_t vox_on;                                   // 1 with a voxel grid
+    uint32_t plain_div;                                // a bin width lies outside of div_range
     // tallies (fixed point, 2^32 per unit weight)
     unsigned long long *sft, *rtd, *rz, *vox, *rbins, *region, *det, *counters;
     // where the r-z deposits go: rz_mask + 1 (a power of two) copies of the image, each of

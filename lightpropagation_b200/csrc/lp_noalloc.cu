@@ -90,7 +90,8 @@ __global__ void __launch_bounds__(256) noalloc_setup_kernel(const float *tri, co
         m.n = q.x; m.mua = q.y; m.mus = q.z; m.g = q.w;
         m.mut = __fadd_rn(q.y, q.z);
         m.alb = __fdiv_rn(q.y, m.mut);
-        m.kind = (q.y > 0.0f && q.z > 0.0f ? kAbsorbs : 0u) | (q.y == 0.0f && q.z == 0.0f ? kAmbient : 0u);
+        m.kind = (q.y > 0.0f && q.z > 0.0f ? kAbsorbs : 0u) | (q.y == 0.0f && q.z == 0.0f ? kAmbient : 0u) |
+                 plain_div_of(q.y, m.mut, q.w);
         m.inv_mut = m.mut > 0.0f ? __fdiv_rn(1.0f, m.mut) : 0.0f;
         m.inv_mua = q.y > 0.0f ? __fdiv_rn(1.0f, q.y) : 0.0f;
         m.hg_a = __fsub_rn(1.0f, __fmul_rn(q.w, q.w));
@@ -353,6 +354,7 @@ extern "C" int lp_run_noalloc(const lp_noalloc_args *a, void *stream)
     P.inv_dz = 1.0f / a->det_grid[2];
     P.inv_vdx = P.inv_vdy = P.inv_vdz = 1.0f;
     P.f_dimR = (float)dimR;
+    P.plain_div = div_range(a->det_grid[2]) && div_range(a->det_grid[3]) ? 0u : 1u;
     P.sft = reinterpret_cast<unsigned long long *>(a->sft);
     P.rtd = reinterpret_cast<unsigned long long *>(a->rtd);
     P.rz = reinterpret_cast<unsigned long long *>(a->rz);
