@@ -1462,7 +1462,8 @@ struct lp_batch {
     // launch of their own inside the graph, with their context's shared-memory plan; the
     // batch kernel sees them with no photons.  The batch kernel pays for its per-warp
     // instance switching on every photon, a launch of its own only once (its drain):
-    // at about 7e5 photons the two cost the same on the abdomen.
+    // at about 7e5 photons the two cost the same on the abdomen (measured when the warps of
+    // the batch launch all began on its first instance).
     struct PlainLaunch {
         KParams P;
         int grid = 0, smem = 0;
@@ -1474,8 +1475,9 @@ struct lp_batch {
     // the batch launch, and one set that the plain launches use in turn
     DevBuf<unsigned long long> rz_part, plain_rz_part;
     // The r-z and voxel tallies (the atomic targets of every scatter event) of the
-    // instances with a launch of their own sit in buffers of their own, like a context's:
-    // as slices of the batch's large arrays the same launch measured up to 15 % slower.
+    // instances with a launch of their own sit in buffers of their own, like a context's: as
+    // slices of the batch's large arrays the same launch measured up to 15 % slower (before the
+    // r-z deposits went to copies).
     struct OwnTallies {
         DevBuf<unsigned long long> rz, vox;
     };

@@ -668,7 +668,11 @@ __device__ __forceinline__ int warp_query(const KParams &P, const MeshView &M, c
         __syncwarp();
         todo &= ~__ballot_sync(0xffffffffu, mine);
     }
-    if (bvh) tri = query_nearest<STACK>(SM, p, v, ref_tri, bound, t_out);
+    if (bvh) {
+        float t;   // the address of t_out would keep it in local memory
+        tri = query_nearest<STACK>(SM, p, v, ref_tri, bound, t);
+        t_out = t;
+    }
     used_bvh = bvh;
     return tri;
 }

@@ -45,16 +45,21 @@ __device__ bool tri_cube_overlap(V3 c, float r, V3 a, V3 b, V3 d)
 // One pass over the triangles (BVH order): every cell that a triangle touches (cells
 // widened by eps) gets a count (refs == nullptr) or, in the second pass, the triangle's
 // index at start[cell] + the next free slot (count re-zeroed before that pass).  One warp
-// per triangle, its lanes striding over the cells of the triangle's box: a large
-// triangle (a slab face covers 10^5 cells) is not left to a single thread.  The order of
-// the entries within a cell is not defined, and no query depends on it.
+// per triangle, its lanes striding over the cells of the triangle's box, and all warps of
+// the launch shared out where there are fewer triangles than those: a slab face covers 10^5
+// cells, and with one warp each the 32 triangles' passes took 23 ms of a first run of 27 (now
+// 0.13 of 5).  The order of the entries within a cell is not defined, and no query depends on
+// it.
 __global__ void __launch_bounds__(256) cell_lists_kernel(const __grid_constant__ KParams P, int n_tri, float h,
                                                          float eps, uint32_t *count, const uint32_t *start,
                                                          int32_t *refs)
 {
-    const int lane = threadIdx.x & 31;
     const int n_warps = (gridDim.x * blockDim.x) >> 5;
-    for (int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < n_tri; j += n_warps) {
+    // warps per triangle: a mesh of few triangles has them large
+    const int share = n_tri < n_warps ? n_warps / n_tri : 1;
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t first = (int64_t)(warp % share) * 32 + (threadIdx.x & 31);
+    for (int j = warp / share; j < n_tri; j += n_warps / share) {
         const TriRec T = load_tri(P.tri, j);
         const float4 ta = T.a, tb = T.b, tc = T.c;
         const V3 a = v3(ta.x, ta.y, ta.z);
@@ -70,7 +75,7 @@ __global__ void __launch_bounds__(256) cell_lists_kernel(const __grid_constant__
         }
         const int ex = c1[0] - c0[0] + 1, ey = c1[1] - c0[1] + 1;
         const int64_t n_cells = (int64_t)ex * ey * (c1[2] - c0[2] + 1);
-        for (int64_t q = lane; q < n_cells; q += 32) {
+        for (int64_t q = first; q < n_cells; q += 32 * share) {
             const int x = c0[0] + (int)(q % ex);
             const int y = c0[1] + (int)((q / ex) % ey);
             const int z = c0[2] + (int)(q / ((int64_t)ex * ey));
@@ -191,7 +196,7 @@ __global__ void __launch_bounds__(256) cell_word_kernel(int64_t layer, int nz, f
 cudaError_t launch_cell_lists(const KParams &P, int n_tri, float h, float eps, uint32_t *count, const uint32_t *start,
                               int32_t *refs, cudaStream_t s)
 {
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n_tri * 32 + 255) / 256, 148 * 16));
+    const int grid = 148 * 16;
     cell_lists_kernel<<<grid, 256, 0, s>>>(P, n_tri, h, eps, count, start, refs);
     return cudaGetLastError();
 }

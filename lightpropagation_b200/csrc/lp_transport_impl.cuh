@@ -30,7 +30,7 @@
 // word overlap; and random numbers drawn several events ahead once lanes are idle
 // (next_draws); the lanes without a photon run along, and rare ends (roulette, step cap)
 // share one branch.  One photon alone takes 0.65 us a step on the slab (1.20 before these),
-// 0.73 on the curved abdomen (1.36); slab, 1e6 photons, 114 -> 90 ms; abdomen at 660 nm,
+// 0.73 on the curved abdomen (1.36; 0.60 and 0.67 without spills); slab, 1e6 photons, 114 -> 90 ms; abdomen at 660 nm,
 // 3e6 photons, 201 -> 175 ms; 1e5 photons 40 -> 24 ms.
 //
 // Exact = true  keeps the reference's arithmetic operation by operation (compiled
@@ -117,7 +117,7 @@ __device__ __forceinline__ float rsqrt_normal(float x)
     return y;
 }
 
-// The correctly rounded square root for x >= 1e-30, 0 below: one Newton correction of
+// The correctly rounded square root for x >= 1e-30, 0 from 0 to there: one Newton correction of
 // x / sqrt(x) with fused multiply-adds (Markstein, IBM J. Res. Dev. 34, 1990).  Compared
 // with sqrtf for every float from 1e-30 to 3e38.  Unlike sqrtf it has no branch to a slow
 // path, which would cut the step's straight line of code.
@@ -125,7 +125,8 @@ __device__ __forceinline__ float sqrt_normal(float x)
 {
     const float y = rsqrt_normal(x), s = x * y;
     const float r = __fmaf_rn(__fmaf_rn(-s, s, x), 0.5f * y, s);
-    return x >= 1e-30f ? r : 0.0f;
+    // one unsigned comparison for 0 <= x < 1e-30; negative x and NaN stay NaN, as sqrtf has them
+    return __float_as_uint(x) < 0x0DA24260u ? 0.0f : r;
 }
 
 // 1 / b correctly rounded, for 2^-100 <= |b| <= 2^100: one Newton step from the
