@@ -9,9 +9,10 @@
 // Scratch layout (offsets below): photon work counter and event counters (cleared at
 // every call), the media table, and a small BVH built on the device from the caller's
 // reference-layout mesh arrays (leaves of 4 triangles in input order, a heap-ordered
-// binary tree over them).  The transport itself is the existing reference-arithmetic
-// kernel, launched with pointers into this array; its results equal those of lp_run
-// in reference-arithmetic mode for the same seed and photon range.
+// binary tree over them).  The transport itself is the reference-arithmetic kernel in an
+// instance without a cell grid (mesh_query), launched with pointers into this array; its
+// results equal those of lp_run in reference-arithmetic mode for the same seed and photon
+// range.
 #include <cuda_runtime.h>
 
 #include <algorithm>
