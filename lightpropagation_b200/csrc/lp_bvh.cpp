@@ -261,20 +261,32 @@ int32_t build_par(Prim *pr, std::vector<BNode> &nodes, int64_t first, int64_t co
     const int sub_bins = std::max(1, bin_threads / 2);
     std::vector<BNode> right;
     std::thread th;
+    std::exception_ptr failed;   // of the other thread: rethrown here, where a caller can catch it
     bool threaded = false;
     try {
         th = std::thread([&]() {
-            build_par(pr, right, mid, first + count - mid, leaf_target, par_depth - 1, sub_bins);
+            try {
+                build_par(pr, right, mid, first + count - mid, leaf_target, par_depth - 1, sub_bins);
+            } catch (...) {
+                failed = std::current_exception();
+            }
         });
         threaded = true;
     } catch (const std::exception &) {
         // no thread to be had: the right child is built here after the left
     }
-    nd.child[0] = build_par(pr, nodes, first, mid - first, leaf_target, par_depth - 1, sub_bins);
-    if (threaded)
+    try {
+        nd.child[0] = build_par(pr, nodes, first, mid - first, leaf_target, par_depth - 1, sub_bins);
+    } catch (...) {
+        if (threaded) th.join();
+        throw;
+    }
+    if (threaded) {
         th.join();
-    else
+        if (failed) std::rethrow_exception(failed);
+    } else {
         build_par(pr, right, mid, first + count - mid, leaf_target, par_depth - 1, sub_bins);
+    }
     const int32_t base = (int32_t)nodes.size();
     for (BNode b : right) {
         for (int c = 0; c < 2; ++c)
