@@ -230,10 +230,12 @@ void build_from(Prim *pr, std::vector<BNode> &nodes, int32_t root, int leaf_targ
     }
 }
 
-constexpr int64_t kParallelGrain = 1024;   // smaller subtrees are built where they are
-// Smaller meshes are built on the calling thread.  16 hardware threads, one against all: 500
-// triangles 0.17 ms either way, 2,000 0.82 -> 0.50, 4,000 1.7 -> 0.7, 25,600 14.0 -> 4.1, 202,500
-// 120 -> 30 (grain 4096: 29).
+// Subtrees smaller than the grain are built where they are: an eighth of the mesh, between
+// 1,024 and 4,096.  16 hardware threads, grain 1,024 / 2,048 / 4,096: 4,000 triangles 0.7 / 1.1 /
+// 1.8 ms, 25,600 4.2 / 3.7 / 4.1, 57,600 9.3 / 8.9 / 8.8, 202,500 34 / 34 / 34.
+int64_t parallel_grain(int64_t n) { return std::min<int64_t>(std::max<int64_t>(n / 8, 1024), 4096); }
+// Smaller meshes are built on the calling thread.  One thread against all: 500 triangles 0.17
+// ms either way, 2,000 0.82 -> 0.50, 4,000 1.7 -> 0.7, 25,600 14.0 -> 3.7, 202,500 120 -> 34.
 constexpr int64_t kParallelMin = 2000;
 
 // Builds the subtree over primitives [first, first + count) into `nodes` and returns its
@@ -242,13 +244,13 @@ constexpr int64_t kParallelMin = 2000;
 // left child is built on this thread.  Every split is the one the serial build makes
 // (split_node on the same primitive range), so the tree is the same.
 int32_t build_par(Prim *pr, std::vector<BNode> &nodes, int64_t first, int64_t count, int leaf_target,
-                  int par_depth, int bin_threads)
+                  int par_depth, int bin_threads, int64_t grain)
 {
     const int32_t root = (int32_t)nodes.size();
     nodes.push_back(BNode());
     nodes[root].first = first;
     nodes[root].count = count;
-    if (par_depth <= 0 || count < kParallelGrain) {
+    if (par_depth <= 0 || count < grain) {
         build_from(pr, nodes, root, leaf_target, bin_threads);
         return root;
     }
@@ -266,7 +268,7 @@ int32_t build_par(Prim *pr, std::vector<BNode> &nodes, int64_t first, int64_t co
     try {
         th = std::thread([&]() {
             try {
-                build_par(pr, right, mid, first + count - mid, leaf_target, par_depth - 1, sub_bins);
+                build_par(pr, right, mid, first + count - mid, leaf_target, par_depth - 1, sub_bins, grain);
             } catch (...) {
                 failed = std::current_exception();
             }
@@ -276,7 +278,7 @@ int32_t build_par(Prim *pr, std::vector<BNode> &nodes, int64_t first, int64_t co
         // no thread to be had: the right child is built here after the left
     }
     try {
-        nd.child[0] = build_par(pr, nodes, first, mid - first, leaf_target, par_depth - 1, sub_bins);
+        nd.child[0] = build_par(pr, nodes, first, mid - first, leaf_target, par_depth - 1, sub_bins, grain);
     } catch (...) {
         if (threaded) th.join();
         throw;
@@ -285,7 +287,7 @@ int32_t build_par(Prim *pr, std::vector<BNode> &nodes, int64_t first, int64_t co
         th.join();
         if (failed) std::rethrow_exception(failed);
     } else {
-        build_par(pr, right, mid, first + count - mid, leaf_target, par_depth - 1, sub_bins);
+        build_par(pr, right, mid, first + count - mid, leaf_target, par_depth - 1, sub_bins, grain);
     }
     const int32_t base = (int32_t)nodes.size();
     for (BNode b : right) {
@@ -332,12 +334,12 @@ void build_bvh(const float *tri, int64_t n, Bvh &out, int leaf_target, int threa
     const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
     const int n_threads = threads > 0 ? std::min(threads, 64) : (int)std::min(hw, 16u);
     if (n < kParallelMin || n_threads == 1) {
-        build_par(pr.data(), nodes, 0, n, leaf_target, 0, 1);
+        build_par(pr.data(), nodes, 0, n, leaf_target, 0, 1, n);
     } else {
         // enough levels of threads for about four subtrees per hardware thread
         int par_depth = 0;
         while ((1 << par_depth) < 4 * n_threads) ++par_depth;
-        build_par(pr.data(), nodes, 0, n, leaf_target, par_depth, n_threads);
+        build_par(pr.data(), nodes, 0, n, leaf_target, par_depth, n_threads, parallel_grain(n));
     }
 
     // A root that is a leaf gets a synthetic internal parent whose two children are
