@@ -471,6 +471,17 @@ __device__ __noinline__ int query_nearest(const MeshView &M, V3 p, V3 v, int ref
     return bid;
 }
 
+// The cell word that a query from p along v begins with (warp_query).  The march, its lists and
+// the distance bounds take t for a distance, which holds for rays of at most unit length (a
+// shorter one moves less far than t): a longer one is answered by the tree, as from a dense
+// cell.  The allowance is that of a direction normalised in float (dot3 within 7e-7 of 1); the
+// plane distances of tri_c allow for twice as much.
+constexpr float kUnitDot = 1.000001f;
+__device__ __forceinline__ uint32_t query_word(const KParams &P, V3 p, V3 v)
+{
+    return dot3(v, v) > kUnitDot ? kCellDense << 24 : cell_at(P, p.x, p.y, p.z);
+}
+
 // Per-warp shared memory of warp_query: the rays and results of up to kQueue queries,
 // and the list segments of one pass.
 constexpr int kQueue = 16;
@@ -507,7 +518,8 @@ __device__ __forceinline__ float grid_entry(const KParams &P, V3 p, V3 v)
 // The warp's nearest-triangle queries over the cell lists; every lane calls it, those with
 // `want` have a query: the nearest triangle along (p, v) with t in (0, bound] and
 // t < kNoHit, ref_tri excluded, equal distances resolving to the lower original index.
-// Returns its original index or -1 with t_out = kNoHit.
+// Returns its original index or -1 with t_out = kNoHit.  word: query_word (cell_at for a
+// direction known to be of unit length).
 //
 // A query marches along its ray.  At distance s it stands in a cell (word: the cell at
 // s = 0), d from the cell's faces:
@@ -569,7 +581,7 @@ __device__ __forceinline__ int warp_query(const KParams &P, const MeshView &M, c
                 bvh = cnt == kCellDense;
                 own = bound <= reach && !bvh;
                 s = 0.9375f * reach;
-                if (!LP_IN_RANGE(M.dbg, (int64_t)off + cnt - 1, P.n_cell_refs)) {
+                if (!bvh && !LP_IN_RANGE(M.dbg, (int64_t)off + cnt - 1, P.n_cell_refs)) {
                     cnt = 0;
                     Q.safe[rank] = 0u;
                 }

@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kBlock) query_kernel(const __grid_constant__ K
         float t, safe = 0.0f;
         bool used_bvh;
         const int id = warp_query(P, M, shared_view, queues[threadIdx.x >> 5], want, p, v, ref[q], tmax[q],
-                                  cell_at(P, p.x, p.y, p.z), t, safe, used_bvh);
+                                  query_word(P, p, v), t, safe, used_bvh);
         if (want) {
             id_out[i] = id;
             t_out[i] = t;

@@ -1,0 +1,35 @@
+"""Directions of any length: a ray's t counts in units of its direction, as in the reference
+(MCLightPropagation.cl:1037-1093), whichever way the query is answered."""
+import numpy as np
+import pytest
+
+from lightpropagation_b200 import Simulation, meshes, workloads
+
+pytestmark = pytest.mark.gpu
+
+
+# a little beyond the rounding of a unit direction, far beyond it, and shorter ones
+@pytest.mark.parametrize("length", [0.1, 0.99, 1.00001, 1.5, 2.0, 50.0])
+@pytest.mark.parametrize("mesh", ["slab", "abdomen"])
+def test_query_takes_directions_of_any_length(mesh, length):
+    """The cell lists against the tree alone: the same triangles and the same bits of t, for
+    bounds from a fraction of a cell to the default, in which the ray's hits lie."""
+    tri, nrm, med = meshes.curved_abdomen(freq=14) if mesh == "abdomen" else (
+        lambda w: (w.tri, w.nrm, w.med))(workloads.plain_slab())
+    rng = np.random.default_rng(8)
+    n = 6007
+    lo, hi = tri.reshape(-1, 3).min(0), tri.reshape(-1, 3).max(0)
+    o = rng.uniform(lo - 0.2 * (hi - lo), hi + 0.2 * (hi - lo), (n, 3))
+    d = rng.normal(size=(n, 3))
+    d *= length / np.linalg.norm(d, axis=1, keepdims=True)
+    t = rng.choice([0.05, 0.7, 5.0, 30.0, 10000.0], n) / length
+    q = (o.astype(np.float32), d.astype(np.float32), np.full(n, -1, np.int32), t.astype(np.float32))
+    got = []
+    for lists in (False, True):
+        with Simulation(0) as s:
+            s.set_mesh(tri, nrm, med)
+            s.set_cell_lists(lists)
+            got.append(s.query(*q))
+    assert np.array_equal(got[0][0], got[1][0])
+    assert np.array_equal(got[0][1].view(np.uint32), got[1][1].view(np.uint32))
+    assert (got[0][0] >= 0).sum() > 300   # enough hits to compare
