@@ -515,7 +515,9 @@ __device__ __forceinline__ void start_photon(const KParams &P, Photon &ph, uint3
     ph.seg_len = 0.0f;
     ph.seg_k = 0;
     ph.safe = 0.0f;
-    ph.word = cell_at(P, ph.px, ph.py, ph.pz);
+    // a source's direction is taken as given: one longer than unit is kept until the first
+    // event, so its first step needs the tree (and no distance bound: a dense cell has none)
+    ph.word = query_word(P, v3(ph.px, ph.py, ph.pz), v3(ph.vx, ph.vy, ph.vz));
 }
 
 // A boundary event (.cl:1443-1465 with TransmitOrReflect, .cl:921-1018): the photon moves

@@ -33,3 +33,37 @@ def test_query_takes_directions_of_any_length(mesh, length):
     assert np.array_equal(got[0][0], got[1][0])
     assert np.array_equal(got[0][1].view(np.uint32), got[1][1].view(np.uint32))
     assert (got[0][0] >= 0).sum() > 300   # enough hits to compare
+
+
+def beam(mesh, length, exterior):
+    """A pencil beam of the workload whose direction has the given length, from air or from a
+    scattering medium around the mesh."""
+    w = workloads.plain_slab() if mesh == "slab" else workloads.curved_abdomen(freq=10)
+    w.fiber_radius = w.fiber_na = 0.0
+    w.v_start = (np.asarray(w.v_start, np.float32) * np.float32(length)).astype(np.float32)
+    w.nmuasg = w.nmuasg.copy()
+    if exterior == "scattering":
+        w.nmuasg[0, 1:] = 0.01, 0.5, 0.8
+    return w
+
+
+@pytest.mark.parametrize("length", [0.3, 1.5, 20.0])
+@pytest.mark.parametrize("exterior", ["air", "scattering"])
+@pytest.mark.parametrize("mesh", ["slab", "abdomen"])
+@pytest.mark.parametrize("exact", [False, True])
+def test_run_takes_a_source_direction_of_any_length(mesh, exterior, length, exact):
+    """The first step goes along the source's direction as given: the tallies of a run with
+    the cell grid are those of a run that descends the tree on every step."""
+    w = beam(mesh, length, exterior)
+    got = []
+    for cells in (0, 1 << 22):
+        with w.apply(Simulation(0), seed=21) as s:
+            s.set_arithmetic(exact)
+            s.set_safety_grid(cells)
+            s.zero()
+            s.run(3000)
+            got.append(s.tallies())
+    for k in ("sft", "rtd", "rz", "vox", "region"):
+        assert np.array_equal(got[0][k], got[1][k]), k
+    c = got[0]["counters"]
+    assert c["scatter"] + c["boundary"] >= 3000   # from air, only a direction of unit length gets in
