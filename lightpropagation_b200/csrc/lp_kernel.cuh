@@ -801,10 +801,11 @@ __device__ __forceinline__ int mesh_query(const KParams &P, const MeshView &SM, 
     const float eps = __ldg(P.mesh_eps);
     int tri = -1;
     t_out = kNoHit;
-    if (P.n_tri > kWholeMesh) {
+    const bool longer = dot3(v, v) > kUnitDot;   // than unit (query_word): no bound, the tree
+    if (P.n_tri > kWholeMesh || __any_sync(0xffffffffu, want && longer)) {
         if (want) {
             bool ray = true;
-            if (ref_tri < 0) {
+            if (ref_tri < 0 && !longer) {
                 const float cap = fminf(64.0f * bound, kNoHit);
                 const float clear = sqrtf(nearest_dist2(SM, p, cap * cap)) * 0.9999f - eps;
                 safe = fmaxf(safe, clear);

@@ -1,9 +1,12 @@
 """Directions of any length: a ray's t counts in units of its direction, as in the reference
 (MCLightPropagation.cl:1037-1093), whichever way the query is answered."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
-from lightpropagation_b200 import Simulation, meshes, workloads
+from lightpropagation_b200 import Simulation, _native, meshes, workloads
+from test_zz_no_alloc import KEYS, _args
 
 pytestmark = pytest.mark.gpu
 
@@ -67,3 +70,37 @@ def test_run_takes_a_source_direction_of_any_length(mesh, exterior, length, exac
         assert np.array_equal(got[0][k], got[1][k]), k
     c = got[0]["counters"]
     assert c["scatter"] + c["boundary"] >= 3000   # from air, only a direction of unit length gets in
+
+
+@pytest.mark.parametrize("length", [0.3, 1.5, 20.0])
+@pytest.mark.parametrize("exterior", ["air", "scattering"])
+@pytest.mark.parametrize("mesh", ["slab", "abdomen"])
+def test_noalloc_takes_a_source_direction_of_any_length(mesh, exterior, length):
+    """lp_run_noalloc with such a beam, on either side of the mesh size up to which a query
+    goes through the whole mesh, gives the tallies of lp_run without the cell grid."""
+    import torch
+
+    w = beam(mesh, length, exterior)
+    w.tri, w.nrm, w.med = w.tri[:_native.NOALLOC_MAX_TRI], w.nrm[:_native.NOALLOC_MAX_TRI], w.med[:_native.NOALLOC_MAX_TRI]
+    n, seed = 3000, 23
+    with w.apply(Simulation(0), seed=seed) as s:
+        s.set_arithmetic(True)
+        s.set_safety_grid(0)
+        s.zero()
+        s.run(n)
+        ref, g = s.tallies(), s.geometry()
+    dev = torch.device("cuda", 0)
+    tri, nrm, med = (torch.from_numpy(np.ascontiguousarray(x, t).ravel()).to(dev)
+                     for x, t in ((w.tri, np.float32), (w.nrm, np.float32), (w.med, np.int32)))
+    nm = np.ascontiguousarray(w.nmuasg, np.float32).ravel()
+    sizes = {"sft": g.sft_nx * g.sft_ny * 3, "rtd": g.dimR * g.dimAlpha * 3, "rz": g.rz_nr * g.rz_nz * 2,
+             "region": w.nmuasg.shape[0], "counters": 16}
+    out = {k: torch.zeros(v, dtype=torch.int64, device=dev) for k, v in sizes.items()}
+    a = _args(w, seed, n, tri, nrm, med, nm, out)
+    rc = _native.lib().lp_run_noalloc(C.byref(a), C.c_void_p(torch.cuda.current_stream(dev).cuda_stream))
+    assert rc == 0
+    torch.cuda.synchronize(dev)
+    for k in KEYS:
+        assert np.array_equal(out[k].cpu().numpy().view(np.uint64), ref[k].ravel()), k
+    cnt = out["counters"].cpu().numpy()
+    assert int(cnt[8]) == n and int(cnt[0]) == ref["counters"]["scatter"]
