@@ -689,40 +689,45 @@ __device__ __forceinline__ int warp_query(const KParams &P, const MeshView &M, c
     return tri;
 }
 
-// Squared distance from p to the triangle (a, a + ab, a + ac): closest point by Voronoi
-// regions of the vertices, edges and face (Ericson, Real-Time Collision Detection, 2005).
-__device__ __forceinline__ float point_triangle_dist2(V3 p, V3 a, V3 ab, V3 ac)
+// Lower bound of the distance from p to the triangle (a, a + ab, a + ac): the closest point q
+// by Voronoi regions of the vertices, edges and face (Ericson, Real-Time Collision Detection,
+// 2005), then the smallest of the vertices' distances along p - q, which no point of the
+// triangle falls short of.  With the right q that is |p - q|; on slivers (aspect ratios from a
+// few hundred on) the weights of q are lost in the rounding, and |p - q| can be far above the
+// distance, where this stays below it (to the rounding of one product).
+__device__ __forceinline__ float triangle_clearance(V3 p, V3 a, V3 ab, V3 ac)
 {
-    const V3 ap = sub3(p, a);
+    const V3 ap = sub3(p, a), bp = sub3(ap, ab), cp = sub3(ap, ac);
     const float d1 = dot3(ab, ap), d2 = dot3(ac, ap);
-    V3 q;
+    const float d3 = dot3(ab, bp), d4 = dot3(ac, bp);
+    const float d5 = dot3(ab, cp), d6 = dot3(ac, cp);
+    const float vc = d1 * d4 - d3 * d2, vb = d5 * d2 - d1 * d6, va = d3 * d6 - d5 * d4;
+    float u, w;   // q = a + u ab + w ac
     if (d1 <= 0.0f && d2 <= 0.0f) {
-        q = a;
+        u = w = 0.0f;
+    } else if (d3 >= 0.0f && d4 <= d3) {
+        u = 1.0f;
+        w = 0.0f;
+    } else if (vc <= 0.0f && d1 >= 0.0f && d3 <= 0.0f) {
+        u = d1 / (d1 - d3);
+        w = 0.0f;
+    } else if (d6 >= 0.0f && d5 <= d6) {
+        u = 0.0f;
+        w = 1.0f;
+    } else if (vb <= 0.0f && d2 >= 0.0f && d6 <= 0.0f) {
+        u = 0.0f;
+        w = d2 / (d2 - d6);
+    } else if (va <= 0.0f && (d4 - d3) >= 0.0f && (d5 - d6) >= 0.0f) {
+        w = (d4 - d3) / ((d4 - d3) + (d5 - d6));
+        u = 1.0f - w;
     } else {
-        const V3 b = add3(a, ab), c = add3(a, ac);
-        const V3 bp = sub3(p, b);
-        const float d3 = dot3(ab, bp), d4 = dot3(ac, bp);
-        const V3 cp = sub3(p, c);
-        const float d5 = dot3(ab, cp), d6 = dot3(ac, cp);
-        const float vc = d1 * d4 - d3 * d2, vb = d5 * d2 - d1 * d6, va = d3 * d6 - d5 * d4;
-        if (d3 >= 0.0f && d4 <= d3) {
-            q = b;
-        } else if (vc <= 0.0f && d1 >= 0.0f && d3 <= 0.0f) {
-            q = add3(a, scl3(d1 / (d1 - d3), ab));
-        } else if (d6 >= 0.0f && d5 <= d6) {
-            q = c;
-        } else if (vb <= 0.0f && d2 >= 0.0f && d6 <= 0.0f) {
-            q = add3(a, scl3(d2 / (d2 - d6), ac));
-        } else if (va <= 0.0f && (d4 - d3) >= 0.0f && (d5 - d6) >= 0.0f) {
-            const float w = (d4 - d3) / ((d4 - d3) + (d5 - d6));
-            q = add3(b, scl3(w, sub3(c, b)));
-        } else {
-            const float den = 1.0f / (va + vb + vc);
-            q = add3(a, add3(scl3(vb * den, ab), scl3(vc * den, ac)));
-        }
+        const float den = 1.0f / (va + vb + vc);
+        u = vb * den;
+        w = vc * den;
     }
-    const V3 d = sub3(p, q);
-    return dot3(d, d);
+    const V3 d = sub3(sub3(ap, scl3(u, ab)), scl3(w, ac));
+    const float m = fminf(fminf(dot3(d, ap), dot3(d, bp)), dot3(d, cp)) * rsqrtf(dot3(d, d));
+    return m > 0.0f ? m : 0.0f;   // 0 too where q is not a number
 }
 
 __device__ __forceinline__ float box_dist2(float lo_x, float hi_x, float lo_y, float hi_y, float lo_z, float hi_z,
@@ -734,10 +739,13 @@ __device__ __forceinline__ float box_dist2(float lo_x, float hi_x, float lo_y, f
     return dx * dx + dy * dy + dz * dz;
 }
 
-// Squared distance from p to the nearest triangle, or cap2 if none is closer.
-static __device__ __noinline__ float nearest_dist2(const MeshView &M, V3 p, float cap2)
+// Lower bound of the distance from p to every triangle (triangle_clearance), at most cap.
+// lp_run_noalloc, 50,000 photons, with the closest points' distances as they were / the bounds /
+// the bounds behind the test of the plane: slab in 512 triangles 618 / 670 / 474 ms, in 2,048
+// 1,823 / 2,079 / 1,417, abdomen in 3,600 251 / 258 / 235.
+static __device__ __noinline__ float mesh_clearance(const MeshView &M, V3 p, float cap)
 {
-    float best = cap2;
+    float best = cap;
     int stack[kStackDepth];
     int sp = 0, node = 0;
     for (;;) {
@@ -754,16 +762,21 @@ static __device__ __noinline__ float nearest_dist2(const MeshView &M, V3 p, floa
         bool open[2];
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-            open[k] = dist[k] < best && ref[k] >= 0;
-            if (!(dist[k] < best) || ref[k] >= 0) continue;
+            const bool near = dist[k] < best * best;
+            open[k] = near && ref[k] >= 0;
+            if (!near || ref[k] >= 0) continue;
             const int e = ~ref[k], f = e >> 3, cnt = (e & 7) + 1;
             for (int j = f; j < f + cnt; ++j) {
                 if (!LP_IN_RANGE(M.dbg, j, M.n_tri)) return 0.0f;
                 TriRec T;
                 if (j < M.tris_smem) T = TriRec{M.s_tri[3 * j], M.s_tri[3 * j + 1], M.s_tri[3 * j + 2]};
                 else T = load_tri(M.tri, j);
-                best = fminf(best, point_triangle_dist2(p, v3(T.a.x, T.a.y, T.a.z), v3(T.a.w, T.b.x, T.b.y),
-                                                        v3(T.b.z, T.b.w, T.c.x)));
+                const V3 a = v3(T.a.x, T.a.y, T.a.z), E = v3(T.a.w, T.b.x, T.b.y), F = v3(T.b.z, T.b.w, T.c.x);
+                // its plane's distance (see warp_query) is a bound too: good enough when hardly
+                // below what there is
+                const V3 G = sub3(p, a);
+                const float d = fabsf(dot3(cross3(G, E), F)) * T.c.z - T.c.w * (fabsf(G.x) + fabsf(G.y) + fabsf(G.z));
+                best = fminf(best, d >= 0.98f * best ? d : triangle_clearance(p, a, E, F));
             }
         }
         if (open[0] && open[1]) {
@@ -807,7 +820,7 @@ __device__ __forceinline__ int mesh_query(const KParams &P, const MeshView &SM, 
             bool ray = true;
             if (ref_tri < 0 && !longer) {
                 const float cap = fminf(64.0f * bound, kNoHit);
-                const float clear = sqrtf(nearest_dist2(SM, p, cap * cap)) * 0.9999f - eps;
+                const float clear = mesh_clearance(SM, p, cap) * 0.9999f - eps;
                 safe = fmaxf(safe, clear);
                 ray = !(bound < clear);
             }
