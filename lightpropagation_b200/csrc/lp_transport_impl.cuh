@@ -75,7 +75,7 @@ struct Photon {
     float seg_len;           // differentiation: path length and interactions in the
     uint32_t seg_k;          // current region since the photon entered it
     float safe;              // lower bound of the distance from the position to any triangle
-    uint32_t word;           // cell word at the position (cell_at)
+    uint32_t word;           // cell word at the position (cell_at); without a grid mesh_query's `rest`
 };
 
 // Per-photon, per-region path lengths and interaction counts of a differentiated run
@@ -677,7 +677,7 @@ struct Pending {
 // whose step needs a query with `want`.
 template <int STACK, bool NoGrid>
 __device__ __forceinline__ int query_step(const KParams &P, const MeshView &M, const MeshView &SM, WarpQueue &Q,
-                                          const Medium *s_media, bool want, const Photon &ph, Counters &cnt,
+                                          const Medium *s_media, bool want, Photon &ph, Counters &cnt,
                                           Pending &pd, float &thit)
 {
     thit = kNoHit;
@@ -688,8 +688,8 @@ __device__ __forceinline__ int query_step(const KParams &P, const MeshView &M, c
         cnt.query += want ? 1u : 0u;
         cnt.bvh += want ? 1u : 0u;
         return mesh_query<STACK>(P, SM, want, v3(ph.px, ph.py, ph.pz), v3(ph.vx, ph.vy, ph.vz),
-                                 (ph.flags & F_ON_FACE) ? ph.last_tri : -1, ambient ? kNoHit : pd.reach, thit,
-                                 pd.safe_here);
+                                 (ph.flags & F_ON_FACE) ? ph.last_tri : -1, ambient ? kNoHit : pd.reach,
+                                 ambient ? 0.0f : P.factor * s_media[ph.curr].inv_mut, thit, pd.safe_here, ph.word);
     }
     // an empty cell: pd.safe_here holds its bound, which the step exceeds; a listed cell
     // raises it from the planes of its triangles when its list decides the step
@@ -847,7 +847,7 @@ __device__ __forceinline__ bool step_photon(const KParams &P, const MeshView &M,
     // A step shorter than it cannot reach a triangle, so its bounded query would return "no
     // hit" and is skipped; after the step the bound shrinks by the step (plus the rounding of
     // the move).
-    pd.safe_here = fmaxf(ph.safe, safe_distance(P, ph.word));
+    pd.safe_here = NoGrid ? ph.safe : fmaxf(ph.safe, safe_distance(P, ph.word));
     const bool want = alive && (ambient || !(pd.reach < pd.safe_here));
     float thit;
     const int tri = query_step<STACK, NoGrid>(P, M, SM, Q, s_media, want, ph, cnt, pd, thit);
@@ -967,6 +967,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) transport_kernel(const __gr
                 const unsigned long long idx = base + __popc(need & lt_mask);
                 if (idx < (unsigned long long)P.n) {
                     start_photon(P, ph, (uint32_t)idx);
+                    if (NoGrid) ph.word = kRestFirst << 8 | kRestFirst;
                     if (Grad) {
                         for (int r = 0; r < P.n_media; ++r) {
                             ga.L[r] = 0.0f;
