@@ -811,8 +811,9 @@ static __device__ __noinline__ float mesh_clearance(const MeshView &M, V3 p, flo
 //     as usual (50,000 photons) / a tenth / a fiftieth (200,000): ray alone 739 / 229 / 67 ms,
 //     search on every query 235 / 403 / 189, this rule 203 / 271 / 76.
 // Slab (32 triangles), 50,000 photons in reference arithmetic: 186 ms with a descent on every
-// step, 118 with the tree's bounds, 55 with the whole mesh (8 rounds at kWholeMesh triangles
-// cost a query about what its descents do).
+// step, 118 with the tree's bounds, 55 with the whole mesh.  256 triangles of an abdomen: 82 ms
+// through the tree, 46 with the whole mesh, so kWholeMesh is on the safe side (400 of them: 114
+// and 82).
 constexpr int kWholeMesh = 256;
 constexpr uint32_t kRestFirst = 31, kRestMost = 63;
 template <int STACK = kStackDepth>

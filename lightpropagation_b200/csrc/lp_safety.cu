@@ -38,8 +38,12 @@ __device__ bool tri_cube_overlap(V3 c, float r, V3 a, V3 b, V3 d)
         rr = r * (fabsf(f.x) + fabsf(f.y));
         if (fminf(p0, fminf(p1, p2)) > rr || fmaxf(p0, fmaxf(p1, p2)) < -rr) return false;
     }
+    // of a sliver the normal may be nothing but rounding: an axis like any other then, along
+    // which the vertices do not coincide
     const V3 n = cross3(e[0], e[1]);
-    return fabsf(dot3(n, v0)) <= r * (fabsf(n.x) + fabsf(n.y) + fabsf(n.z));
+    const float p0 = dot3(n, v0), p1 = dot3(n, v1), p2 = dot3(n, v2);
+    const float rr = r * (fabsf(n.x) + fabsf(n.y) + fabsf(n.z));
+    return fminf(p0, fminf(p1, p2)) <= rr && fmaxf(p0, fmaxf(p1, p2)) >= -rr;
 }
 
 // One pass over the triangles (BVH order): every cell that a triangle touches (cells

@@ -60,3 +60,40 @@ def test_noalloc_bounds_on_slivers(parts, turn):
     for k in KEYS:
         assert np.array_equal(out[k].cpu().numpy().view(np.uint64), ref[k].ravel()), k
     assert int(cnt[8]) == n and int(cnt[0]) == ref["counters"]["scatter"]
+
+
+@pytest.mark.parametrize("aspect", [1e3, 1e5, 1e6])
+def test_cell_lists_hold_slivers(aspect):
+    """Needles in every direction and rays aimed at them: the lists' triangles and bits of t are
+    the tree's, with a margin and without one that neighbouring cells would make up for.  (From
+    1e7 on a width is a unit or two of the coordinates, and the hit test itself, as the
+    reference has it, can put a hit millimetres off the needle, where no list looks for it.)"""
+    rng = np.random.default_rng(3)
+    n = 3000
+    a = rng.uniform(-60, 60, (n, 3))
+    e, f = rng.normal(size=(2, n, 3))
+    e *= rng.uniform(10, 80, (n, 1)) / np.linalg.norm(e, axis=1, keepdims=True)
+    f *= np.linalg.norm(e, axis=1, keepdims=True) / aspect / np.linalg.norm(f, axis=1, keepdims=True)
+    tri = np.stack([a, a + e, a + rng.uniform(0, 1, (n, 1)) * e + f], 1).astype(np.float32)
+    nrm = np.tile(np.array([0, 0, 1], np.float32), (n, 1))
+    med = np.tile(np.array([1, 0], np.int32), (n, 1))
+    k = rng.integers(0, n, 40000)
+    u = rng.uniform(0, 1, (len(k), 2))
+    u = np.where(u.sum(1, keepdims=True) > 1, 1 - u, u)
+    t = tri.astype(np.float64)[k]
+    x = t[:, 0] + u[:, :1] * (t[:, 1] - t[:, 0]) + u[:, 1:] * (t[:, 2] - t[:, 0])
+    d = rng.normal(size=x.shape)
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    o = (x - d * rng.choice([0.3, 3.0, 30.0], (len(k), 1))).astype(np.float32)
+    q = (o, d.astype(np.float32), np.full(len(k), -1, np.int32),
+         rng.choice([0.4, 4.0, 40.0, 10000.0], len(k)).astype(np.float32))
+    for margin in (0.0, 0.5):
+        got = []
+        for lists in (False, True):
+            with Simulation(0) as s:
+                s.set_mesh(tri.reshape(-1, 9), nrm, med)
+                s.set_cell_margin(margin)
+                s.set_cell_lists(lists)
+                got.append(s.query(*q))
+        assert np.array_equal(got[0][0], got[1][0]), margin
+        assert np.array_equal(got[0][1].view(np.uint32), got[1][1].view(np.uint32)), margin
