@@ -320,6 +320,9 @@ int lp_l2_atomic_peak(int device, double *per_s);
  * (the call that needed it returns LP_ERR_NOMEM and leaves its context usable); -1
  * switches the injection off.  Process-wide. */
 int lp_debug_fail_allocation(int64_t after);
+/* Test hook, the same for the launches of the transport, batch and r-z fold kernels: the one
+ * after `after` more fails (the call returns LP_ERR_CUDA) without being made. */
+int lp_debug_fail_launch(int64_t after);
 
 /* --- transport without device allocation ------------------------------------- */
 /* No counterpart in the reference.  For callers that must not allocate device memory

@@ -133,6 +133,7 @@ _SIGS = {
     "lp_fp32_peak": ([C.c_int, C.POINTER(C.c_double)], C.c_int),
     "lp_l2_atomic_peak": ([C.c_int, C.POINTER(C.c_double)], C.c_int),
     "lp_debug_fail_allocation": ([C.c_int64], C.c_int),
+    "lp_debug_fail_launch": ([C.c_int64], C.c_int),
     "lp_run_noalloc": ([C.POINTER(NoAllocArgs), C.c_void_p], C.c_int),
     "lp_batch_config_count": ([], C.c_int),
     "lp_batch_config_info": ([C.c_int32, _ip, _ip, _ip], C.c_int),

@@ -71,14 +71,24 @@ struct Phase {
 // Allocation-failure injection (lp_debug_fail_allocation): the allocation that brings the
 // countdown from 0 to -1 reports cudaErrorMemoryAllocation without allocating.
 std::atomic<int64_t> g_alloc_countdown{-1};
+// Launch-failure injection (lp_debug_fail_launch), the same for the transport, batch and fold
+// launches: cudaErrorLaunchOutOfResources without launching.
+std::atomic<int64_t> g_launch_countdown{-1};
 
-bool injected_alloc_failure()
+bool counted_down(std::atomic<int64_t> &countdown)
 {
-    int64_t v = g_alloc_countdown.load();
+    int64_t v = countdown.load();
     while (v >= 0) {
-        if (g_alloc_countdown.compare_exchange_weak(v, v - 1)) return v == 0;
+        if (countdown.compare_exchange_weak(v, v - 1)) return v == 0;
     }
     return false;
+}
+bool injected_alloc_failure() { return counted_down(g_alloc_countdown); }
+
+template <class Launch>
+cudaError_t launch_unless_injected(Launch launch)
+{
+    return counted_down(g_launch_countdown) ? cudaErrorLaunchOutOfResources : launch();
 }
 
 template <class T>
@@ -239,6 +249,7 @@ struct lp_ctx {
     DevBuf<Medium> media;
     DevBuf<unsigned long long> sft, rtd, rz, vox, rbins, region, det, counters, work;
     DevBuf<unsigned long long> rz_part;   // copies of rz (KParams::rz_part), zero between launches
+    bool rz_pending = false;              // but for deposits that are still to be folded (fold_rz)
     DevBuf<float> exit_rec;
     // safety grid (lp_set_safety_grid)
     // shared memory per block for staged BVH nodes and triangles: 8 KB stages a small mesh whole,
@@ -360,6 +371,7 @@ int alloc_tallies(lp_ctx *c)
         LP_CUDA(c, c->rz_part.ensure(rz_values(c) * copies));
         LP_CUDA(c, cudaMemsetAsync(c->rz_part.p, 0, rz_values(c) * copies * 8, c->stream));
     }
+    c->rz_pending = false;
     LP_CUDA(c, c->vox.ensure((size_t)std::max<int64_t>(n_vox(c), 1)));
     LP_CUDA(c, c->rbins.ensure((size_t)std::max(c->n_rbins, 1) * 2));
     LP_CUDA(c, c->region.ensure(lp::kMaxMedia));
@@ -370,10 +382,35 @@ int alloc_tallies(lp_ctx *c)
     return LP_OK;
 }
 
+// Adds the deposits in the copies of the r-z image to it: after the launches of every run, the
+// ones that did start when a later one failed included, and once more where the tallies are
+// read if that launch failed too.
+cudaError_t fold_rz(lp_ctx *c)
+{
+    if (!c->rz_pending) return cudaSuccess;
+    const int copies = rz_copies(rz_values(c));
+    const cudaError_t e = launch_unless_injected([&] {
+        return lp::launch_fold(c->rz.p, c->rz_part.p, copies, (int64_t)rz_values(c), 1, c->stream);
+    });
+    if (e == cudaSuccess) c->rz_pending = false;
+    return e;
+}
+
+// Drops deposits that are still to be folded, before the tallies are set to something else.
+cudaError_t clear_rz_copies(lp_ctx *c)
+{
+    if (!c->rz_pending) return cudaSuccess;
+    const cudaError_t e =
+        cudaMemsetAsync(c->rz_part.p, 0, rz_values(c) * rz_copies(rz_values(c)) * 8, c->stream);
+    if (e == cudaSuccess) c->rz_pending = false;
+    return e;
+}
+
 int zero_tallies(lp_ctx *c)
 {
     const lp_geometry &g = c->geo;
     cudaStream_t s = c->stream;
+    LP_CUDA(c, clear_rz_copies(c));
     LP_CUDA(c, cudaMemsetAsync(c->sft.p, 0, (size_t)g.sft_nx * g.sft_ny * 3 * 8, s));
     LP_CUDA(c, cudaMemsetAsync(c->rtd.p, 0, (size_t)g.dimR * g.dimAlpha * 3 * 8, s));
     LP_CUDA(c, cudaMemsetAsync(c->rz.p, 0, (size_t)g.rz_nr * g.rz_nz * 2 * 8, s));
@@ -1110,7 +1147,9 @@ int lp_run_async(lp_ctx *c, int64_t first, int64_t n)
     // The kernel indexes the photons of one launch with 32 bits: a longer range runs as
     // several launches in order (the same photon ids, so the same tallies).  Exit records
     // (at most 2^30 slots, indexed from the range's first photon) all come from the first.
-    for (int64_t off = 0; off < n; off += lp::kMaxLaunchPhotons) {
+    const bool copies = rz_copies(rz_values(c)) > 1;
+    cudaError_t e = cudaSuccess;
+    for (int64_t off = 0; off < n && e == cudaSuccess; off += lp::kMaxLaunchPhotons) {
         const int64_t m = std::min<int64_t>(n - off, lp::kMaxLaunchPhotons);
         KParams P;
         fill_params(c, P, first + off, m, nodes_smem, tris_smem);
@@ -1121,14 +1160,18 @@ int lp_run_async(lp_ctx *c, int64_t first, int64_t n)
         int grid;
         lp::plan_launch(m, lp::block_size(), c->num_sms, per_sm, grid, P.lane_mask, P.few_blocks);
         c->st_grid = grid;
-        LP_CUDA(c, cudaMemsetAsync(c->work.p, 0, 8, c->stream));
         c->h2d_bytes += (int64_t)sizeof(KParams);
-        LP_CUDA(c, c->exact ? lp::launch_transport_exact(P, grid, smem, c->stream)
-                            : lp::launch_transport_fast(P, grid, smem, c->stream));
+        e = cudaMemsetAsync(c->work.p, 0, 8, c->stream);
+        if (e == cudaSuccess)
+            e = launch_unless_injected([&] {
+                return c->exact ? lp::launch_transport_exact(P, grid, smem, c->stream)
+                                : lp::launch_transport_fast(P, grid, smem, c->stream);
+            });
+        if (e == cudaSuccess) c->rz_pending = copies;
     }
-    const int copies = rz_copies(rz_values(c));
-    if (copies > 1)
-        LP_CUDA(c, lp::launch_fold(c->rz.p, c->rz_part.p, copies, (int64_t)rz_values(c), 1, c->stream));
+    const cudaError_t folded = fold_rz(c);
+    if (e == cudaSuccess) e = folded;
+    if (e != cudaSuccess) return cuda_fail(c, e, "lp_run: launch");
     LP_CUDA(c, cudaEventRecord(c->ev1, c->stream));
     c->launched = true;
     return LP_OK;
@@ -1184,6 +1227,7 @@ int lp_get_tallies(lp_ctx *c, lp_tallies *out)
     LP_CUDA(c, c->h_rbins.resize((size_t)c->n_rbins * 2));
     LP_CUDA(c, c->h_region.resize((size_t)c->n_media));
     LP_CUDA(c, c->h_det.resize(c->det_r.size()));
+    LP_CUDA(c, fold_rz(c));
     cudaStream_t s = c->stream;
     LP_CUDA(c, cudaMemcpyAsync(c->h_sft.data(), c->sft.p, c->h_sft.size() * 8, cudaMemcpyDeviceToHost, s));
     LP_CUDA(c, cudaMemcpyAsync(c->h_rtd.data(), c->rtd.p, c->h_rtd.size() * 8, cudaMemcpyDeviceToHost, s));
@@ -1235,6 +1279,7 @@ int lp_set_tallies(lp_ctx *c, const lp_tallies *in)
         if (r) return r;
         c->tally_dirty = false;
     }
+    LP_CUDA(c, clear_rz_copies(c));
     cudaStream_t s = c->stream;
     LP_CUDA(c, cudaMemcpyAsync(c->sft.p, in->sft, (size_t)g.sft_nx * g.sft_ny * 3 * 8, cudaMemcpyHostToDevice, s));
     LP_CUDA(c, cudaMemcpyAsync(c->rtd.p, in->rtd, (size_t)g.dimR * g.dimAlpha * 3 * 8, cudaMemcpyHostToDevice, s));
@@ -1311,6 +1356,7 @@ int lp_get_device_tallies(lp_ctx *c, lp_device_tallies *out)
 {
     if (!c || !out) return fail(c, LP_ERR_INVALID, "lp_get_device_tallies: NULL argument");
     if (c->tally_dirty || !c->sft.p) return fail(c, LP_ERR_STATE, "lp_get_device_tallies: tallies not allocated yet");
+    LP_CUDA(c, fold_rz(c));
     const lp_geometry &g = c->geo;
     out->sft = (uint64_t *)c->sft.p;
     out->rtd = (uint64_t *)c->rtd.p;
@@ -1350,6 +1396,12 @@ int lp_fp32_peak(int device, double *tflops)
 int lp_debug_fail_allocation(int64_t after)
 {
     g_alloc_countdown.store(after < 0 ? -1 : after);
+    return LP_OK;
+}
+
+int lp_debug_fail_launch(int64_t after)
+{
+    g_launch_countdown.store(after < 0 ? -1 : after);
     return LP_OK;
 }
 
@@ -1474,6 +1526,7 @@ struct lp_batch {
     // copies of the r-z images (KParams::rz_part), zero between launches: [instance][copy] of
     // the batch launch, and one set that the plain launches use in turn
     DevBuf<unsigned long long> rz_part, plain_rz_part;
+    bool rz_pending = false;   // rz_part holds deposits of a launch whose fold failed
     // The r-z and voxel tallies (the atomic targets of every scatter event) of the
     // instances with a launch of their own sit in buffers of their own, like a context's: as
     // slices of the batch's large arrays the same launch measured up to 15 % slower (before the
@@ -1678,10 +1731,12 @@ int enqueue_launch(lp_batch *b, int config)
     B.cum = b->cum.p;
     B.n_inst = (int32_t)b->inst.size();
     B.lane_mask = b->lane_mask;
-    LP_BCUDA(b, lp::launch_batch(config, b->grad_on, B, b->grid, b->stream));
+    LP_BCUDA(b, launch_unless_injected([&] { return lp::launch_batch(config, b->grad_on, B, b->grid, b->stream); }));
     const int copies = rz_copies(b->n_rz, b->inst.size());
     if (copies > 1)
-        LP_BCUDA(b, lp::launch_fold(b->rz.p, b->rz_part.p, copies, (int64_t)b->n_rz, (int64_t)b->inst.size(), b->stream));
+        LP_BCUDA(b, launch_unless_injected([&] {
+            return lp::launch_fold(b->rz.p, b->rz_part.p, copies, (int64_t)b->n_rz, (int64_t)b->inst.size(), b->stream);
+        }));
     return LP_OK;
 }
 
@@ -1701,14 +1756,27 @@ int64_t total_photons(const std::vector<lp_instance> &v)
     return t;
 }
 
+// Drops deposits that a failed fold left in the copies of the r-z images (every launch zeroes
+// the tallies, so they belong to none).
+int clear_rz_copies(lp_batch *b)
+{
+    if (!b->rz_pending) return LP_OK;
+    LP_BCUDA(b, cudaMemsetAsync(b->rz_part.p, 0, b->rz_part.n * 8, b->stream));
+    b->rz_pending = false;
+    return LP_OK;
+}
+
 // One direct (ungraphed) launch of `config`; device milliseconds of the kernel.
 int timed_launch(lp_batch *b, int config, float *ms)
 {
     int r = prepare_grid(b, config);
     if (r) return r;
+    if ((r = clear_rz_copies(b))) return r;
     if ((r = enqueue_zero(b))) return r;
     LP_BCUDA(b, cudaEventRecord(b->ev0, b->stream));
+    b->rz_pending = true;
     if ((r = enqueue_launch(b, config))) return r;
+    b->rz_pending = false;
     LP_BCUDA(b, cudaEventRecord(b->ev1, b->stream));
     LP_BCUDA(b, cudaEventSynchronize(b->ev1));
     LP_BCUDA(b, cudaEventElapsedTime(ms, b->ev0, b->ev1));
@@ -1968,6 +2036,7 @@ int lp_batch_run(lp_batch *b)
         b->graph = g;
         LP_BCUDA(b, cudaGraphInstantiate(&b->exec, b->graph, 0));
     }
+    if ((r = clear_rz_copies(b))) return r;
     LP_BCUDA(b, cudaEventRecord(b->ev0, b->stream));
     LP_BCUDA(b, cudaGraphLaunch(b->exec, b->stream));
     LP_BCUDA(b, cudaEventRecord(b->ev1, b->stream));
