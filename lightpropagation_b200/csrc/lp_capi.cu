@@ -1783,6 +1783,34 @@ int timed_launch(lp_batch *b, int config, float *ms)
     return LP_OK;
 }
 
+// Times every eligible configuration on the instances as they are set: the fastest one's index
+// and the nanoseconds per photon of each (-1: not eligible).
+int time_configs(lp_batch *b, int &chosen, double *ns_per_photon)
+{
+    const double n_trial = (double)std::max<int64_t>(total_photons(b->inst), 1);
+    double best_ns = 0.0;
+    bool warmed = false;
+    int r;
+    for (int k = 0; k < lp::batch_config_count(); ++k) {
+        double ns = -1.0;
+        if (config_eligible(b, k)) {
+            float ms = 0.0f;
+            if (!warmed) {   // first launch of the process pays for module loading
+                if ((r = timed_launch(b, k, &ms))) return r;
+                warmed = true;
+            }
+            if ((r = timed_launch(b, k, &ms))) return r;
+            ns = (double)ms * 1e6 / n_trial;
+            if (chosen < 0 || ns < best_ns) {
+                chosen = k;
+                best_ns = ns;
+            }
+        }
+        if (ns_per_photon) ns_per_photon[k] = ns;
+    }
+    return LP_OK;
+}
+
 int copy_counts(lp_batch *b)
 {
     const size_t I = b->inst.size();
@@ -1968,7 +1996,6 @@ int lp_batch_autotune(lp_batch *b, int64_t photons, int32_t *best, double *ns_pe
     if (!b) return fail(nullptr, LP_ERR_INVALID, "lp_batch_autotune: batch is NULL");
     if (b->inst.empty()) return bfail(b, LP_ERR_STATE, "lp_batch_autotune: no instances");
     LP_BCUDA(b, cudaSetDevice(b->device));
-    const int K = lp::batch_config_count();
     const std::vector<lp_instance> saved = b->inst;
     const int64_t total = std::max<int64_t>(total_photons(saved), 1);
     const double scale = photons > 0 ? std::min(1.0, (double)photons / (double)total) : 1.0;
@@ -1976,29 +2003,13 @@ int lp_batch_autotune(lp_batch *b, int64_t photons, int32_t *best, double *ns_pe
     for (lp_instance &x : trial)
         if (x.n_photons > 0) x.n_photons = std::max<int64_t>(std::min<int64_t>(x.n_photons, 32), (int64_t)(x.n_photons * scale));
     int r = lp_batch_set_instances(b, (int32_t)trial.size(), trial.data());
-    if (r) return r;
-    const double n_trial = (double)std::max<int64_t>(total_photons(trial), 1);
     int chosen = -1;
-    double best_ns = 0.0;
-    bool warmed = false;
-    for (int k = 0; k < K; ++k) {
-        double ns = -1.0;
-        if (config_eligible(b, k)) {
-            float ms = 0.0f;
-            if (!warmed) {   // first launch of the process pays for module loading
-                if ((r = timed_launch(b, k, &ms))) return r;
-                warmed = true;
-            }
-            if ((r = timed_launch(b, k, &ms))) return r;
-            ns = (double)ms * 1e6 / n_trial;
-            if (chosen < 0 || ns < best_ns) {
-                chosen = k;
-                best_ns = ns;
-            }
-        }
-        if (ns_per_photon) ns_per_photon[k] = ns;
-    }
-    if ((r = lp_batch_set_instances(b, (int32_t)saved.size(), saved.data()))) return r;
+    if (!r) r = time_configs(b, chosen, ns_per_photon);
+    // the caller's budgets are put back whatever the trials came to
+    const std::string err = b->err;
+    const int back = lp_batch_set_instances(b, (int32_t)saved.size(), saved.data());
+    if (r) return bfail(b, r, "%s", err.c_str());
+    if (back) return back;
     if (chosen < 0) return bfail(b, LP_ERR_RANGE, "lp_batch_autotune: no configuration fits these meshes");
     drop_graph(b);
     b->config = chosen;

@@ -77,3 +77,19 @@ def test_batch(fail_launch, which):
         b.run()
         equal(b.tallies(0), clean([(32, 0)]))
         equal(b.tallies(1), clean([(28, 32)]))
+
+
+@pytest.mark.parametrize("which", [0, 1, 4])
+def test_autotuner_puts_the_budgets_back(fail_launch, which):
+    w = workloads.plain_slab()
+    with w.apply(Simulation(0), seed=4) as s, Batch([s]) as b:
+        b.set_plain_threshold(0)
+        b.set_instances([Instance(0, w.nmuasg, N, 0), Instance(0, w.nmuasg, 2 * N, N)])
+        fail_launch(which)
+        with pytest.raises(_native.LPError, match="launch"):
+            b.autotune(64)
+        fail_launch(-1)
+        b.set_config(0)
+        b.run()
+        equal(b.tallies(0), clean([(N, 0)]))
+        equal(b.tallies(1), clean([(2 * N, N)]))
