@@ -1572,9 +1572,44 @@ void drop_graph(lp_batch *b)
 
 size_t grad_stride(const lp_batch *b) { return std::max<size_t>(b->n_det, 1) * lp::kBatchMedia * 5; }
 
+// After a failure between the old and the new instances: buffers may have been replaced that
+// the parameters on the device still point to, so the batch has no instances until the next
+// lp_batch_set_instances.
+void drop_instances(lp_batch *b)
+{
+    drop_graph(b);
+    b->inst.clear();
+    b->plain.clear();
+}
+
+// The tallies and parameters of I instances.
+int alloc_instances(lp_batch *b, size_t I)
+{
+    const size_t J = std::max<size_t>(I, 1);
+    LP_BCUDA(b, b->sft.ensure(J * b->n_sft));
+    LP_BCUDA(b, b->rtd.ensure(J * b->n_rtd));
+    LP_BCUDA(b, b->rz.ensure(J * b->n_rz));
+    const int copies = rz_copies(b->n_rz, J);
+    if (copies > 1) {
+        LP_BCUDA(b, b->rz_part.ensure(J * copies * b->n_rz));
+        LP_BCUDA(b, cudaMemsetAsync(b->rz_part.p, 0, J * copies * b->n_rz * 8, b->stream));
+    }
+    LP_BCUDA(b, b->vox.ensure(J * std::max<size_t>(b->n_vox, 1)));
+    LP_BCUDA(b, b->rbins.ensure(J * std::max<size_t>(b->n_rbins, 1)));
+    LP_BCUDA(b, b->region.ensure(J * lp::kBatchMedia));
+    LP_BCUDA(b, b->det.ensure(J * std::max<size_t>(b->n_det, 1) * 2));
+    LP_BCUDA(b, b->counters.ensure(J * LP_NCOUNTERS));
+    LP_BCUDA(b, b->grad.ensure(J * grad_stride(b)));
+    LP_BCUDA(b, b->claimed.ensure(J));
+    LP_BCUDA(b, b->cum.ensure(J + 1));
+    LP_BCUDA(b, b->media.ensure(J * lp::kBatchMedia));
+    LP_BCUDA(b, b->params.ensure(J));
+    return LP_OK;
+}
+
 // Per-instance parameters: the context's (mesh, source, tally layout, run parameters)
 // with the instance's media, photon range and tally slices.
-int upload_instances(lp_batch *b)
+int fill_instances(lp_batch *b)
 {
     const size_t I = b->inst.size();
     std::vector<KParams> P(I);
@@ -1657,6 +1692,13 @@ int upload_instances(lp_batch *b)
         LP_BCUDA(b, cudaStreamSynchronize(b->stream));
     }
     return LP_OK;
+}
+
+int upload_instances(lp_batch *b)
+{
+    const int r = fill_instances(b);
+    if (r) drop_instances(b);
+    return r;
 }
 
 // Zero the tallies and claim counters of all instances (enqueued on the batch stream).
@@ -1924,25 +1966,11 @@ int lp_batch_set_instances(lp_batch *b, int32_t n_inst, const lp_instance *in)
     const size_t I = (size_t)n_inst;
     if (I != b->inst.size() || !b->params.p) {
         drop_graph(b);
-        const size_t J = std::max<size_t>(I, 1);
-        LP_BCUDA(b, b->sft.ensure(J * b->n_sft));
-        LP_BCUDA(b, b->rtd.ensure(J * b->n_rtd));
-        LP_BCUDA(b, b->rz.ensure(J * b->n_rz));
-        const int copies = rz_copies(b->n_rz, J);
-        if (copies > 1) {
-            LP_BCUDA(b, b->rz_part.ensure(J * copies * b->n_rz));
-            LP_BCUDA(b, cudaMemsetAsync(b->rz_part.p, 0, J * copies * b->n_rz * 8, b->stream));
+        const int r = alloc_instances(b, I);
+        if (r) {
+            drop_instances(b);
+            return r;
         }
-        LP_BCUDA(b, b->vox.ensure(J * std::max<size_t>(b->n_vox, 1)));
-        LP_BCUDA(b, b->rbins.ensure(J * std::max<size_t>(b->n_rbins, 1)));
-        LP_BCUDA(b, b->region.ensure(J * lp::kBatchMedia));
-        LP_BCUDA(b, b->det.ensure(J * std::max<size_t>(b->n_det, 1) * 2));
-        LP_BCUDA(b, b->counters.ensure(J * LP_NCOUNTERS));
-        LP_BCUDA(b, b->grad.ensure(J * grad_stride(b)));
-        LP_BCUDA(b, b->claimed.ensure(J));
-        LP_BCUDA(b, b->cum.ensure(J + 1));
-        LP_BCUDA(b, b->media.ensure(J * lp::kBatchMedia));
-        LP_BCUDA(b, b->params.ensure(J));
     }
     b->inst.assign(in, in + n_inst);
     // the plain launches hold their parameters by value in the graph
