@@ -384,6 +384,10 @@ int lp_run_noalloc(const lp_noalloc_args *args, void *stream);
 int lp_query_triangles(lp_ctx *ctx, int64_t n, const float *orig, const float *dir,
                        const int32_t *ref_tri, const float *t_max, int32_t *id_out,
                        float *t_out);
+/* The roots and divisions of the reference arithmetic on the device, n of them: out = the square
+ * root of a (op 0), 1 / a (op 1), a / b (op 2), correctly rounded over the ranges that the
+ * transport takes them from. */
+int lp_exact_ops(int device, int32_t op, int64_t n, const float *a, const float *b, float *out);
 /* Philox4x32-10 blocks on the device: out[4*i..] = philox(ctr + (0,0,i,0), key). */
 int lp_philox_blocks(int device, const uint32_t *ctr, const uint32_t *key, int64_t n,
                      uint32_t *out);

@@ -127,6 +127,7 @@ _SIGS = {
     "lp_get_exit_records": ([C.c_void_p, _fp, C.c_int64], C.c_int),
     "lp_last_kernel_ms": ([C.c_void_p, _fp], C.c_int),
     "lp_query_triangles": ([C.c_void_p, C.c_int64, _fp, _fp, _ip, _fp, _ip, _fp], C.c_int),
+    "lp_exact_ops": ([C.c_int, C.c_int32, C.c_int64, _fp, _fp, _fp], C.c_int),
     "lp_philox_blocks": ([C.c_int, _u32p, _u32p, C.c_int64, _u32p], C.c_int),
     "lp_get_stats": ([C.c_void_p, C.POINTER(Stats)], C.c_int),
     "lp_get_device_tallies": ([C.c_void_p, C.POINTER(DeviceTallies)], C.c_int),

@@ -39,6 +39,7 @@ cudaError_t launch_query(const KParams &P, int smem, int64_t n, const float *ori
                          cudaStream_t s);
 cudaError_t launch_philox(const uint32_t *ctr, const uint32_t *key, int64_t n, uint32_t *out,
                           cudaStream_t s);
+cudaError_t launch_exact_ops(int op, int64_t n, const float *a, const float *b, float *out, cudaStream_t s);
 cudaError_t launch_cell_lists(const KParams &P, int n_tri, float h, float eps, uint32_t *count, const uint32_t *start,
                               int32_t *refs, cudaStream_t s);
 cudaError_t launch_cell_words(const KParams &P, float m, const uint32_t *count, const uint32_t *start, bool lists,
@@ -1460,6 +1461,24 @@ int lp_query_triangles(lp_ctx *c, int64_t n, const float *orig, const float *dir
     LP_CUDA(c, cudaMemcpyAsync(t_out, to.p, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
     LP_CUDA(c, cudaStreamSynchronize(s));
     o.release(); d.release(); tm.release(); to.release(); rf.release(); io.release();
+    return LP_OK;
+}
+
+int lp_exact_ops(int device, int32_t op, int64_t n, const float *a, const float *b, float *out)
+{
+    if (op < 0 || op > 2 || n < 0 || !a || !out || (op == 2 && !b))
+        return fail(nullptr, LP_ERR_INVALID, "lp_exact_ops: bad argument");
+    if (n == 0) return LP_OK;
+    cudaError_t e = cudaSetDevice(device);
+    DevBuf<float> da, db, dr;
+    if (e == cudaSuccess) e = da.ensure((size_t)n);
+    if (e == cudaSuccess) e = db.ensure((size_t)n);
+    if (e == cudaSuccess) e = dr.ensure((size_t)n);
+    if (e == cudaSuccess) e = cudaMemcpy(da.p, a, (size_t)n * 4, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && op == 2) e = cudaMemcpy(db.p, b, (size_t)n * 4, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = lp::launch_exact_ops(op, n, da.p, db.p, dr.p, 0);
+    if (e == cudaSuccess) e = cudaMemcpy(out, dr.p, (size_t)n * 4, cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) return cuda_fail(nullptr, e, "lp_exact_ops");
     return LP_OK;
 }
 

@@ -93,6 +93,13 @@ __global__ void __launch_bounds__(256) fold_kernel(unsigned long long *dst, unsi
     }
 }
 
+// op 0: sqrt_normal(a), 1: rcp_rn(a), 2: div_rn(a, b) with the reciprocal of rcp_rn.
+__global__ void __launch_bounds__(256) exact_ops_kernel(int op, int64_t n, const float *a, const float *b, float *out)
+{
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        out[i] = op == 0 ? sqrt_normal(a[i]) : op == 1 ? rcp_rn(a[i]) : div_rn(a[i], b[i], rcp_rn(b[i]));
+}
+
 __global__ void philox_kernel(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, uint32_t k0,
                               uint32_t k1, int64_t n, uint32_t *out)
 {
@@ -168,6 +175,12 @@ cudaError_t launch_fold(unsigned long long *dst, unsigned long long *part, int c
 {
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n * images + 255) / 256, 148 * 8));
     fold_kernel<<<grid, 256, 0, s>>>(dst, part, copies, n, images);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_exact_ops(int op, int64_t n, const float *a, const float *b, float *out, cudaStream_t s)
+{
+    exact_ops_kernel<<<(int)std::min<int64_t>((n + 255) / 256, 148 * 8), 256, 0, s>>>(op, n, a, b, out);
     return cudaGetLastError();
 }
 
