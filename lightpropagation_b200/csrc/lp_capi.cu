@@ -245,7 +245,7 @@ struct lp_ctx {
     float fiber_radius = 0.0f, fiber_na = 0.0f;
     lp_geometry geo{};
     // device buffers
-    DevBuf<float4> node_a, node_b, node_c, tri, tri_soa, attr;   // tri_soa: as uploaded
+    DevBuf<float4> node_a, node_b, node_c, tri, attr;
     DevBuf<int4> node_d;
     DevBuf<Medium> media;
     DevBuf<unsigned long long> sft, rtd, rz, vox, rbins, region, det, counters, work;
@@ -435,18 +435,18 @@ int upload_mesh(lp_ctx *c)
     LP_CUDA(c, c->node_c.ensure(nn));
     LP_CUDA(c, c->node_d.ensure(nn));
     LP_CUDA(c, c->tri.ensure(3 * nt));
-    LP_CUDA(c, c->tri_soa.ensure(3 * nt));
+    DevBuf<float4> soa;   // the three arrays of the host tree, put together per triangle on the device
+    LP_CUDA(c, soa.ensure(3 * nt));
     LP_CUDA(c, c->attr.ensure(nt));
     cudaStream_t s = c->stream;
     LP_CUDA(c, cudaMemcpyAsync(c->node_a.p, b.node_a.data(), nn * 16, cudaMemcpyHostToDevice, s));
     LP_CUDA(c, cudaMemcpyAsync(c->node_b.p, b.node_b.data(), nn * 16, cudaMemcpyHostToDevice, s));
     LP_CUDA(c, cudaMemcpyAsync(c->node_c.p, b.node_c.data(), nn * 16, cudaMemcpyHostToDevice, s));
     LP_CUDA(c, cudaMemcpyAsync(c->node_d.p, b.node_d.data(), nn * 16, cudaMemcpyHostToDevice, s));
-    // the three arrays of the host tree, put together per triangle on the device
-    LP_CUDA(c, cudaMemcpyAsync(c->tri_soa.p, b.tri_a.data(), nt * 16, cudaMemcpyHostToDevice, s));
-    LP_CUDA(c, cudaMemcpyAsync(c->tri_soa.p + nt, b.tri_b.data(), nt * 16, cudaMemcpyHostToDevice, s));
-    LP_CUDA(c, cudaMemcpyAsync(c->tri_soa.p + 2 * nt, b.tri_c.data(), nt * 16, cudaMemcpyHostToDevice, s));
-    LP_CUDA(c, lp::launch_interleave(c->tri_soa.p, (int64_t)nt, c->tri.p, s));
+    LP_CUDA(c, cudaMemcpyAsync(soa.p, b.tri_a.data(), nt * 16, cudaMemcpyHostToDevice, s));
+    LP_CUDA(c, cudaMemcpyAsync(soa.p + nt, b.tri_b.data(), nt * 16, cudaMemcpyHostToDevice, s));
+    LP_CUDA(c, cudaMemcpyAsync(soa.p + 2 * nt, b.tri_c.data(), nt * 16, cudaMemcpyHostToDevice, s));
+    LP_CUDA(c, lp::launch_interleave(soa.p, (int64_t)nt, c->tri.p, s));
     LP_CUDA(c, cudaMemcpyAsync(c->attr.p, c->tri_attr.data(), nt * 16, cudaMemcpyHostToDevice, s));
     c->h2d_bytes += (int64_t)(nn * 64 + nt * 64);
     c->mesh_dirty = false;
@@ -826,7 +826,7 @@ void lp_destroy(lp_ctx *c)
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     c->node_a.release(); c->node_b.release(); c->node_c.release(); c->node_d.release();
-    c->tri.release(); c->tri_soa.release(); c->attr.release();
+    c->tri.release(); c->attr.release();
     c->media.release();
     c->sft.release(); c->rtd.release(); c->rz.release(); c->vox.release(); c->rbins.release();
     c->region.release(); c->det.release(); c->counters.release(); c->work.release();
