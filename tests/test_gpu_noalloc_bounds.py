@@ -56,3 +56,29 @@ def test_bounds_change_no_tally(n_tri, scale, shift):
         assert np.array_equal(out[k].cpu().numpy().view(np.uint64), ref[k].ravel()), k
     cnt = out["counters"].cpu().numpy()
     assert int(cnt[8]) == n and int(cnt[0]) == ref["counters"]["scatter"]
+
+
+@pytest.mark.parametrize("mesh", ["slab", "abdomen"])
+def test_many_photons_change_no_tally(mesh):
+    """Above 64 photons for each of 16 warps per SM (151,552 on 148 SMs) the kernel's other
+    instance runs, with more blocks and fewer registers."""
+    import torch
+
+    dev = torch.device("cuda", 0)
+    n, seed = 64 * 16 * torch.cuda.get_device_properties(dev).multi_processor_count + 4099, 29
+    w = workloads.plain_slab() if mesh == "slab" else workloads.curved_abdomen(freq=3)
+    ref, g = regular(w, n, seed)
+    tri, nrm, med = (torch.from_numpy(np.ascontiguousarray(x, t).ravel()).to(dev)
+                     for x, t in ((w.tri, np.float32), (w.nrm, np.float32), (w.med, np.int32)))
+    nm = np.ascontiguousarray(w.nmuasg, np.float32).ravel()
+    sizes = {"sft": g.sft_nx * g.sft_ny * 3, "rtd": g.dimR * g.dimAlpha * 3, "rz": g.rz_nr * g.rz_nz * 2,
+             "region": w.nmuasg.shape[0], "counters": 16}
+    out = {k: torch.zeros(v, dtype=torch.int64, device=dev) for k, v in sizes.items()}
+    a = _args(w, seed, n, tri, nrm, med, nm, out)
+    rc = _native.lib().lp_run_noalloc(C.byref(a), C.c_void_p(torch.cuda.current_stream(dev).cuda_stream))
+    assert rc == 0
+    torch.cuda.synchronize(dev)
+    for k in KEYS:
+        assert np.array_equal(out[k].cpu().numpy().view(np.uint64), ref[k].ravel()), k
+    cnt = out["counters"].cpu().numpy()
+    assert int(cnt[8]) == n and int(cnt[0]) == ref["counters"]["scatter"]
