@@ -17,7 +17,6 @@
 #include <cstdio>
 #include <cstring>
 #include <memory>
-#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -777,13 +776,6 @@ void smem_plan(const lp_ctx *c, int budget, int &nodes_smem, int &tris_smem)
 
 // helpers shared with lp_noalloc.cu
 namespace lp {
-// Held from setting a transport kernel's shared-memory attribute to its launch: the
-// attribute belongs to the kernel, not to a context or a call.
-std::mutex &launch_mutex()
-{
-    static std::mutex m;
-    return m;
-}
 void set_thread_error(const char *msg) { g_thread_error = msg; }
 float rspecular_of(const float *nmuasg, int n_media) { return rspecular(nmuasg, n_media); }
 }  // namespace lp
@@ -1129,9 +1121,6 @@ int lp_run_async(lp_ctx *c, int64_t first, int64_t n)
     smem_plan(c, c->smem_budget, nodes_smem, tris_smem);
     const int smem = lp::smem_bytes(nodes_smem, tris_smem);
     int per_sm = 0;
-    // the shared-memory attribute set by the occupancy query is process-wide; the lock
-    // keeps another thread's setting from landing between it and this launch
-    std::lock_guard<std::mutex> launch_lock(lp::launch_mutex());
     if (c->grad_on)
         LP_CUDA(c, c->exact ? lp::transport_occupancy_exact_grad(smem, &per_sm)
                             : lp::transport_occupancy_fast_grad(smem, &per_sm));
@@ -1747,14 +1736,12 @@ int enqueue_zero(lp_batch *b)
 // launch's shared memory (queried outside stream capture).
 int prepare_plain(lp_batch *b)
 {
-    std::lock_guard<std::mutex> launch_lock(lp::launch_mutex());
     for (lp_batch::PlainLaunch &L : b->plain) {
         int per_sm = 0;
         LP_BCUDA(b, b->grad_on ? lp::transport_occupancy_fast_grad(L.smem, &per_sm)
                                : lp::transport_occupancy_fast(L.smem, &per_sm));
         if (per_sm < 1) return bfail(b, LP_ERR_CUDA, "batch: transport kernel does not fit on an SM");
         lp::plan_launch(L.P.n, lp::block_size(), b->num_sms, per_sm, L.grid, L.P.lane_mask, L.P.few_blocks);
-        L.P.few_blocks = 0;   // that instance sets its shared-memory attribute at the launch, here a capture
     }
     return LP_OK;
 }

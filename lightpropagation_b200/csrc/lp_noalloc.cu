@@ -30,7 +30,6 @@ cudaError_t launch_transport_no_grid(const KParams &P, int grid, int smem, cudaS
 cudaError_t transport_occupancy_no_grid(int smem, int *blocks_per_sm);
 void set_thread_error(const char *msg);
 float rspecular_of(const float *nmuasg, int n_media);
-std::mutex &launch_mutex();
 }  // namespace lp
 
 namespace {
@@ -368,17 +367,12 @@ extern "C" int lp_run_noalloc(const lp_noalloc_args *a, void *stream)
     const int smem = smem_bytes(P.nodes_smem, P.tris_smem);
     int per_sm = 0, sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    {
-        // the kernel's shared-memory attribute is process-wide: lp_run on another thread
-        // sets it too, so the setting and the launch are made under the same lock
-        std::lock_guard<std::mutex> lk(lp::launch_mutex());
-        if ((e = transport_occupancy_no_grid(smem, &per_sm)) != cudaSuccess || per_sm < 1)
-            return reject(LP_ERR_CUDA, "lp_run_noalloc: occupancy query failed");
-        int grid;
-        plan_launch(P.n, block_size(), sms, per_sm, grid, P.lane_mask, P.few_blocks);
-        if ((e = launch_transport_no_grid(P, grid, smem, s)) != cudaSuccess)
-            return reject(LP_ERR_CUDA, "lp_run_noalloc: transport launch failed");
-    }
+    if ((e = transport_occupancy_no_grid(smem, &per_sm)) != cudaSuccess || per_sm < 1)
+        return reject(LP_ERR_CUDA, "lp_run_noalloc: occupancy query failed");
+    int grid;
+    plan_launch(P.n, block_size(), sms, per_sm, grid, P.lane_mask, P.few_blocks);
+    if ((e = launch_transport_no_grid(P, grid, smem, s)) != cudaSuccess)
+        return reject(LP_ERR_CUDA, "lp_run_noalloc: transport launch failed");
     if (a->counters) {
         e = cudaMemcpyAsync(a->counters, sb + OFF_CNT, LP_NCOUNTERS * sizeof(uint64_t), cudaMemcpyDeviceToDevice, s);
         if (e != cudaSuccess) return reject(LP_ERR_CUDA, "lp_run_noalloc: counter copy failed");

@@ -25,8 +25,7 @@ cudaError_t launch_transport_no_grid(const KParams &P, int grid, int smem, cudaS
 
 cudaError_t transport_occupancy_no_grid(int smem, int *blocks_per_sm)
 {
-    cudaError_t e = cudaFuncSetAttribute(transport_kernel<true, false, false, true>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t e = allow_smem(transport_kernel<true, false, false, true>, smem);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, transport_kernel<true, false, false, true>, kBlock,
                                                          smem);
@@ -155,7 +154,7 @@ cudaError_t launch_query(const KParams &P, int smem, int64_t n, const float *ori
                          const int32_t *ref, const float *tmax, int32_t *id_out, float *t_out,
                          cudaStream_t s)
 {
-    cudaError_t e = cudaFuncSetAttribute(query_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t e = allow_smem(query_kernel, smem);
     if (e != cudaSuccess) return e;
     int grid = (int)std::min<int64_t>((n + kBlock - 1) / kBlock, 148 * 8);
     if (grid < 1) grid = 1;

@@ -45,6 +45,7 @@
 //               device function gives the same bits in every kernel that inlines it.
 #pragma once
 #include <algorithm>
+#include <mutex>
 
 #include "lp_kernel.cuh"
 
@@ -1023,11 +1024,24 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) transport_kernel(const __gr
         if (s_region[i]) atomicAdd(P.region + i, s_region[i]);
 }
 
+// Lets `kernel` be launched with smem bytes of dynamic shared memory.  The limit belongs to the
+// kernel (on the current device), so it is raised where it is too low and never lowered: another
+// thread's launch, or one that is captured into a graph later, may need more than this one.
+template <class Kernel>
+cudaError_t allow_smem(Kernel *kernel, int smem)
+{
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    cudaFuncAttributes a;
+    const cudaError_t e = cudaFuncGetAttributes(&a, kernel);
+    if (e != cudaSuccess || a.maxDynamicSharedSizeBytes >= smem) return e;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+}
+
 template <bool Exact, bool Grad, bool Agg, bool NoGrid, int MinBlocks>
 cudaError_t launch_instance(const KParams &P, int grid, int smem, cudaStream_t s)
 {
-    cudaError_t e = cudaFuncSetAttribute(transport_kernel<Exact, Grad, Agg, NoGrid, MinBlocks>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t e = allow_smem(transport_kernel<Exact, Grad, Agg, NoGrid, MinBlocks>, smem);
     if (e != cudaSuccess) return e;
     transport_kernel<Exact, Grad, Agg, NoGrid, MinBlocks><<<grid, kBlock, smem, s>>>(P);
     return cudaGetLastError();
@@ -1035,9 +1049,7 @@ cudaError_t launch_instance(const KParams &P, int grid, int smem, cudaStream_t s
 
 // P.grad selects the differentiating instantiation.
 // The warp-aggregated form exists for the production arithmetic without differentiation
-// only (P.agg_tallies is ignored otherwise).  The instance for few blocks sets its own
-// shared-memory attribute; the occupancy query has set the other's (prepare_plain outside of
-// stream capture).
+// only (P.agg_tallies is ignored otherwise).
 template <bool Exact>
 cudaError_t launch_transport_t(const KParams &P, int grid, int smem, cudaStream_t s)
 {
@@ -1046,16 +1058,14 @@ cudaError_t launch_transport_t(const KParams &P, int grid, int smem, cudaStream_
     if (P.few_blocks)
         return P.grad ? launch_instance<Exact, true, false, false, kFewBlocks>(P, grid, smem, s)
                       : launch_instance<Exact, false, false, false, kFewBlocks>(P, grid, smem, s);
-    if (P.grad) transport_kernel<Exact, true><<<grid, kBlock, smem, s>>>(P);
-    else transport_kernel<Exact, false><<<grid, kBlock, smem, s>>>(P);
-    return cudaGetLastError();
+    return P.grad ? launch_instance<Exact, true, false, false, LP_TRANSPORT_MIN_BLOCKS>(P, grid, smem, s)
+                  : launch_instance<Exact, false, false, false, LP_TRANSPORT_MIN_BLOCKS>(P, grid, smem, s);
 }
 
 template <bool Exact, bool Grad>
 cudaError_t transport_occupancy_t(int smem, int *blocks_per_sm)
 {
-    cudaError_t e = cudaFuncSetAttribute(transport_kernel<Exact, Grad>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         smem);
+    const cudaError_t e = allow_smem(transport_kernel<Exact, Grad>, smem);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, transport_kernel<Exact, Grad>, kBlock, smem);
 }

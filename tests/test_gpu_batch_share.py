@@ -31,3 +31,35 @@ def test_every_instance_is_traced_once(counts, config):
                 want = s.tallies()
                 for key in ("sft", "rz", "vox", "rbins"):
                     assert np.array_equal(got[k][key], want[key]), key
+
+
+@pytest.mark.parametrize("config", [0, 2])
+@pytest.mark.parametrize("plain", [0, 3000])    # 3000: the large ones as launches of their own
+def test_every_instance_gets_its_own_tallies(plain, config):
+    """Instances that differ in photons and media, on two meshes: the tallies of each one are
+    those of a run by itself."""
+    slab, abdomen = workloads.plain_slab(), workloads.curved_abdomen(freq=8)
+    for w in (slab, abdomen):
+        w.vox_n, w.n_rbins, w.det_r = (0, 0, 0), 0, None
+        w.dimensions, w.det_grid = slab.dimensions, slab.det_grid
+    rng = np.random.default_rng(2)
+    inst = []
+    for i, n in enumerate((1, 4000, 0, 33, 700, 5000, 2, 64, 3000, 90, 1, 250)):
+        w = (slab, abdomen)[i % 2]
+        media = np.array(w.nmuasg, np.float32)
+        media[1:, 1:3] *= rng.uniform(0.8, 1.2, media[1:, 1:3].shape).astype(np.float32)
+        inst.append(Instance(i % 2, media, n, 1000 * i))
+    with slab.apply(Simulation(0), seed=3) as a, abdomen.apply(Simulation(0), seed=3) as c, Batch([a, c]) as b:
+        b.set_plain_threshold(plain)
+        b.set_config(config)
+        b.set_instances(inst)
+        b.run()
+        for i, x in enumerate(inst):
+            got, s = b.tallies(i), (a, c)[x.context]
+            s.set_media(x.nmuasg)
+            s.zero()
+            s.run(x.n_photons, x.first)
+            want = s.tallies()
+            for key in ("sft", "rtd", "rz", "region"):
+                assert np.array_equal(got[key], want[key]), (i, key)
+            assert got["counters"]["photons"] == x.n_photons
