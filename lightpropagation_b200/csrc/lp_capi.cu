@@ -301,6 +301,7 @@ int fail(lp_ctx *c, int code, const char *fmt, ...)
 
 int cuda_fail(lp_ctx *c, cudaError_t e, const char *what)
 {
+    cudaGetLastError();   // reported here: a later launch must not take it for its own
     return fail(c, e == cudaErrorMemoryAllocation ? LP_ERR_NOMEM : LP_ERR_CUDA, "%s: %s", what,
                 cudaGetErrorString(e));
 }
@@ -1567,7 +1568,10 @@ int bfail(lp_batch *b, int code, const char *fmt, ...)
 #define LP_BCUDA(b, call)                                                        \
     do {                                                                         \
         cudaError_t _e = (call);                                                 \
-        if (_e != cudaSuccess) return bfail(b, LP_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(_e)); \
+        if (_e != cudaSuccess) {                                                 \
+            cudaGetLastError(); /* as cuda_fail */                               \
+            return bfail(b, LP_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(_e)); \
+        }                                                                        \
     } while (0)
 
 void drop_graph(lp_batch *b)
@@ -1927,7 +1931,7 @@ int lp_batch_create(lp_batch **out, int32_t n_ctx, lp_ctx *const *ctxs)
     if (e == cudaSuccess) e = cudaEventCreate(&b->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&b->ev1);
     if (e != cudaSuccess) {
-        int r = fail(nullptr, LP_ERR_CUDA, "lp_batch_create: %s", cudaGetErrorString(e));
+        int r = cuda_fail(nullptr, e, "lp_batch_create");
         lp_batch_destroy(b);
         return r;
     }
@@ -2073,11 +2077,11 @@ int lp_batch_run(lp_batch *b)
         if (!r) r = enqueue_launch(b, b->config);
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamEndCapture(b->stream, &g);
-        if (r) {
+        if (r || e != cudaSuccess) {
+            cudaGetLastError();   // as cuda_fail
             if (g) cudaGraphDestroy(g);
-            return r;
+            return r ? r : bfail(b, LP_ERR_CUDA, "lp_batch_run: capture: %s", cudaGetErrorString(e));
         }
-        if (e != cudaSuccess) return bfail(b, LP_ERR_CUDA, "lp_batch_run: capture: %s", cudaGetErrorString(e));
         b->graph = g;
         LP_BCUDA(b, cudaGraphInstantiate(&b->exec, b->graph, 0));
     }

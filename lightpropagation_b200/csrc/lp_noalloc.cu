@@ -240,6 +240,7 @@ int scratch_address(int dev, cudaStream_t s, void **out)
 
 int reject(int code, const char *msg)
 {
+    if (code == LP_ERR_CUDA) cudaGetLastError();   // reported here: a later launch must not take it for its own
     lp::set_thread_error(msg);
     return code;
 }
