@@ -50,9 +50,9 @@ __global__ void __launch_bounds__(kBlock) query_kernel(const __grid_constant__ K
     __syncthreads();
     // A march costs by the cell, a descent of a small tree little: on meshes below 2,048
     // triangles rays of more than n_tri / 16 cells go to the tree.  1e6 rays, march / tree, us:
-    // slab (32 triangles) of 3 cells 139 / 107, of 34 517 / 181, unbounded 1221 / 271; abdomen of
-    // 100 triangles, 3 cells 183 / 538, 40 753 / 719, unbounded 1178 / 864; of 900, 10 cells 413 /
-    // 704, unbounded 1229 / 1350.
+    // slab (32 triangles) of 3 cells 139 / 96, of 34 517 / 159, unbounded 1221 / 237; abdomen of
+    // 100 triangles, 3 cells 183 / 477, 40 753 / 638, unbounded 1178 / 766; of 1,600, 10 cells 319 /
+    // 622, unbounded 1220 / 1208.
     const float march = P.n_tri < 2048 ? (float)P.n_tri * P.g_h * (1.0f / 16.0f) : 3.0e38f;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     // warp-uniform trip count: the query is the whole warp's
@@ -162,7 +162,8 @@ cudaError_t launch_query(const KParams &P, int smem, int64_t n, const float *ori
 {
     const cudaError_t e = allow_smem(query_kernel, smem);
     if (e != cudaSuccess) return e;
-    int grid = (int)std::min<int64_t>((n + kBlock - 1) / kBlock, 148 * 8);
+    // 2,048 threads per SM; half of them took a fifth longer for 1e6 rays
+    int grid = (int)std::min<int64_t>((n + kBlock - 1) / kBlock, 148 * 16);
     if (grid < 1) grid = 1;
     query_kernel<<<grid, kBlock, smem, s>>>(P, n, orig, dir, ref, tmax, id_out, t_out);
     return cudaGetLastError();
