@@ -361,6 +361,7 @@ __device__ __forceinline__ float fresnel(float n1, float n2, float cosIn)
 // redux.sync, and each slice's sum over at most 32 lanes fits in 32 bits.
 __device__ __forceinline__ unsigned long long group_sum_u64(unsigned grp, unsigned long long x)
 {
+    if ((grp & (grp - 1u)) == 0u) return x;   // a group of one, as most are
     const unsigned a = __reduce_add_sync(grp, (unsigned)(x & 0xffffull));
     const unsigned b = __reduce_add_sync(grp, (unsigned)((x >> 16) & 0xffffull));
     const unsigned c = __reduce_add_sync(grp, (unsigned)(x >> 32));
