@@ -232,7 +232,7 @@ int lp_set_smem_budget(lp_ctx *ctx, int32_t bytes);
  * identical either way; lp_query_triangles follows the same setting. */
 int lp_set_cell_lists(lp_ctx *ctx, int enable);
 /* Margin of the cell lists, in cells (default 0.5, or 0.75 where the triangles span many
- * cells; 0 to 4): each cell lists the
+ * cells; 0 to 4, a quarter being the least that is built): each cell lists the
  * triangles that touch the cell widened by this margin on every side.  A wider margin
  * lets more short-step queries be answered from one cell's list and gives larger
  * distance bounds from the planes of the listed triangles, at the cost of longer lists.

@@ -714,7 +714,10 @@ int build_safety_grid(lp_ctx *c)
     cudaEventRecord(e0, s);
     bool lists = false;
     const int nt = (int)c->bvh.tri_a.size();
-    c->grid_margin = c->cell_margin;
+    // A march stands still between a cell's faces without a margin, and its queries go to the
+    // tree: 0 cells / a quarter, ms: slab 2e5 photons 51 / 33, abdomen 25,600 triangles 1e5 75 / 23,
+    // 202,500 3e5 133 / 39, 2.25 M 1e5 72 / 32.
+    c->grid_margin = std::max(c->cell_margin, 0.25f);
     // every list holds the triangles that touch its cell widened by the margin plus g_eps
     auto list_eps = [c]() { return c->grid_margin * c->g_h + c->g_eps; };
     // counts, their scan and the number of entries

@@ -186,8 +186,8 @@ class Simulation:
 
     def set_cell_margin(self, cells: float):
         """Margin of the cell lists in cells (default 0.5, or 0.75 where the triangles span
-        many cells): each list holds the triangles touching its cell widened by this much
-        (results are unchanged)."""
+        many cells; at least a quarter is built): each list holds the triangles touching its
+        cell widened by this much (results are unchanged)."""
         self._ck(self._L.lp_set_cell_margin(self._h, float(cells)))
 
     def set_tally_aggregation(self, enable: bool):
