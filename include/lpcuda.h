@@ -201,8 +201,8 @@ int lp_batch_set_gradient(lp_batch *b, int enable);
 /* Instances of at least `photons` photons run as a persistent transport launch of their
  * own inside the batch's graph (the rest share the batch launch); photons <= 0: all
  * share it.  Default 2^20: the batch kernel's instance switching costs every photon a
- * little, a launch of its own costs one drain, and the two meet near 7e5 photons on the
- * abdomen.  Tallies are the same either way. */
+ * little, a launch of its own costs one drain, and the two meet at 1e6 photons on the slab
+ * and 2e6 to 3e6 on the abdomen.  Tallies are the same either way. */
 int lp_batch_set_plain_threshold(lp_batch *b, int64_t photons);
 /* Instances the current setting runs as launches of their own. */
 int lp_batch_plain_count(const lp_batch *b, int32_t *count);
@@ -225,7 +225,9 @@ int lp_batch_get_gradient(lp_batch *b, int32_t inst, lp_gradient *out);
 
 /* Shared memory per block (bytes) for BVH nodes and triangles staged by the transport
  * kernel; what a block does not take stays L1 cache for the cell grid, tallies and the
- * rest of the mesh.  Default 8192.  No reference counterpart; results do not depend on it. */
+ * rest of the mesh.  Default 8192; above 38 KB fewer than five blocks fit on an SM (202,500
+ * triangles, 2e6 photons: 8 to 38 KB 124 ms, 64 KB 162, 200 KB 390).  No reference counterpart;
+ * results do not depend on it. */
 int lp_set_smem_budget(lp_ctx *ctx, int32_t bytes);
 /* Whether cells touched by triangles list them (1, default) or hold no information
  * (0: every query that the safety bound does not skip descends the BVH).  Results are

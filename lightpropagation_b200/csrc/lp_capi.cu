@@ -349,9 +349,10 @@ int64_t n_vox(const lp_ctx *c)
 // near it take most of the adds: the L2 works them off one after the other.  On the curved
 // abdomen at 660 nm (3e6 photons, 1.2 MB image, the step as it was then) one copy took
 // 400 ms, two 277, four 217 and eight or more 216; without the deposits it was 215.
-// Sixteen leave room for a faster step.  The limit keeps the copies within a quarter of the
-// L2 (a larger image has finer cells, so fewer adds to each).  The instances of a batch
-// launch run side by side, each with an image of its own, and share out the sixteen.
+// Sixteen leave room for a faster step.  The limit keeps the copies of one image within a
+// quarter of the L2 (a larger image has finer cells, so fewer adds to each).  The instances of
+// a batch launch run side by side, each with an image of its own, and share out the sixteen:
+// together they can be twice the L2 (eight images of 16 MB).
 int rz_copies(size_t n, size_t images = 1)
 {
     size_t k = 16;
@@ -1525,9 +1526,10 @@ struct lp_batch {
     // Instances of at least plain_min photons (plain_min > 0) run as a persistent transport
     // launch of their own inside the graph, with their context's shared-memory plan; the
     // batch kernel sees them with no photons.  The batch kernel pays for its per-warp
-    // instance switching on every photon, a launch of its own only once (its drain):
-    // at about 7e5 photons the two cost the same on the abdomen (measured when the warps of
-    // the batch launch all began on its first instance).
+    // instance switching on every photon, a launch of its own only once (its drain).  Equal
+    // instances, shared / own, ms: abdomen 2 x 1e6 128 / 141, 2 x 3e6 351 / 342, 2 x 1e7 1136 /
+    // 1049, 8 x 1e6 467 / 572, 8 x 3e6 1387 / 1374; slab 2 x 1e6 178 / 178, 2 x 3e6 503 / 472, 8 x
+    // 1e6 665 / 713.  So they meet at 1e6 to 3e6 photons; the default is the callers' to raise.
     struct PlainLaunch {
         KParams P;
         int grid = 0, smem = 0;

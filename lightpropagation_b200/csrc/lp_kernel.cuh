@@ -135,7 +135,7 @@ struct KParams {
 // -> 27.3; at 300,000 more warps win on the slab (43.7 against 47.7) and lose on the abdomen
 // (42.8 against 40.2).
 // few: the launch has no more than those warps, so the kernel instance compiled for them runs
-// (106 registers instead of 95): 30,000 slab photons 16.7 -> 15.7 ms, 50,000 on 25,600
+// (107 registers instead of 95): 30,000 slab photons 16.7 -> 15.7 ms, 50,000 on 25,600
 // triangles 17.3 -> 16.4, 1e5 on the abdomen 23.7 -> 23.0.
 inline void plan_launch(int64_t n, int block, int num_sms, int per_sm, int &grid, uint32_t &lane_mask, uint32_t &few)
 {

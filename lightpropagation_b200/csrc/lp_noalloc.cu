@@ -70,7 +70,7 @@ __device__ __forceinline__ void grow(float *b, float x, float y, float z)
     b[3] = fmaxf(b[3], x); b[4] = fmaxf(b[4], y); b[5] = fmaxf(b[5], z);
 }
 
-// One block: media table, triangles in the kernel's SoA layout, per-triangle attributes
+// One block: media table, triangles in the kernel's 48-byte records, per-triangle attributes
 // and the BVH.  Explicit round-to-nearest intrinsics reproduce the host's IEEE values
 // (no contraction), so the transport sees exactly the inputs lp_set_* would produce.
 __global__ void __launch_bounds__(256) noalloc_setup_kernel(const float *tri, const float *nrm, const int32_t *med,

@@ -5,9 +5,9 @@
 // persistent: each warp refills the lanes whose photon has finished with new photon
 // ids taken from a global counter, one atomicAdd per warp refill, so lanes stay busy
 // until the photon budget is spent.  Photon i draws its random numbers from Philox
-// blocks (key = seed, counter = (i, event, stream)), so results do not depend on
-// which thread traced which photon; every loop iteration computes exactly one block,
-// which keeps the warp converged on the RNG.
+// blocks (key = seed, counter = (i, event, stream)), one per event, so results do not
+// depend on which thread traced which photon, nor on whether its own lane drew the event or
+// an idle one did some events ahead (next_draws).
 //
 // Per loop iteration (MCLightPropagation.cl:1375-1575), the warp's lanes together:
 //   step length (.cl:1405-1442) -> nearest triangle within the step (replaces the O(T)
@@ -524,11 +524,9 @@ __device__ __forceinline__ void start_photon(const KParams &P, Photon &ph, uint3
 
 // A boundary event (.cl:1443-1465 with TransmitOrReflect, .cl:921-1018): the photon moves
 // thit to the face `tri` (-1: no face, it leaves the model), then is transmitted or
-// reflected with probability from the Fresnel equations (xi against R).  Out of line: it
-// runs about once per hundred steps, and keeping its code out of the step loop keeps the
-// loop's instructions in cache for the warps that scatter.  The photon goes in and comes
-// back by value: a reference would take its address out of the step loop, and the
-// compiler would then keep the photon in local memory on every step.
+// reflected with probability from the Fresnel equations (xi against R).  Inline, although it
+// runs about once per hundred steps: the photon goes in and comes back by value, and out of
+// line that would be a copy of it through local memory.
 template <bool Exact, bool Grad>
 static __device__ __forceinline__ Photon boundary_event(const KParams &P, const Medium *s_media,
                                                      unsigned long long *s_region, unsigned long long *s_cnt,
