@@ -181,7 +181,9 @@ int lp_backward(lp_ctx *ctx, const double *grad_signal, double *grad_mua, double
  * (CalculatePropagation.cpp:1389-1759); here wavelengths x optical-property draws x
  * meshes with uneven budgets share the GPU and drain once.  Each instance's tallies
  * equal, bit for bit, those of lp_run on its context with its media and photon range.
- * All contexts must live on the same device and share one tally layout. */
+ * All contexts must live on the same device and share one tally layout, which is the batch's
+ * for its life; a mesh or cell grid that a context got since is taken up by the next
+ * lp_batch_set_instances or lp_batch_run. */
 #define LP_BATCH_MAX_MEDIA 8
 typedef struct lp_instance {
     int32_t context;                          /* index into the batch's contexts         */

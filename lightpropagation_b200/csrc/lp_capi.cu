@@ -223,6 +223,7 @@ struct lp_ctx {
     bool mesh_dirty = false, media_dirty = false, tally_dirty = true;
     int64_t n_tri = 0;
     int32_t max_region = 0;   // largest region id referenced by the mesh
+    uint64_t mesh_gen = 0;    // counts the meshes and cell grids put on the device
     lp::Bvh bvh;
     std::vector<float4> tri_attr;
     std::vector<float> nmuasg;
@@ -431,6 +432,7 @@ int upload_mesh(lp_ctx *c)
     if (!c->mesh_dirty) return LP_OK;
     const lp::Bvh &b = c->bvh;
     const size_t nn = b.node_a.size(), nt = b.tri_a.size();
+    ++c->mesh_gen;
     LP_CUDA(c, c->node_a.ensure(nn));
     LP_CUDA(c, c->node_b.ensure(nn));
     LP_CUDA(c, c->node_c.ensure(nn));
@@ -652,6 +654,7 @@ int build_safety_grid(lp_ctx *c)
 {
     Phase phase("lp cell grid build");
     c->n_cell_refs = 0;
+    ++c->mesh_gen;
     if (c->grid_max_cells <= 0 || c->n_tri == 0) {
         c->cell_word.release();
         c->cell_refs.release();
@@ -1549,6 +1552,9 @@ struct lp_batch {
         DevBuf<unsigned long long> rz, vox;
     };
     std::vector<std::unique_ptr<OwnTallies>> own;
+    std::vector<uint64_t> mesh_gen;   // lp_ctx::mesh_gen of each context in the parameters
+    lp_geometry geo{};                // the tally layout that the buffers are for
+    int32_t vox_dim[3] = {0, 0, 0};
     std::vector<unsigned long long *> rz_of, vox_of;   // per instance: where its r-z, voxel tallies are
     float last_ms = 0.0f;
     std::vector<uint64_t> h_sft, h_rtd, h_rz, h_vox, h_rbins, h_region, h_det, h_cnt;
@@ -1629,6 +1635,25 @@ int alloc_instances(lp_batch *b, size_t I)
 int fill_instances(lp_batch *b)
 {
     const size_t I = b->inst.size();
+    // the contexts may have been changed since lp_batch_create
+    b->mesh_gen.assign(b->ctx.size(), 0);
+    for (size_t k = 0; I > 0 && k < b->ctx.size(); ++k) {
+        lp_ctx *c = b->ctx[k];
+        if (!c->have_mesh || !c->have_source || !c->have_grid)
+            return bfail(b, LP_ERR_STATE, "batch: context %d has no mesh, source or tally grid", (int)k);
+        int r = upload_mesh(c);
+        if (!r && c->grid_dirty) r = build_safety_grid(c);
+        if (r) return bfail(b, r, "batch: context %d: %s", (int)k, c->err.c_str());
+        if (std::memcmp(&c->geo, &b->geo, sizeof b->geo) != 0 || (size_t)c->n_rbins * 2 != b->n_rbins ||
+            c->det_r.size() / 2 != b->n_det || std::memcmp(c->vox_n, b->vox_dim, sizeof b->vox_dim) != 0)
+            return bfail(b, LP_ERR_STATE, "batch: the tally layout of context %d is not the one of lp_batch_create",
+                         (int)k);
+        b->mesh_gen[k] = c->mesh_gen;
+    }
+    for (size_t i = 0; i < I; ++i)
+        if (b->ctx[b->inst[i].context]->max_region >= b->inst[i].n_media)
+            return bfail(b, LP_ERR_INVALID, "batch: instance %d: mesh uses region %d", (int)i,
+                         b->ctx[b->inst[i].context]->max_region);
     std::vector<KParams> P(I);
     std::vector<Medium> M(I * lp::kBatchMedia);
     b->plain.clear();
@@ -1716,6 +1741,17 @@ int upload_instances(lp_batch *b)
     const int r = fill_instances(b);
     if (r) drop_instances(b);
     return r;
+}
+
+// A context that got another mesh or cell grid since the parameters were formed has replaced
+// what they point to: they are formed again.
+int refresh_instances(lp_batch *b)
+{
+    bool same = true;
+    for (size_t k = 0; k < b->ctx.size(); ++k) same = same && b->ctx[k]->mesh_gen == b->mesh_gen[k];
+    if (same) return LP_OK;
+    drop_graph(b);
+    return upload_instances(b);
 }
 
 // Zero the tallies and claim counters of all instances (enqueued on the batch stream).
@@ -1929,6 +1965,8 @@ int lp_batch_create(lp_batch **out, int32_t n_ctx, lp_ctx *const *ctxs)
     b->n_rtd = (size_t)g.dimR * g.dimAlpha * 3;
     b->n_rz = (size_t)g.rz_nr * g.rz_nz * 2;
     b->n_vox = (size_t)n_vox(c0);
+    b->geo = g;
+    std::memcpy(b->vox_dim, c0->vox_n, sizeof b->vox_dim);
     b->n_rbins = (size_t)c0->n_rbins * 2;
     b->n_det = c0->det_r.size() / 2;
     cudaError_t e = cudaSetDevice(b->device);
@@ -2067,6 +2105,11 @@ int lp_batch_run(lp_batch *b)
     if (b->inst.empty()) return LP_OK;
     LP_BCUDA(b, cudaSetDevice(b->device));
     int r;
+    if ((r = refresh_instances(b))) return r;
+    if (b->config >= 0 && !config_eligible(b, b->config)) {   // a deeper tree since it was chosen
+        drop_graph(b);
+        b->config = -1;
+    }
     if (b->config < 0) {
         int32_t best;
         if ((r = lp_batch_autotune(b, 4000000, &best, nullptr))) return r;
