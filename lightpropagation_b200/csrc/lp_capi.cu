@@ -392,7 +392,9 @@ cudaError_t fold_rz(lp_ctx *c)
 {
     if (!c->rz_pending) return cudaSuccess;
     const int copies = rz_copies(rz_values(c));
-    const cudaError_t e = launch_unless_injected([&] {
+    cudaError_t e = cudaSetDevice(c->device);   // the reading calls need no device of their own
+    if (e != cudaSuccess) return e;
+    e = launch_unless_injected([&] {
         return lp::launch_fold(c->rz.p, c->rz_part.p, copies, (int64_t)rz_values(c), 1, c->stream);
     });
     if (e == cudaSuccess) c->rz_pending = false;
@@ -1635,6 +1637,7 @@ int alloc_instances(lp_batch *b, size_t I)
 int fill_instances(lp_batch *b)
 {
     const size_t I = b->inst.size();
+    LP_BCUDA(b, cudaSetDevice(b->device));
     // the contexts may have been changed since lp_batch_create
     b->mesh_gen.assign(b->ctx.size(), 0);
     for (size_t k = 0; I > 0 && k < b->ctx.size(); ++k) {
